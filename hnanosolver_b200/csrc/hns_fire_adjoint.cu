@@ -36,132 +36,185 @@ enum { kD = 0, kT = 1, kF = 2, kW = 3, kFL = 4 };
 
 unsigned blocks_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-__device__ __forceinline__ void coords_at(const TopoView& t, int64_t s, int& i, int& j, int& k) {
-    const int4 o = t.origin[s >> 9];
-    const int n = (int)(s & 511);
-    i = o.x + ((n >> 6) & 7);
-    j = o.y + ((n >> 3) & 7);
-    k = o.z + (n & 7);
-}
-
-// Slot of (i, j, k), with the multi-field advection's fallback: slot 0 outside the domain.
-__device__ __forceinline__ int64_t slot0(const TopoView& t, int i, int j, int k) {
-    const int s = dev::leaf_from_table(t, i, j, k);
-    return s < 0 ? 0 : ((int64_t)s << 9) + dev::local_offset(i, j, k);
-}
-
-// setupInterpolation (src/Cuda/Kernel.cu:204-233) as the forward computes it (x fastest in the
-// tap index, the same weight products), with the weights' position derivatives.
-struct WTaps {
-    int64_t s[8];
-    float w[8], gx[8], gy[8], gz[8];
+// The advected fields of the step and their adjoints, up to kFields of them in any order.
+struct AdvectedBars {
+    const float* d[kFields];        // the fields the advection read
+    const float* out_bar[kFields];  // the adjoints of the advected fields
+    float* d_bar[kFields];          // += the adjoints of d
+    int count;
 };
 
-__device__ __forceinline__ void wtaps(const TopoView& t, float x, float y, float z, WTaps& T) {
-    const int i0 = __float2int_rd(x), j0 = __float2int_rd(y), k0 = __float2int_rd(z);
-    const float tx = x - (float)i0, ty = y - (float)j0, tz = z - (float)k0;
-    const float itx = 1.0f - tx, ity = 1.0f - ty, itz = 1.0f - tz;
-    const float w00 = itx * ity, w10 = tx * ity, w01 = itx * ty, w11 = tx * ty;
-    T.w[0] = w00 * itz, T.w[1] = w10 * itz, T.w[2] = w01 * itz, T.w[3] = w11 * itz;
-    T.w[4] = w00 * tz, T.w[5] = w10 * tz, T.w[6] = w01 * tz, T.w[7] = w11 * tz;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int a = q & 1, b = (q >> 1) & 1, c = (q >> 2) & 1;
-        const float wx = a ? tx : itx, wy = b ? ty : ity, wz = c ? tz : itz;
-        T.gx[q] = (a ? 1.f : -1.f) * wy * wz;
-        T.gy[q] = wx * (b ? 1.f : -1.f) * wz;
-        T.gz[q] = wx * wy * (c ? 1.f : -1.f);
-        T.s[q] = slot0(t, i0 + a, j0 + b, k0 + c);
-    }
-}
-
-// Adjoint of advect_scalars for one field d advected along vel (the projected velocity):
-// d_bar += (d out / d d)^T out_bar, vel_bar += (d out / d vel)^T out_bar.
-__global__ void __launch_bounds__(kThreads) adj_advect_scalars_kernel(TopoView t, const float* __restrict__ vel,
-                                                                      const float* __restrict__ d,
-                                                                      const float* __restrict__ out_bar,
-                                                                      float* __restrict__ d_bar,
-                                                                      float* __restrict__ vel_bar, float sdt, int64_t n) {
+// Interleaves the fields the adjoint gathers: fields 0..3 of a slot, and its velocity with field 4.
+__global__ void __launch_bounds__(kThreads) pack_records_kernel(AdvectedBars F, const float* __restrict__ vel,
+                                                                float4* __restrict__ in4, float4* __restrict__ vel_in4,
+                                                                int64_t n) {
     const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (s >= n) return;
-    const float ob = __ldg(out_bar + s);
-    if (ob == 0.f) return;
-    int i, j, k;
-    coords_at(t, s, i, j, k);
-    const float3 vc = make_float3(__ldg(vel + 3 * s), __ldg(vel + 3 * s + 1), __ldg(vel + 3 * s + 2));
+    float v[kFields];
+#pragma unroll
+    for (int c = 0; c < kFields; ++c) v[c] = c < F.count ? __ldg(F.d[c] + s) : 0.f;
+    in4[s] = make_float4(v[0], v[1], v[2], v[3]);
+    vel_in4[s] = make_float4(__ldg(vel + 3 * s), __ldg(vel + 3 * s + 1), __ldg(vel + 3 * s + 2), v[4]);
+}
+
+__device__ __forceinline__ float comp(const float4& a, const float4& b, int c) {
+    return c == 0 ? a.x : c == 1 ? a.y : c == 2 ? a.z : c == 3 ? a.w : b.w;
+}
+
+// Adjoint of advect_scalars for all fields along vel (the projected velocity), one thread per
+// voxel: the trace, the taps and their weights are computed once for all fields, and the position
+// adjoints of every field are summed before they are scattered to the velocity.
+//   d_bar += (d out / d d)^T out_bar,  vel_bar += (d out / d vel)^T out_bar.
+// Bound by the scatters' L2 atomics and the taps' gathers, so both go by records of 16 bytes: in4
+// and vel_in4 hold the gathered fields (pack_records_kernel), rec4 one float4 per slot that
+// receives the adjoints of fields 0..3 of a tap in one vector reduction, vel4 the three velocity
+// components and field 4; fold_records_kernel adds both into the caller's arrays. Weights and
+// slots as setupInterpolation (src/Cuda/Kernel.cu:204-233) computes them in the forward
+// (interp_setup_fast, x fastest in the tap index), an out-of-domain tap reading slot 0. Slot 0
+// takes the adjoints of all of those taps, one after the other on one address, which is most of
+// what is left: the records make it one reduction per tap for all fields where each field's
+// launch queued by itself. (Summing them per warp first takes 5 ms less but sums them in another
+// order, up to 9e-4 away from the sums of one tap at a time.) On a 28,103-leaf grid with four
+// fields 45.7 ms in four launches -> 8 ms.
+template <typename I>
+__global__ void __launch_bounds__(kThreads, 2) adj_advect_scalars_kernel(TopoView t, AdvectedBars F,
+                                                                      const float4* __restrict__ in4,
+                                                                      const float4* __restrict__ vel_in4,
+                                                                      float4* __restrict__ rec4,
+                                                                      float4* __restrict__ vel4, float sdt) {
+    __shared__ dev::LeafNbhd L;
+    const dev::VoxelIdx vx = dev::voxel_of_block();
+    dev::load_nbhd(L, t, vx.leaf);
+    __syncthreads();
+    const int i = (L.lx << 3) + (vx.n >> 6), j = (L.ly << 3) + ((vx.n >> 3) & 7), k = (L.lz << 3) + (vx.n & 7);
+    const int64_t s = (vx.leaf << 9) + vx.n;
+    const float4 vc = __ldg(vel_in4 + s), dc = __ldg(in4 + s);
     const float bx = (float)i - vc.x * sdt, by = (float)j - vc.y * sdt, bz = (float)k - vc.z * sdt;
-    WTaps tb, tf;
-    wtaps(t, bx, by, bz, tb);
+    I bs[8], fs[8];
+    float bw[8], fw[8];
+    dev::interp_setup_fast(t, L, bx, by, bz, bs, bw);
+    float pf[kFields] = {}, pb[kFields] = {};
     float3 vf = make_float3(0.f, 0.f, 0.f);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const int64_t r = tb.s[q];
-        vf.x = vf.x + __ldg(vel + 3 * r) * tb.w[q];
-        vf.y = vf.y + __ldg(vel + 3 * r + 1) * tb.w[q];
-        vf.z = vf.z + __ldg(vel + 3 * r + 2) * tb.w[q];
+        const float4 a = __ldg(vel_in4 + bs[q]), d = __ldg(in4 + bs[q]);
+        vf.x = vf.x + a.x * bw[q];
+        vf.y = vf.y + a.y * bw[q];
+        vf.z = vf.z + a.z * bw[q];
+#pragma unroll
+        for (int c = 0; c < kFields; ++c) pf[c] = __fmaf_rn(comp(d, a, c), bw[q], pf[c]);
     }
-    wtaps(t, bx + vf.x * sdt, by + vf.y * sdt, bz + vf.z * sdt, tf);
-    const float po = __ldg(d + s);
-    float pf = 0.f, pb = 0.f;
-    float3 gpf = make_float3(0.f, 0.f, 0.f), gpb = make_float3(0.f, 0.f, 0.f);
+    const float fx = bx + vf.x * sdt, fy = by + vf.y * sdt, fz = bz + vf.z * sdt;
+    dev::interp_setup_fast(t, L, fx, fy, fz, fs, fw);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const float a = __ldg(d + tb.s[q]), b = __ldg(d + tf.s[q]);
-        pf = __fmaf_rn(a, tb.w[q], pf);
-        pb = __fmaf_rn(b, tf.w[q], pb);
-        gpf.x += a * tb.gx[q], gpf.y += a * tb.gy[q], gpf.z += a * tb.gz[q];
-        gpb.x += b * tf.gx[q], gpb.y += b * tf.gy[q], gpb.z += b * tf.gz[q];
+        const float4 d = __ldg(in4 + fs[q]);
+        const float w = F.count > 4 ? __ldg(&vel_in4[fs[q]].w) : 0.f;
+#pragma unroll
+        for (int c = 0; c < kFields; ++c) pb[c] = __fmaf_rn(c < 4 ? comp(d, d, c) : w, fw[q], pb[c]);
     }
-    const float corr = __fmaf_rn(0.5f, po - pb, pf);
-    // The clamp set in the forward's order: centre, x-1, x+1, y-1, y+1, z-1, z+1, the forward sample.
-    const int64_t ns[6] = {slot0(t, i - 1, j, k), slot0(t, i + 1, j, k), slot0(t, i, j - 1, k),
-                           slot0(t, i, j + 1, k), slot0(t, i, j, k - 1), slot0(t, i, j, k + 1)};
-    float mn = po, mx = po;
-    int imn = -2, imx = -2;  // -2 centre, 0..5 a neighbour, 6 the forward sample
+    // The clamp: which value of {centre, x-1, x+1, y-1, y+1, z-1, z+1, the forward sample}, in the
+    // forward's order, the output is, and so where its adjoint goes.
+    I ns[6];
+    dev::face_slots(L, (I)s, vx.n, ns);
+    float mn[kFields], mx[kFields];
+    int imn[kFields], imx[kFields];  // -2 centre, 0..5 a neighbour, 6 the forward sample
+#pragma unroll
+    for (int c = 0; c < kFields; ++c) mn[c] = mx[c] = comp(dc, vc, c), imn[c] = imx[c] = -2;
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-        const float a = __ldg(d + ns[q]);
-        if (a < mn) mn = a, imn = q;
-        if (a > mx) mx = a, imx = q;
-    }
-    if (pf < mn) mn = pf, imn = 6;
-    if (pf > mx) mx = pf, imx = 6;
-    const int pick = corr > mx ? imx : corr < mn ? imn : -1;
-    float g_po = 0.f, g_pf = 0.f, g_pb = 0.f;
-    if (pick == -1) {
-        g_pf = ob, g_po = 0.5f * ob, g_pb = -0.5f * ob;
-    } else if (pick == -2) {
-        g_po = ob;
-    } else if (pick == 6) {
-        g_pf = ob;
-    } else {
-        atomicAdd(d_bar + ns[pick], ob);
-    }
-    if (g_po != 0.f) atomicAdd(d_bar + s, g_po);
+        ns[q] = ns[q] < 0 ? I(0) : ns[q];
+        const float4 d = __ldg(in4 + ns[q]);
+        const float w = F.count > 4 ? __ldg(&vel_in4[ns[q]].w) : 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        if (g_pf != 0.f) atomicAdd(d_bar + tb.s[q], g_pf * tb.w[q]);
-        if (g_pb != 0.f) atomicAdd(d_bar + tf.s[q], g_pb * tf.w[q]);
-    }
-    // Positions: pf at back, pb at fwd = back + vf(back) sdt, back = x - vc sdt.
-    const float3 fb = make_float3(g_pb * gpb.x, g_pb * gpb.y, g_pb * gpb.z);
-    float3 bb = make_float3(g_pf * gpf.x + fb.x, g_pf * gpf.y + fb.y, g_pf * gpf.z + fb.z);
-    const float3 vfb = make_float3(fb.x * sdt, fb.y * sdt, fb.z * sdt);
-    if (vfb.x != 0.f || vfb.y != 0.f || vfb.z != 0.f) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int64_t r = tb.s[q];
-            atomicAdd(vel_bar + 3 * r, vfb.x * tb.w[q]);
-            atomicAdd(vel_bar + 3 * r + 1, vfb.y * tb.w[q]);
-            atomicAdd(vel_bar + 3 * r + 2, vfb.z * tb.w[q]);
-            const float ux = __ldg(vel + 3 * r), uy = __ldg(vel + 3 * r + 1), uz = __ldg(vel + 3 * r + 2);
-            const float dv = vfb.x * ux + vfb.y * uy + vfb.z * uz;
-            bb.x += dv * tb.gx[q], bb.y += dv * tb.gy[q], bb.z += dv * tb.gz[q];
+        for (int c = 0; c < kFields; ++c) {
+            const float a = c < 4 ? comp(d, d, c) : w;
+            if (a < mn[c]) mn[c] = a, imn[c] = q;
+            if (a > mx[c]) mx[c] = a, imx[c] = q;
         }
     }
-    if (bb.x != 0.f) atomicAdd(vel_bar + 3 * s, -sdt * bb.x);
-    if (bb.y != 0.f) atomicAdd(vel_bar + 3 * s + 1, -sdt * bb.y);
-    if (bb.z != 0.f) atomicAdd(vel_bar + 3 * s + 2, -sdt * bb.z);
+    float gpf[kFields] = {}, gpb[kFields] = {}, own[kFields] = {};
+#pragma unroll
+    for (int c = 0; c < kFields; ++c) {
+        const float ob = c < F.count ? __ldg(F.out_bar[c] + s) : 0.f;
+        const float corr = __fmaf_rn(0.5f, comp(dc, vc, c) - pb[c], pf[c]);
+        if (pf[c] < mn[c]) mn[c] = pf[c], imn[c] = 6;
+        if (pf[c] > mx[c]) mx[c] = pf[c], imx[c] = 6;
+        const int pick = corr > mx[c] ? imx[c] : corr < mn[c] ? imn[c] : -1;
+        if (pick == -1) {
+            gpf[c] = ob, own[c] = 0.5f * ob, gpb[c] = -0.5f * ob;
+        } else if (pick == -2) {
+            own[c] = ob;
+        } else if (pick == 6) {
+            gpf[c] = ob;
+        } else if (ob != 0.f) {
+            I at = ns[0];
+#pragma unroll
+            for (int q = 1; q < 6; ++q) at = pick == q ? ns[q] : at;
+            atomicAdd(c < 4 ? reinterpret_cast<float*>(rec4 + at) + c : &vel4[at].w, ob);
+        }
+    }
+    // Positions: pf at back, pb at fwd = back + vf(back) sdt, back = x - vc sdt. A weight's
+    // derivative in x is +-wy wz. The adjoint of a sample's position is the sum over its taps of
+    // (the fields' adjoints . the tap's values) times the weight's gradient.
+    auto grad = [](float x, float y, float z, int q) {
+        const float tx = x - (float)__float2int_rd(x), ty = y - (float)__float2int_rd(y), tz = z - (float)__float2int_rd(z);
+        const float wx = (q & 1) ? tx : 1.0f - tx, wy = (q & 2) ? ty : 1.0f - ty, wz = (q & 4) ? tz : 1.0f - tz;
+        return make_float3(((q & 1) ? wy : -wy) * wz, ((q & 2) ? wx : -wx) * wz, ((q & 4) ? wx : -wx) * wy);
+    };
+    const bool fwd = gpb[0] != 0.f || gpb[1] != 0.f || gpb[2] != 0.f || gpb[3] != 0.f || gpb[4] != 0.f;
+    const bool back = gpf[0] != 0.f || gpf[1] != 0.f || gpf[2] != 0.f || gpf[3] != 0.f || gpf[4] != 0.f;
+    float3 fb = make_float3(0.f, 0.f, 0.f), bb = make_float3(0.f, 0.f, 0.f);
+    if (fwd) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float4 d = __ldg(in4 + fs[q]);
+            float a = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) a += gpb[c] != 0.f ? gpb[c] * comp(d, d, c) : 0.f;
+            if (gpb[4] != 0.f) a += gpb[4] * __ldg(&vel_in4[fs[q]].w);
+            const float3 w = grad(fx, fy, fz, q);
+            fb.x += a * w.x, fb.y += a * w.y, fb.z += a * w.z;
+            const float m = fw[q];
+            dev::red4(rec4 + fs[q], gpb[0] * m, gpb[1] * m, gpb[2] * m, gpb[3] * m);
+            if (gpb[4] != 0.f) atomicAdd(&vel4[fs[q]].w, gpb[4] * m);
+        }
+    }
+    const float3 vfb = make_float3(fb.x * sdt, fb.y * sdt, fb.z * sdt);
+    const bool trace = vfb.x != 0.f || vfb.y != 0.f || vfb.z != 0.f;
+    if (back || trace) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float4 u = __ldg(vel_in4 + bs[q]), d = __ldg(in4 + bs[q]);
+            float a = trace ? vfb.x * u.x + vfb.y * u.y + vfb.z * u.z : 0.f;
+#pragma unroll
+            for (int c = 0; c < kFields; ++c) a += gpf[c] != 0.f ? gpf[c] * comp(d, u, c) : 0.f;
+            const float3 w = grad(bx, by, bz, q);
+            bb.x += a * w.x, bb.y += a * w.y, bb.z += a * w.z;
+            const float m = bw[q];
+            if (back) dev::red4(rec4 + bs[q], gpf[0] * m, gpf[1] * m, gpf[2] * m, gpf[3] * m);
+            if (trace || gpf[4] != 0.f) dev::red4(vel4 + bs[q], vfb.x * m, vfb.y * m, vfb.z * m, gpf[4] * m);
+        }
+    }
+    bb.x += fb.x, bb.y += fb.y, bb.z += fb.z;
+    dev::red4(rec4 + s, own[0], own[1], own[2], own[3]);
+    dev::red4(vel4 + s, -sdt * bb.x, -sdt * bb.y, -sdt * bb.z, own[4]);
+}
+
+// Adds the records of adj_advect_scalars_kernel into the fields' and the velocity's adjoints.
+__global__ void __launch_bounds__(kThreads) fold_records_kernel(AdvectedBars F, const float4* __restrict__ rec4,
+                                                                const float4* __restrict__ vel4,
+                                                                float* __restrict__ vel_bar, int64_t n) {
+    const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (s >= n) return;
+    const float4 a = __ldg(rec4 + s), b = __ldg(vel4 + s);
+    const float v[kFields] = {a.x, a.y, a.z, a.w, b.w};
+#pragma unroll
+    for (int c = 0; c < kFields; ++c)
+        if (c < F.count) F.d_bar[c][s] += v[c];
+    vel_bar[3 * s] += b.x;
+    vel_bar[3 * s + 1] += b.y;
+    vel_bar[3 * s + 2] += b.z;
 }
 
 // s1 = s + dt src (add_scalar_source, out of place; the forward's arithmetic).
@@ -266,11 +319,17 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
     const float* srcs[kFields] = {src.density, src.temperature, src.fuel, nullptr, nullptr};
     static const char* nm[kFields] = {"density", "temperature", "fuel", "waste", "flame"};
 
+    // One scratch block of 16 n floats whose parts the phases use in turn: the forward's adv2, adv3
+    // and div; the scalar advection's records; then p_bar, div_bar, the velocity's adjoints and the
+    // self-advection's records. Fewer bytes to allocate on a grid's first pass, which costs more
+    // than the pass itself.
+    float* arena = sf(c, "arena", 16 * n);
+
     // ---- the forward, recomputed ----
     float* adv = sf(c, "adv", 3 * n);
-    float* adv2 = sf(c, "adv2", 3 * n);
-    float* adv3 = sf(c, "adv3", 3 * n);
-    float* div = sf(c, "div", n);
+    float* adv2 = arena;
+    float* adv3 = arena + 3 * n;
+    float* div = arena + 6 * n;
     FieldSet none{};
     launch_advect_fused(c, in.velocity, adv, none, dt);
     launch_confine_sources(c, adv, adv2, dt, P.vorticityScale, P.factorScale, src.velocity, P.gravity);
@@ -305,19 +364,40 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
     float* vb = sf(c, "vb", 3 * n);
     HNS_CUDA(cudaMemcpyAsync(vb, out_bar.velocity, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
     float* mid[kFields] = {};
+    AdvectedBars bars{};
     for (int f = 0; f < kFields; ++f) {
         if (!sin[f]) continue;
         mid[f] = sf(c, std::string("mid_") + nm[f], n);
         HNS_CUDA(cudaMemsetAsync(mid[f], 0, n * sizeof(float), c.stream));
-        if (sbar_out[f]) {
-            adj_advect_scalars_kernel<<<blocks_for(nn), kThreads, 0, c.stream>>>(c.topo.view, velp, s2[f], sbar_out[f],
-                                                                                 mid[f], vb, dt * (1.0f / c.dx), nn);
-            HNS_LAUNCHED();
-        }
+        if (!sbar_out[f]) continue;
+        bars.d[bars.count] = s2[f];
+        bars.out_bar[bars.count] = sbar_out[f];
+        bars.d_bar[bars.count] = mid[f];
+        ++bars.count;
+    }
+    if (bars.count > 0) {
+        auto* rec4 = reinterpret_cast<float4*>(arena);
+        auto* vel4 = reinterpret_cast<float4*>(arena + 4 * n);
+        auto* in4 = reinterpret_cast<float4*>(arena + 8 * n);
+        auto* vel_in4 = reinterpret_cast<float4*>(arena + 12 * n);
+        pack_records_kernel<<<blocks_for(nn), kThreads, 0, c.stream>>>(bars, velp, in4, vel_in4, nn);
+        HNS_LAUNCHED();
+        HNS_CUDA(cudaMemsetAsync(rec4, 0, 8 * n * sizeof(float), c.stream));  // rec4 and vel4
+        const float sdt = dt * (1.0f / c.dx);
+        const unsigned blocks = (unsigned)(2 * c.topo.num_leaves);
+        if (c.topo.num_leaves < (int64_t(1) << 22))
+            adj_advect_scalars_kernel<int32_t><<<blocks, kThreads, 0, c.stream>>>(c.topo.view, bars, in4, vel_in4, rec4,
+                                                                                  vel4, sdt);
+        else
+            adj_advect_scalars_kernel<int64_t><<<blocks, kThreads, 0, c.stream>>>(c.topo.view, bars, in4, vel_in4, rec4,
+                                                                                  vel4, sdt);
+        HNS_LAUNCHED();
+        fold_records_kernel<<<blocks_for(nn), kThreads, 0, c.stream>>>(bars, rec4, vel4, vb, nn);
+        HNS_LAUNCHED();
     }
     // The projection: vel' = adv3 - grad p, p = M div.
-    float* pbar = sf(c, "pbar", n);
-    float* dbar = sf(c, "dbar", n);
+    float* pbar = arena;
+    float* dbar = arena + n;
     HNS_CUDA(cudaMemsetAsync(pbar, 0, n * sizeof(float), c.stream));
     HNS_CUDA(cudaMemsetAsync(dbar, 0, n * sizeof(float), c.stream));
     launch_adj_gradient(c, vb, pbar);
@@ -328,10 +408,10 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
                              S.refined->flags);
         convert_array(c, p64, HNS_DTYPE_F64, dbar, HNS_DTYPE_F32, nn);
     } else {
-        adj_rbgs(c, pbar, dbar, S.iterations, S.omega);
+        adj_rbgs(c, pbar, dbar, S.iterations, S.omega, arena + 8 * n);
     }
     // adv2_bar = adv3_bar (the buoyancy adds to adv2) + D^T div_bar.
-    float* adv2b = sf(c, "adv2b", 3 * n);
+    float* adv2b = arena + 2 * n;
     HNS_CUDA(cudaMemcpyAsync(adv2b, vb, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
     launch_adj_divergence(c, dbar, adv2b);
     // Burn, buoyancy and sources, per voxel.
@@ -356,10 +436,10 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
             M.density_buoyancy, dt, P.ambientTemp, P.buoyancyStrength, nn);
     HNS_LAUNCHED();
     // Confinement and the velocity's self-advection.
-    float* advb = sf(c, "advb", 3 * n);
+    float* advb = arena + 5 * n;
     HNS_CUDA(cudaMemsetAsync(advb, 0, 3 * n * sizeof(float), c.stream));
     launch_adj_confinement(c, adv, adv2b, advb, dt, P.vorticityScale, P.factorScale);
-    launch_adj_advect_vec3(c, in.velocity, advb, in_bar.velocity, dt);
+    launch_adj_advect(c, in.velocity, advb, nullptr, nullptr, nullptr, 0, in_bar.velocity, dt, arena + 8 * n);
 }
 
 }  // namespace hns

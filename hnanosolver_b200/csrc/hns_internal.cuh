@@ -358,17 +358,20 @@ void launch_rbgs_bulk_unit(const Context& c, const float* rhs, const float* e_in
                            const double* check, double tol2);
 
 // ---- adjoints (hns_adjoint.cu): each adds its transpose into the adjoint arrays ----
-void launch_adj_advect_scalar(const Context& c, const float* vel, const float* in, const float* out_bar, float* in_bar,
-                              float* vel_bar, float dt);
-void launch_adj_advect_vec3(const Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt);
+// The advections along vel: of the velocity (vel_out_bar, null: not advected) and of nscalars
+// scalars. work: 8 floats per voxel of scratch (null: the context's).
+void launch_adj_advect(Context& c, const float* vel, const float* vel_out_bar, const float* const* in,
+                       const float* const* out_bar, float* const* in_bar, int nscalars, float* vel_bar, float dt,
+                       float* work = nullptr);
 void launch_adj_divergence(const Context& c, const float* div_bar, float* vel_bar);
 void launch_adj_gradient(const Context& c, const float* out_bar, float* p_bar);
 void launch_adj_rbgs_colour(const Context& c, float* lam, float* div_bar, int colour, float keep, float nbr, float dmul);
 void launch_adj_confinement(const Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt,
                             float scale, float factor_scale);
 void launch_adj_accumulate(const Context& c, const float* src, float* dst, int64_t n);
-// div_bar += M^T p_bar for `iterations` red-black iterations from p = 0 (p = M div).
-void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, float omega);
+// div_bar += M^T p_bar for `iterations` red-black iterations from p = 0 (p = M div). lam: n floats
+// of scratch (null: the context's).
+void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, float omega, float* lam = nullptr);
 
 // ---- mixed precision and refinement (hns_mixed.cu) ----
 void convert_array(const Context& c, const void* src, int src_dt, void* dst, int dst_dt, int64_t n);

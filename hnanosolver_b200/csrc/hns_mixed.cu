@@ -596,6 +596,8 @@ bool capturing(const Context& c) {
     return st != cudaStreamCaptureStatusNone;
 }
 
+constexpr size_t kMaxSpareGraphs = 64;
+
 // Condition of a spare outer iteration's graph: 1 while the refinement has not converged (the
 // test every kernel of the iteration makes before it does anything).
 __global__ void spare_gate_kernel(cudaGraphConditionalHandle h, const double* __restrict__ check, double tol2) {
@@ -614,7 +616,10 @@ bool run_spare_graph(Context& c, const std::vector<uintptr_t>& key, const double
     for (auto& g : c.spare_graphs)
         if (g.key == key) found = &g;
     if (found == nullptr) {
-        if (c.spare_graphs.size() >= 16) c.release_spare_graphs();
+        // Bounded: a step's one or two solves have at most max_outer - 1 spare iterations each. At 16
+        // graphs the two solves of the fire adjoint (11 each) released and made them anew on every
+        // call, 10 ms of host time a call on a 28,103-leaf grid.
+        if (c.spare_graphs.size() >= kMaxSpareGraphs) c.release_spare_graphs();
         Context::SpareGraph sg;
         sg.key = key;
         bool ok = cudaGraphCreate(&sg.graph, 0) == cudaSuccess;

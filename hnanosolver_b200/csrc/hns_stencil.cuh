@@ -319,6 +319,12 @@ __device__ __forceinline__ void collide(const TopoView& t, const LeafNbhd& L, co
     }
 }
 
+// *p += (x, y, z, w) as one 16-byte vector reduction in L2.
+__device__ __forceinline__ void red4(float4* p, float x, float y, float z, float w) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w)
+                 : "memory");
+}
+
 // Voxel handled by this thread in the "two CTAs per leaf" kernels.
 struct VoxelIdx {
     int64_t leaf;
