@@ -536,6 +536,10 @@ float* adj_scratch(Context& c) { return c.scratch_f32("adjoint_work", 8 * (size_
 // to the initial p is not needed (p starts at 0), so lam is never rescaled at the end.
 void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, float omega, float* lam) {
     if (iterations <= 0) return;
+    if (use_chip(c, 2 * iterations) && aligned16(p_bar) && aligned16(div_bar) && chip_fits(c, sizeof(float), true)) {
+        launch_chip_transpose(c, c.split_faces(), p_bar, div_bar, iterations, omega);
+        return;
+    }
     const size_t n = (size_t)c.num_voxels();
     if (lam == nullptr) lam = adj_scratch(c);
     HNS_CUDA(cudaMemcpyAsync(lam, p_bar, n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));

@@ -260,6 +260,12 @@ void rbgs_solve(Context& c, const float* div, float* p, int iterations, float om
         split32_solve(c, div, p, iterations, omega, flags, nullptr);
         return;
     }
+    if ((flags & HNS_SOLVE_NEUMANN) && c.rbgs_kernel == HNS_RBGS_SPLIT && use_chip(c, 2 * iterations) && aligned16(div) &&
+        aligned16(p) && chip_fits(c, sizeof(float), true)) {
+        launch_chip_solve_f32(c, c.split_faces(), div, true, p, true, 2 * iterations, (flags & HNS_SOLVE_ZERO_INIT) != 0, omega,
+                              c.dx * c.dx, true, nullptr, nullptr, 0, 0.0);
+        return;
+    }
     const size_t n = (size_t)c.num_voxels();
     float* tmp = c.scratch_f32("rbgs_pingpong", n);
     // Ping-pong so that the last iteration writes into p.
@@ -448,7 +454,7 @@ HNS_API hns_status hns_set_option(hns_ctx* ctx, int option, int value) {
                 fail(HNS_ERR_INVALID_ARG, "unknown inner layout");
             c->inner_layout = value;
         } else if (option == HNS_OPT_SPLIT_SOLVE) {
-            if (value != HNS_SPLIT_PER_COLOUR && value != HNS_SPLIT_PERSISTENT)
+            if (value != HNS_SPLIT_PER_COLOUR && value != HNS_SPLIT_PERSISTENT && value != HNS_SPLIT_AUTO)
                 fail(HNS_ERR_INVALID_ARG, "unknown inner-solve launch form");
             c->split_solve = value;
         } else if (option == HNS_OPT_COARSE_SOLVE) {

@@ -175,7 +175,9 @@ struct Context {
     int rbgs_kernel = HNS_RBGS_SPLIT;     // hns_set_option(HNS_OPT_RBGS_KERNEL)
     int inner_layout = HNS_INNER_SPLIT;  // hns_set_option(HNS_OPT_INNER_LAYOUT)
     int first_wait_polls = -1;           // hns_set_option(HNS_OPT_WAIT_POLLS); -1: the kernel's default
-    int split_solve = HNS_SPLIT_PER_COLOUR;  // hns_set_option(HNS_OPT_SPLIT_SOLVE)
+    int split_solve = HNS_SPLIT_AUTO;    // hns_set_option(HNS_OPT_SPLIT_SOLVE)
+    uint32_t chip_tag = 1;       // the next launch's first tag (hns_rbgs_chip.cu)
+    bool chip_words_clear = false;  // its face words have been cleared
     int coarse_solve = HNS_COARSE_CLUSTER;   // hns_set_option(HNS_OPT_COARSE_SOLVE)
     int l2_persist = 1;                      // hns_set_option(HNS_OPT_L2_PERSIST)
     // The access-policy window of the inner solve's launches while a refined solve runs
@@ -254,6 +256,8 @@ struct DeviceGuard {
 
 Context* check_ctx(hns_ctx* ctx);
 const Context* check_ctx(const hns_ctx* ctx);
+
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- kernels (hns_kernels.cu) --------------------------------------------------------------
 
@@ -345,6 +349,25 @@ void launch_rbgs_split_solve_f32(Context& c, const int* nb8, const float* rhs, f
 void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* rhs, float* e, int colour, bool e_zero,
                                 float omega, float dx2, const double* check, double tol2, bool short_grid = false,
                                 bool pdl = true);
+// The solve held in the SMs' shared memory (hns_rbgs_chip.cu): `half_sweeps` half-sweeps (red
+// first) in one cooperative launch, the values of the launch-per-colour kernels to the bit.
+// chip_fits: whether the grid's values of `bytes` each fit, in_place_slots with their right-hand
+// side (needed where the right-hand side is in slot order). walls: zero-gradient walls. The launch
+// does nothing when `check` has passed, and ends before half-sweep mid_half when check_mid has.
+bool chip_fits(const Context& c, size_t bytes, bool in_place_slots);
+void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,
+                           int half_sweeps, bool e_zero, float omega, float dx2, bool walls, const double* check,
+                           const double* check_mid, int mid_half, double tol2);
+void launch_chip_solve_f16(Context& c, const int* nb8, const void* rhs, void* e, int half_sweeps, bool e_zero, float omega,
+                           const double* check, double tol2);
+// div_bar += M^T p_bar (adj_rbgs) on the chip; both 16-byte aligned.
+void launch_chip_transpose(Context& c, const int* nb8, const float* p_bar, float* div_bar, int iterations, float omega);
+// Solves of fewer half-sweeps launch per colour: loading and storing the values costs the chip's
+// launch about what four half-sweep launches cost.
+constexpr int kChipMinHalfSweeps = 8;
+inline bool use_chip(const Context& c, int half_sweeps) {
+    return c.split_solve == HNS_SPLIT_AUTO && half_sweeps >= kChipMinHalfSweeps && c.topo.num_leaves < (int64_t(1) << 22);
+}
 // FP32 slot order <-> colour-split order (n values).
 void convert_split_f32(const Context& c, const float* src, float* dst, bool to_split);
 // acc += {sum r^2, sum b^2} of the FP32 split iterate e (FP64), unless check has passed.

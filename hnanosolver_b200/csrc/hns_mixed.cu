@@ -917,8 +917,17 @@ RefinePlan refine_solve(Context& c, const float* div, double* p, int max_outer, 
         // The persistent form: the whole inner solve in one launch. An outer iteration past the
         // forecast takes it whatever the option: it most likely returns at once, and one launch
         // then costs a few microseconds where 2 * inner returning half-sweeps cost 2.3 us each.
-        const bool persistent = layout == HNS_INNER_SPLIT && (c.split_solve == HNS_SPLIT_PERSISTENT || spare);
-        if (persistent) {
+        // Where the values fit the SMs' shared memory, the solve held there (hns_rbgs_chip.cu).
+        const bool chip = layout == HNS_INNER_SPLIT && use_chip(c, 2 * plan.inner) && chip_fits(c, sizeof(TI), false);
+        const bool persistent = layout == HNS_INNER_SPLIT && (c.split_solve == HNS_SPLIT_PERSISTENT || spare || chip);
+        if (chip) {
+            if constexpr (sizeof(TI) == 2)
+                launch_chip_solve_f16(c, nb8, rhat, e_split, 2 * plan.inner, true, omega, chk, tol2);
+            else
+                launch_chip_solve_f32(c, nb8, reinterpret_cast<const float*>(rhat), false, reinterpret_cast<float*>(e_split),
+                                      false, 2 * plan.inner, true, omega, 1.0f, false, chk, nullptr, 0, tol2);
+            src = e_split;
+        } else if (persistent) {
             if constexpr (sizeof(TI) == 2)
                 launch_rbgs_split_solve(c, nb8, rhat, e_split, 2 * plan.inner, true, omega, chk, tol2);
             else

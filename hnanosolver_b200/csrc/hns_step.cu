@@ -35,10 +35,23 @@ Split32 split32_workspace(Context& c) {
 // before iteration (c + 1) E - 1 into its slot and every later half-sweep tests the latest slot,
 // the schedule of the staged kernel (rbgs_solve_checked), so both give the same iterates.
 void split32_solve(Context& c, const float* div, float* p, int K, float omega, unsigned flags, const SolvePlan* plan) {
-    const Split32 w = split32_workspace(c);
     const float dx2 = c.dx * c.dx;
-    convert_split_f32(c, div, w.rhs, true);
     const bool zero = (flags & HNS_SOLVE_ZERO_INIT) != 0;
+    if (plan == nullptr && use_chip(c, 2 * K) && chip_fits(c, sizeof(float), false)) {
+        // The whole solve in one launch, p in and out in slot order; the divergence too where it is
+        // held on the chip, else it is streamed in the split layout.
+        const bool held = chip_fits(c, sizeof(float), true);
+        const float* rhs = div;
+        if (!held) {
+            float* s = c.scratch_f32("split32_rhs", (size_t)c.num_voxels());
+            convert_split_f32(c, div, s, true);
+            rhs = s;
+        }
+        launch_chip_solve_f32(c, c.split_faces(), rhs, held, p, true, 2 * K, zero, omega, dx2, false, nullptr, nullptr, 0, 0.0);
+        return;
+    }
+    const Split32 w = split32_workspace(c);
+    convert_split_f32(c, div, w.rhs, true);
     if (!zero) convert_split_f32(c, p, w.e, true);
     const double tol2 = plan ? plan->tol * plan->tol : 0.0;
     if (c.split_solve == HNS_SPLIT_PERSISTENT) {
@@ -60,6 +73,24 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
                 }
             }
             launch_rbgs_split_solve_f32(c, w.nb8, w.rhs, w.e, 2 * (end - it), zero && it == 0, omega, dx2, chk, tol2);
+            it = end;
+        }
+        convert_split_f32(c, w.e, p, false);
+        return;
+    }
+    if (plan != nullptr && use_chip(c, 2 * plan->check_every) && chip_fits(c, sizeof(float), false)) {
+        // One launch from each residual evaluation to the next: iteration (c + 1) E - 1, which tests
+        // the check before it, and from the second iteration on the check just evaluated.
+        const int E = plan->check_every;
+        for (int it = 0; it < K;) {
+            const int q = it / E - 1;  // the check tested by iteration `it`
+            const bool eval = (it + 1) % E == 0;
+            const double* chk = q >= 0 ? plan->slots + 2 * q : nullptr;
+            double* next = eval ? plan->slots + 2 * (q + 1) : nullptr;
+            if (eval) launch_split_residual_f32(c, w.nb8, w.rhs, w.e, (double)dx2, chk, tol2, next);
+            const int end = std::min(K, eval ? it + E : E - 1);
+            launch_chip_solve_f32(c, w.nb8, w.rhs, false, w.e, false, 2 * (end - it), zero && it == 0, omega, dx2, false, chk,
+                                  next, 2, tol2);
             it = end;
         }
         convert_split_f32(c, w.e, p, false);
