@@ -5,19 +5,19 @@
 // (src/Cuda/HNanoSolver.cu:498-504). The solver's grids are leaf-dense, so the build produces
 // the set of leaves that the dilated voxels touch, in NanoVDB leaf order, and the leaf tables.
 //
-//   1. Per voxel: its leaf's 63-bit key, which both identifies the leaf and sorts in NanoVDB
-//      order (root tile, then upper-node child, then lower-node child; PointsToGrid orders
-//      leaves this way), and a 27-bit mask of the neighbour leaves its dilation box reaches
-//      (per axis: -1 when z & 7 < padding, +1 when (z & 7) + padding >= 8).
-//   2. Radix sort of (key, mask) pairs, reduce-by-key with OR: the active leaves and the
-//      union of their reach masks.
-//   3. Each active leaf emits the keys of the leaves its mask names; sort and unique: the
-//      dilated leaf set, already in NanoVDB order.
-//   4. Leaf origins from the keys, the dense leaf table and the 27-neighbour table, on the
-//      device; only the origins go back to the host (the context keeps a host copy).
-// Library primitives (CUB radix sort, scan, reduce-by-key, unique) do the sorting; this is the
-// set-up before the step, not the step's hot path.
-#include <cub/cub.cuh>
+//   1. The voxels' bounding box (and the check of their range): one read of the list.
+//   2. A flag per leaf of the dilated bounding box, in the leaf lookup table that the grid needs
+//      anyway: per voxel the leaves its dilation box reaches (per axis: -1 when z & 7 < padding,
+//      +1 when (z & 7) + padding >= 8), found once per warp where its voxels share a leaf.
+//   3. NanoVDB leaf order is root tile, then upper-node child, then lower-node child, each in
+//      x, y, z order (PointsToGrid orders leaves this way). A lower node is 16^3 leaves, so the flags
+//      are counted and then numbered node by node, the nodes in that order: one CTA per node of
+//      the box, no sort.
+//   4. Leaf origins and the table entries as the leaves are numbered, then the 27-neighbour table;
+//      only the origins go back to the host (the context keeps a host copy).
+// Bound by the two reads of the voxel list and by the call's allocations and three host waits: the
+// band of a 512^3 shell (12M voxels, padding 2, 46,000 leaves), context made and destroyed, took
+// 8.7 ms with a radix sort of one key per voxel (1.4 ms of kernels, 300 MB of temporary arrays).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,86 +38,179 @@ constexpr int kMaxPadding = 8;
 
 unsigned grid_for(int64_t n) { return (unsigned)((n + kTopoThreads - 1) / kTopoThreads); }
 
-__device__ __forceinline__ uint64_t leaf_key(int i, int j, int k) {
-    const uint64_t rx = (uint64_t)((i >> 12) + 2048), ry = (uint64_t)((j >> 12) + 2048), rz = (uint64_t)((k >> 12) + 2048);
-    return (rx << 51) | (ry << 39) | (rz << 27) | ((uint64_t)((i >> 7) & 31) << 22) | ((uint64_t)((j >> 7) & 31) << 17) |
-           ((uint64_t)((k >> 7) & 31) << 12) | ((uint64_t)((i >> 3) & 15) << 8) | ((uint64_t)((j >> 3) & 15) << 4) |
-           (uint64_t)((k >> 3) & 15);
-}
-
-__device__ __forceinline__ int3 key_origin(uint64_t key) {
-    const int rx = (int)((key >> 51) & 4095) - 2048, ry = (int)((key >> 39) & 4095) - 2048,
-              rz = (int)((key >> 27) & 4095) - 2048;
-    const int ux = (int)((key >> 22) & 31), uy = (int)((key >> 17) & 31), uz = (int)((key >> 12) & 31);
-    const int lx = (int)((key >> 8) & 15), ly = (int)((key >> 4) & 15), lz = (int)(key & 15);
-    return make_int3(rx * 4096 + ux * 128 + lx * 8, ry * 4096 + uy * 128 + ly * 8, rz * 4096 + uz * 128 + lz * 8);
-}
-
-// Step 1. bad[0] is set when a coordinate is out of range.
-__global__ void voxel_key_kernel(const int32_t* __restrict__ ijk, int64_t n, int padding, uint64_t* __restrict__ keys,
-                                 uint32_t* __restrict__ masks, int* __restrict__ bad) {
-    const int64_t q = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
-    if (q >= n) return;
-    const int i = ijk[3 * q], j = ijk[3 * q + 1], k = ijk[3 * q + 2];
-    if (i <= -kCoordLimit || i >= kCoordLimit || j <= -kCoordLimit || j >= kCoordLimit || k <= -kCoordLimit ||
-        k >= kCoordLimit) {
-        atomicExch(bad, 1);
-        keys[q] = 0;
-        masks[q] = 0;
-        return;
-    }
-    keys[q] = leaf_key(i, j, k);
-    // Neighbour offsets the box [x - padding, x + padding] reaches, per axis (bit 0: -1, 1: 0, 2: +1).
-    auto reach = [padding](int c) { return 2u | ((c & 7) < padding ? 1u : 0u) | ((c & 7) + padding >= 8 ? 4u : 0u); };
-    const uint32_t rx = reach(i), ry = reach(j), rz = reach(k);
-    uint32_t m = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                if (((rx >> a) & 1u) && ((ry >> b) & 1u) && ((rz >> c) & 1u)) m |= 1u << (a * 9 + b * 3 + c);
-    masks[q] = m;
-}
-
-struct BitOr {
-    __device__ __forceinline__ uint32_t operator()(uint32_t a, uint32_t b) const { return a | b; }
+struct Box {
+    int lo[3], dim[3];  // in leaf units
 };
 
-__global__ void count_kernel(const uint32_t* __restrict__ masks, const int* __restrict__ num, int* __restrict__ counts) {
-    const int64_t l = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
-    if (l < *num) counts[l] = __popc(masks[l]);
-}
-
-// Step 3: the keys of the leaves each active leaf's mask names.
-__global__ void expand_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ masks,
-                              const int* __restrict__ offsets, const int* __restrict__ num, uint64_t* __restrict__ out) {
-    const int64_t l = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
-    if (l >= *num) return;
-    const int3 o = key_origin(keys[l]);
-    uint32_t m = masks[l];
-    int w = offsets[l];
-    while (m) {
-        const int q = __ffs(m) - 1;
-        m &= m - 1;
-        out[w++] = leaf_key(o.x + 8 * (q / 9 - 1), o.y + 8 * ((q / 3) % 3 - 1), o.z + 8 * (q % 3 - 1));
+// Step 1: bounds[0..2] minima, [3..5] maxima of the coordinates, [6] set when one is out of range.
+__global__ void __launch_bounds__(kTopoThreads) bounds_kernel(const int32_t* __restrict__ ijk, int64_t n,
+                                                              int* __restrict__ bounds) {
+    int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+    for (int64_t q = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x; q < n; q += (int64_t)gridDim.x * kTopoThreads)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int v = __ldg(ijk + 3 * q + d);
+            lo[d] = min(lo[d], v), hi[d] = max(hi[d], v);
+        }
+    __shared__ int red[6];
+    if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = __reduce_min_sync(0xffffffffu, lo[d]);
+        hi[d] = __reduce_max_sync(0xffffffffu, hi[d]);
+    }
+    if ((threadIdx.x & 31) == 0)
+        for (int d = 0; d < 3; ++d) atomicMin(red + d, lo[d]), atomicMax(red + 3 + d, hi[d]);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        atomicMin(bounds + threadIdx.x, red[threadIdx.x]);
+        if (red[threadIdx.x] <= -kCoordLimit) atomicExch(bounds + 6, 1);
+    } else if (threadIdx.x < 6) {
+        atomicMax(bounds + threadIdx.x, red[threadIdx.x]);
+        if (red[threadIdx.x] >= kCoordLimit) atomicExch(bounds + 6, 1);
     }
 }
 
-__global__ void origin_kernel(const uint64_t* __restrict__ keys, int64_t n, int4* __restrict__ org) {
-    const int64_t l = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
-    if (l >= n) return;
-    const int3 o = key_origin(keys[l]);
-    org[l] = make_int4(o.x, o.y, o.z, 0);
+// Step 2: flags (one int per leaf of the box, 0 before) of the leaves the dilated voxels touch.
+__global__ void __launch_bounds__(kTopoThreads) flag_kernel(const int32_t* __restrict__ ijk, int64_t n, int padding, Box box,
+                                                            int* flags) {
+    const int64_t q = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
+    const bool live = q < n;
+    int c[3] = {0, 0, 0};
+    uint32_t reach[3] = {0u, 0u, 0u};  // per axis bit 0: -1, bit 1: 0, bit 2: +1
+    if (live)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int v = __ldg(ijk + 3 * q + d);
+            c[d] = (v >> 3) - box.lo[d];
+            reach[d] = 2u | ((v & 7) < padding ? 1u : 0u) | ((v & 7) + padding >= 8 ? 4u : 0u);
+        }
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 27; ++k)
+        if (((reach[0] >> (k / 9)) & 1u) && ((reach[1] >> ((k / 3) % 3)) & 1u) && ((reach[2] >> (k % 3)) & 1u)) m |= 1u << k;
+    auto at = [&](int k) {
+        return ((int64_t)(c[0] + k / 9 - 1) * box.dim[1] + (c[1] + (k / 3) % 3 - 1)) * box.dim[2] + (c[2] + k % 3 - 1);
+    };
+    // A flag already set is not written again: the list's voxels set few flags many times.
+    auto set = [&](int k) {
+        int* f = flags + at(k);
+        if (*reinterpret_cast<volatile int*>(f) == 0) *f = 1;
+    };
+    const int64_t leaf = ((int64_t)c[0] * box.dim[1] + c[1]) * box.dim[2] + c[2];
+    const int64_t first = __shfl_sync(0xffffffffu, leaf, 0);
+    if (__all_sync(0xffffffffu, live && leaf == first)) {
+        const uint32_t all = __reduce_or_sync(0xffffffffu, m);
+        const int lane = threadIdx.x & 31;
+        if (lane < 27 && ((all >> lane) & 1u)) set(lane);
+    } else {
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            set(k);
+        }
+    }
 }
 
-__global__ void lookup_fill_kernel(const int4* __restrict__ org, int64_t n, TopoView t, int* __restrict__ lookup) {
-    const int64_t l = (int64_t)blockIdx.x * kTopoThreads + threadIdx.x;
-    if (l >= n) return;
-    const int4 o = org[l];
-    const int64_t a = (o.x >> 3) - t.lo_x, b = (o.y >> 3) - t.lo_y, c = (o.z >> 3) - t.lo_z;
-    lookup[(a * t.dim_y + b) * t.dim_z + c] = (int)l;
+// The part of the box that lower node (x, y, z) (coordinates in units of 16 leaves) covers.
+struct NodePart {
+    int lo[3], dim[3];  // box-relative
+    __device__ __forceinline__ int64_t entry(const Box& box, int q) const {
+        const int x = q / (dim[1] * dim[2]), r = q - x * dim[1] * dim[2], y = r / dim[2], z = r - y * dim[2];
+        return ((int64_t)(lo[0] + x) * box.dim[1] + (lo[1] + y)) * box.dim[2] + (lo[2] + z);
+    }
+    __device__ __forceinline__ int size() const { return dim[0] * dim[1] * dim[2]; }
+};
+
+__device__ __forceinline__ NodePart node_part(const Box& box, const int3& node) {
+    NodePart p;
+    const int n[3] = {node.x, node.y, node.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int a = max(16 * n[d] - box.lo[d], 0), b = min(16 * n[d] + 16 - box.lo[d], box.dim[d]);
+        p.lo[d] = a, p.dim[d] = b - a;
+    }
+    return p;
+}
+
+// Step 3a: flagged leaves per lower node.
+__global__ void __launch_bounds__(kTopoThreads) node_count_kernel(const int3* __restrict__ nodes, Box box,
+                                                                  const int* __restrict__ flags, int* __restrict__ counts) {
+    __shared__ int total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    const NodePart p = node_part(box, nodes[blockIdx.x]);
+    int c = 0;
+    for (int q = threadIdx.x; q < p.size(); q += kTopoThreads) c += flags[p.entry(box, q)];
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total, c);
+    __syncthreads();
+    if (threadIdx.x == 0) counts[blockIdx.x] = total;
+}
+
+// Inclusive scan of one value per thread over a CTA of kTopoThreads threads; `sums` has a word per
+// warp. Returns the thread's inclusive sum; `total` receives the CTA's.
+__device__ __forceinline__ int block_scan(int v, int* sums, int& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    if (lane == 31) sums[w] = v;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+#pragma unroll
+    for (int k = 0; k < kTopoThreads / 32; ++k) {
+        if (k < w) before += sums[k];
+        total += sums[k];
+    }
+    __syncthreads();
+    return before + v;
+}
+
+// Step 3b: first leaf number of each node (exclusive scan, one CTA), the total after the last.
+__global__ void __launch_bounds__(kTopoThreads) node_scan_kernel(int* counts, int n) {
+    __shared__ int sums[kTopoThreads / 32];
+    int base = 0;
+    for (int q0 = 0; q0 < n; q0 += kTopoThreads) {
+        const int q = q0 + (int)threadIdx.x, v = q < n ? counts[q] : 0;
+        int total;
+        const int inc = block_scan(v, sums, total);
+        if (q < n) counts[q] = base + inc - v;
+        base += total;
+    }
+    if (threadIdx.x == 0) counts[n] = base;
+}
+
+// Step 4: numbers each node's leaves in x, y, z order: their origins (int4, and packed for the
+// host) and the lookup table's entries (in place of the flags).
+__global__ void __launch_bounds__(kTopoThreads) number_kernel(const int3* __restrict__ nodes, Box box,
+                                                              const int* __restrict__ first, int* __restrict__ lookup,
+                                                              int4* __restrict__ org, int* __restrict__ org3) {
+    __shared__ int sums[kTopoThreads / 32];
+    const NodePart p = node_part(box, nodes[blockIdx.x]);
+    int base = first[blockIdx.x];
+    for (int q0 = 0; q0 < p.size(); q0 += kTopoThreads) {
+        const int q = q0 + (int)threadIdx.x;
+        const int64_t e = q < p.size() ? p.entry(box, q) : 0;
+        const int v = q < p.size() ? lookup[e] : 0;
+        int total;
+        const int l = base + block_scan(v, sums, total) - v;
+        if (q < p.size()) {
+            lookup[e] = v ? l : -1;
+            if (v) {
+                const int z = (int)(e % box.dim[2]), y = (int)((e / box.dim[2]) % box.dim[1]),
+                          x = (int)(e / ((int64_t)box.dim[1] * box.dim[2]));
+                const int o[3] = {8 * (x + box.lo[0]), 8 * (y + box.lo[1]), 8 * (z + box.lo[2])};
+                org[l] = make_int4(o[0], o[1], o[2], 0);
+                org3[3 * l] = o[0], org3[3 * l + 1] = o[1], org3[3 * l + 2] = o[2];
+            }
+        }
+        base += total;
+    }
 }
 
 __global__ void nbr27_kernel(const int4* __restrict__ org, int64_t n, TopoView t, int* __restrict__ nbr) {
@@ -133,15 +226,6 @@ __global__ void nbr27_kernel(const int4* __restrict__ org, int64_t n, TopoView t
         nbr[l * 27 + q] = v;
     }
 }
-
-// CUB temporary storage, grown on demand.
-struct Temp {
-    DeviceBuffer buf;
-    void* get(size_t bytes) {
-        if (buf.bytes < bytes) buf.alloc(std::max<size_t>(bytes, 256));
-        return buf.ptr;
-    }
-};
 
 }  // namespace
 
@@ -159,83 +243,70 @@ void Topology::build_from_voxels(const int32_t* ijk, int64_t n, bool ijk_on_devi
         HNS_CUDA(cudaMemcpyAsync(d_ijk.ptr, ijk, sizeof(int32_t) * 3 * (size_t)n, cudaMemcpyHostToDevice, s));
         dv = d_ijk.as<int32_t>();
     }
-    DeviceBuffer keys(sizeof(uint64_t) * n), masks(sizeof(uint32_t) * n), keys2(sizeof(uint64_t) * n),
-        masks2(sizeof(uint32_t) * n), small(sizeof(int) * 4);
-    int* d_small = small.as<int>();  // [0] bad coordinate, [1] active leaves, [2] candidate count, [3] leaves
-    HNS_CUDA(cudaMemsetAsync(d_small, 0, small.bytes, s));
-    Temp tmp;
-    voxel_key_kernel<<<grid_for(n), kTopoThreads, 0, s>>>(dv, n, padding, keys.as<uint64_t>(), masks.as<uint32_t>(), d_small);
+    DeviceBuffer small(sizeof(int) * 7);
+    const int init[7] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0};
+    HNS_CUDA(cudaMemcpyAsync(small.ptr, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    bounds_kernel<<<(unsigned)std::min<int64_t>(grid_for(n), 2048), kTopoThreads, 0, s>>>(dv, n, small.as<int>());
     HNS_LAUNCHED();
-    size_t tb = 0;
-    HNS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.as<uint64_t>(), keys2.as<uint64_t>(), masks.as<uint32_t>(),
-                                             masks2.as<uint32_t>(), (int)n, 0, 63, s));
-    HNS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(tb), tb, keys.as<uint64_t>(), keys2.as<uint64_t>(),
-                                             masks.as<uint32_t>(), masks2.as<uint32_t>(), (int)n, 0, 63, s));
-    // Active leaves (unique keys) with the OR of their voxels' masks, back into keys / masks.
-    HNS_CUDA(cub::DeviceReduce::ReduceByKey(nullptr, tb, keys2.as<uint64_t>(), keys.as<uint64_t>(), masks2.as<uint32_t>(),
-                                            masks.as<uint32_t>(), d_small + 1, BitOr(), (int)n, s));
-    HNS_CUDA(cub::DeviceReduce::ReduceByKey(tmp.get(tb), tb, keys2.as<uint64_t>(), keys.as<uint64_t>(),
-                                            masks2.as<uint32_t>(), masks.as<uint32_t>(), d_small + 1, BitOr(), (int)n, s));
-    int h_small[4];
-    HNS_CUDA(cudaMemcpyAsync(h_small, d_small, sizeof(h_small), cudaMemcpyDeviceToHost, s));
+    int b[7];
+    HNS_CUDA(cudaMemcpyAsync(b, small.ptr, sizeof(b), cudaMemcpyDeviceToHost, s));
     HNS_CUDA(cudaStreamSynchronize(s));
-    if (h_small[0]) fail(HNS_ERR_INVALID_ARG, "a voxel coordinate is outside +-(2^23 - 64)");
-    const int active = h_small[1];
-    // Candidates: every leaf an active leaf's mask names (at most 27 per active leaf).
-    DeviceBuffer counts(sizeof(int) * ((size_t)active + 1)), offsets(sizeof(int) * ((size_t)active + 1));
-    count_kernel<<<grid_for(active), kTopoThreads, 0, s>>>(masks.as<uint32_t>(), d_small + 1, counts.as<int>());
+    if (b[6]) fail(HNS_ERR_INVALID_ARG, "a voxel coordinate is outside +-(2^23 - 64)");
+    Box box;
+    int64_t entries = 1;
+    for (int d = 0; d < 3; ++d) {
+        // The outermost voxels' dilation boxes reach the outermost leaves: the leaves' bounding box.
+        box.lo[d] = (b[d] - padding) >> 3;
+        box.dim[d] = ((b[3 + d] + padding) >> 3) - box.lo[d] + 1;
+        entries *= box.dim[d];
+    }
+    if (entries > kMaxLookupEntriesDevice)
+        fail(HNS_ERR_UNSUPPORTED, "leaf bounding box exceeds the dense leaf table limit of 2^28 entries");
+    // The box's lower nodes (16^3 leaves) in NanoVDB order: by root tile (32^3 nodes), then by node,
+    // each in x, y, z order.
+    std::vector<int3> nodes;
+    int lo[3], hi[3];
+    for (int d = 0; d < 3; ++d) lo[d] = box.lo[d] >> 4, hi[d] = (box.lo[d] + box.dim[d] - 1) >> 4;
+    auto tile = [](int node) { return node >> 5; };
+    auto span = [&](int d, int t, auto&& body) {
+        for (int v = std::max(lo[d], 32 * t); v <= std::min(hi[d], 32 * t + 31); ++v) body(v);
+    };
+    for (int rx = tile(lo[0]); rx <= tile(hi[0]); ++rx)
+        for (int ry = tile(lo[1]); ry <= tile(hi[1]); ++ry)
+            for (int rz = tile(lo[2]); rz <= tile(hi[2]); ++rz)
+                span(0, rx, [&](int x) { span(1, ry, [&](int y) { span(2, rz, [&](int z) { nodes.push_back(make_int3(x, y, z)); }); }); });
+    const int num_nodes = (int)nodes.size();
+    DeviceBuffer d_nodes(sizeof(int3) * nodes.size()), first(sizeof(int) * (nodes.size() + 1));
+    HNS_CUDA(cudaMemcpyAsync(d_nodes.ptr, nodes.data(), d_nodes.bytes, cudaMemcpyHostToDevice, s));
+    d_lookup.alloc(sizeof(int32_t) * (size_t)entries);
+    HNS_CUDA(cudaMemsetAsync(d_lookup.ptr, 0, d_lookup.bytes, s));
+    flag_kernel<<<grid_for(n), kTopoThreads, 0, s>>>(dv, n, padding, box, d_lookup.as<int>());
     HNS_LAUNCHED();
-    HNS_CUDA(cudaMemsetAsync(counts.as<int>() + active, 0, sizeof(int), s));
-    HNS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts.as<int>(), offsets.as<int>(), active + 1, s));
-    HNS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(tb), tb, counts.as<int>(), offsets.as<int>(), active + 1, s));
-    int total = 0;
-    HNS_CUDA(cudaMemcpyAsync(&total, offsets.as<int>() + active, sizeof(int), cudaMemcpyDeviceToHost, s));
-    HNS_CUDA(cudaStreamSynchronize(s));
-    DeviceBuffer cand(sizeof(uint64_t) * (size_t)total), cand2(sizeof(uint64_t) * (size_t)total);
-    expand_kernel<<<grid_for(active), kTopoThreads, 0, s>>>(keys.as<uint64_t>(), masks.as<uint32_t>(), offsets.as<int>(),
-                                                            d_small + 1, cand.as<uint64_t>());
+    node_count_kernel<<<(unsigned)num_nodes, kTopoThreads, 0, s>>>(d_nodes.as<int3>(), box, d_lookup.as<int>(), first.as<int>());
     HNS_LAUNCHED();
-    HNS_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb, cand.as<uint64_t>(), cand2.as<uint64_t>(), total, 0, 63, s));
-    HNS_CUDA(cub::DeviceRadixSort::SortKeys(tmp.get(tb), tb, cand.as<uint64_t>(), cand2.as<uint64_t>(), total, 0, 63, s));
-    HNS_CUDA(cub::DeviceSelect::Unique(nullptr, tb, cand2.as<uint64_t>(), cand.as<uint64_t>(), d_small + 3, total, s));
-    HNS_CUDA(cub::DeviceSelect::Unique(tmp.get(tb), tb, cand2.as<uint64_t>(), cand.as<uint64_t>(), d_small + 3, total, s));
+    node_scan_kernel<<<1, kTopoThreads, 0, s>>>(first.as<int>(), num_nodes);
+    HNS_LAUNCHED();
     int L = 0;
-    HNS_CUDA(cudaMemcpyAsync(&L, d_small + 3, sizeof(int), cudaMemcpyDeviceToHost, s));
+    HNS_CUDA(cudaMemcpyAsync(&L, first.as<int>() + num_nodes, sizeof(int), cudaMemcpyDeviceToHost, s));
     HNS_CUDA(cudaStreamSynchronize(s));
 
     num_leaves = L;
     d_origin.alloc(sizeof(int4) * (size_t)L);
-    origin_kernel<<<grid_for(L), kTopoThreads, 0, s>>>(cand.as<uint64_t>(), L, d_origin.as<int4>());
-    HNS_LAUNCHED();
-    std::vector<int4> org((size_t)L);
-    HNS_CUDA(cudaMemcpyAsync(org.data(), d_origin.ptr, d_origin.bytes, cudaMemcpyDeviceToHost, s));
-    HNS_CUDA(cudaStreamSynchronize(s));
-    origins.resize((size_t)L * 3);
-    int32_t lo[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    for (int64_t l = 0; l < L; ++l) {
-        const int32_t v[3] = {org[l].x, org[l].y, org[l].z};
-        for (int d = 0; d < 3; ++d) {
-            origins[3 * l + d] = v[d];
-            lo[d] = std::min(lo[d], v[d] >> 3);
-            hi[d] = std::max(hi[d], v[d] >> 3);
-        }
-    }
-    nanovdb_order = true;
-    const int64_t dims[3] = {int64_t(hi[0]) - lo[0] + 1, int64_t(hi[1]) - lo[1] + 1, int64_t(hi[2]) - lo[2] + 1};
-    const int64_t entries = dims[0] * dims[1] * dims[2];
-    if (entries > kMaxLookupEntriesDevice)
-        fail(HNS_ERR_UNSUPPORTED, "leaf bounding box exceeds the dense leaf table limit of 2^28 entries");
-    d_lookup.alloc(sizeof(int32_t) * (size_t)entries);
     d_nbr27.alloc(sizeof(int32_t) * 27 * (size_t)L);
-    HNS_CUDA(cudaMemsetAsync(d_lookup.ptr, 0xFF, d_lookup.bytes, s));  // -1: no leaf
+    // The origins for the host pass through the neighbour table's memory, which is written after.
+    int* org3 = d_nbr27.as<int>();
+    number_kernel<<<(unsigned)num_nodes, kTopoThreads, 0, s>>>(d_nodes.as<int3>(), box, first.as<int>(), d_lookup.as<int>(),
+                                                               d_origin.as<int4>(), org3);
+    HNS_LAUNCHED();
+    origins.resize((size_t)L * 3);
+    HNS_CUDA(cudaMemcpyAsync(origins.data(), org3, sizeof(int32_t) * origins.size(), cudaMemcpyDeviceToHost, s));
+    nanovdb_order = true;
     view.num_leaves = L;
     view.origin = d_origin.as<int4>();
     view.nbr27 = d_nbr27.as<int>();
     view.lookup = d_lookup.as<int>();
-    view.lo_x = lo[0], view.lo_y = lo[1], view.lo_z = lo[2];
-    view.dim_x = (int)dims[0], view.dim_y = (int)dims[1], view.dim_z = (int)dims[2];
-    lookup_fill_kernel<<<grid_for(L), kTopoThreads, 0, s>>>(d_origin.as<int4>(), L, view, d_lookup.as<int>());
-    HNS_LAUNCHED();
+    view.lo_x = box.lo[0], view.lo_y = box.lo[1], view.lo_z = box.lo[2];
+    view.dim_x = box.dim[0], view.dim_y = box.dim[1], view.dim_z = box.dim[2];
     nbr27_kernel<<<grid_for(L), kTopoThreads, 0, s>>>(d_origin.as<int4>(), L, view, d_nbr27.as<int>());
     HNS_LAUNCHED();
     HNS_CUDA(cudaStreamSynchronize(s));
