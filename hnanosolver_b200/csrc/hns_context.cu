@@ -256,14 +256,8 @@ void rbgs_solve(Context& c, const float* div, float* p, int iterations, float om
         if (flags & HNS_SOLVE_ZERO_INIT) HNS_CUDA(cudaMemsetAsync(p, 0, sizeof(float) * c.num_voxels(), c.stream));
         return;
     }
-    if (use_split32(c, flags, div, p)) {
+    if (use_split32(c, div, p)) {
         split32_solve(c, div, p, iterations, omega, flags, nullptr);
-        return;
-    }
-    if ((flags & HNS_SOLVE_NEUMANN) && c.rbgs_kernel == HNS_RBGS_SPLIT && use_chip(c, 2 * iterations) && aligned16(div) &&
-        aligned16(p) && chip_fits(c, sizeof(float), true)) {
-        launch_chip_solve_f32(c, c.split_faces(), div, true, p, true, 2 * iterations, (flags & HNS_SOLVE_ZERO_INIT) != 0, omega,
-                              c.dx * c.dx, true, nullptr, nullptr, 0, 0.0);
         return;
     }
     const size_t n = (size_t)c.num_voxels();

@@ -345,10 +345,10 @@ void launch_rbgs_split_solve_f32(Context& c, const int* nb8, const float* rhs, f
 // The FP32 half-sweep on colour-split leaves (the reference's update and precision): rhs the
 // divergence in the split layout, scaled by dx2 in each update; e in place with the zero leaf.
 // Launches with e_zero false are programmatic dependent launches: pdl false for one that follows
-// a kernel other than a half-sweep.
+// a kernel other than a half-sweep. walls: zero-gradient walls.
 void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* rhs, float* e, int colour, bool e_zero,
                                 float omega, float dx2, const double* check, double tol2, bool short_grid = false,
-                                bool pdl = true);
+                                bool pdl = true, bool walls = false);
 // The solve held in the SMs' shared memory (hns_rbgs_chip.cu): `half_sweeps` half-sweeps (red
 // first) in one cooperative launch, the values of the launch-per-colour kernels to the bit.
 // chip_fits: whether the grid's values of `bytes` each fit, in_place_slots with their right-hand
@@ -372,7 +372,7 @@ inline bool use_chip(const Context& c, int half_sweeps) {
 void convert_split_f32(const Context& c, const float* src, float* dst, bool to_split);
 // acc += {sum r^2, sum b^2} of the FP32 split iterate e (FP64), unless check has passed.
 void launch_split_residual_f32(const Context& c, const int* nb8, const float* rhs, const float* e, double h2,
-                               const double* check, double tol2, double* acc);
+                               const double* check, double tol2, double* acc, bool walls = false);
 void launch_rbgs_packed_half(const Context& c, const void* rhs, const void* halo, const void* e_in, const void* faces_in,
                              void* e_out, void* faces_out, float omega, const double* check, double tol2);
 
@@ -427,9 +427,9 @@ void launch_div_combust_buoy(const Context& c, const float* vel, float* vel_out,
 
 // Runs `iterations` fused RBGS iterations from `p` (or zero) and leaves the result in `p`.
 void rbgs_solve(Context& c, const float* div, float* p, int iterations, float omega, unsigned flags);
-// The FP32 solve on colour-split leaves (hns_step.cu): whether a solve with these flags takes it,
+// The FP32 solve on colour-split leaves (hns_step.cu): whether a solve of these arrays takes it,
 // and the solve (plan: the convergence checks of rbgs_solve_checked, or null).
-bool use_split32(const Context& c, unsigned flags, const float* div, const float* p);
+bool use_split32(const Context& c, const float* div, const float* p);
 void split32_solve(Context& c, const float* div, float* p, int K, float omega, unsigned flags, const SolvePlan* plan);
 
 // Convergence-checked solve: at most `max_iterations` (rounded up to even) iterations; the

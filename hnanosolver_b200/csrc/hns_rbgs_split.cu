@@ -225,28 +225,36 @@ __global__ void __launch_bounds__(kThreads, kHalfCtasPerSm) rbgs_split_half_kern
 constexpr int kF32LeavesPerBlock = 2;
 constexpr int kF32LeavesPerThread = 2;
 constexpr int kF32Threads = 64 * kF32LeavesPerBlock;
-constexpr int kF32ShortGridCtasPerSm = 8;
+// Register limit: 8 CTAs per SM (64 registers) spilled 40 bytes a thread. us per half-sweep at 8, 7
+// and 6 per SM: 45,198 leaves 35.8, 31.9, 32.6 (walls 38.9, 35.8, 35.5); 17,576 leaves 12.2, 9.8, 9.2
+// (13.2, 11.3, 10.7); one leaf per thread at 12: 33.0, 34.4, 11.7, 11.9; three at 5: 36.3, 41.3, 11.1, 14.3.
+constexpr int kF32ShortGridCtasPerSm = 6;
 
 __device__ __forceinline__ float4 ldf4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 ldf4_rw(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float at4(const float4& v, int j) { return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w)); }
 
+// kWalls: zero-gradient walls, the mean of the n in-domain neighbours (a missing one reads the zero
+// leaf, so it adds 0 to the sum), as the staged kernel's Neumann form computes it.
+template <bool kWalls>
 __device__ __forceinline__ float relax_f32(float xp, float xm, float yp, float ym, float zp, float zm, float b, float c,
-                                           float omega, float dx2) {
+                                           float omega, float dx2, int n) {
     const float sum = xp + xm + yp + ym + zp + zm;
-    const float pgs = (sum - b * dx2) * dev::kInv6;
+    const float pgs = kWalls ? (sum - b * dx2) / (float)n : (sum - b * dx2) * dev::kInv6;
     return c + omega * (pgs - c);
 }
 
-template <int P>
+// n: in-domain neighbours of the row's voxels (walls only), less one at the z end if z_missing.
+template <int P, bool kWalls>
 __device__ __forceinline__ float4 relax_row_f32(float4 XP, float4 XM, float4 YP, float4 YM, float4 K, float ZC, float4 B,
-                                                float4 C, float omega, float dx2) {
+                                                float4 C, float omega, float dx2, int n, bool z_missing) {
     float v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float zm = P ? at4(K, j) : (j > 0 ? at4(K, j - 1) : ZC);
         const float zp = P ? (j < 3 ? at4(K, j + 1) : ZC) : at4(K, j);
-        v[j] = relax_f32(at4(XP, j), at4(XM, j), at4(YP, j), at4(YM, j), zp, zm, at4(B, j), at4(C, j), omega, dx2);
+        v[j] = relax_f32<kWalls>(at4(XP, j), at4(XM, j), at4(YP, j), at4(YM, j), zp, zm, at4(B, j), at4(C, j), omega, dx2,
+                                 n - (z_missing && j == (P ? 3 : 0) ? 1 : 0));
     }
     return make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -255,7 +263,7 @@ __device__ __forceinline__ float4 relax_row_f32(float4 XP, float4 XM, float4 YP,
 // scales the right-hand side.
 constexpr int kF32LeavesPerGroup = kF32LeavesPerBlock * kF32LeavesPerThread;
 
-template <bool kZero, bool kShared, bool kPdl, typename Mid>
+template <bool kZero, bool kShared, bool kPdl, bool kWalls, typename Mid>
 __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, const float* __restrict__ rhs, float* e,
                                                 int num_leaves, int g, int colour, float omega, float dx2, Mid&& mid) {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;
@@ -275,20 +283,32 @@ __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, con
     float4 B[kF32LeavesPerThread], out[kF32LeavesPerThread];
 #pragma unroll
     for (int k = 0; k < kF32LeavesPerThread; ++k) B[k] = ldf4(rhs + own[k]);
+    const int sx = a == 7 ? 0 : a == 0 ? 1 : 6, sy = b == 7 ? 2 : b == 0 ? 3 : 6, sz = 5 - p;
+    auto neighbours = [&](uint32_t x, uint32_t y) {  // in-domain ones in x, y and z (the leaf itself for 6)
+        return 6 - (x == (uint32_t)num_leaves ? 1 : 0) - (y == (uint32_t)num_leaves ? 1 : 0);
+    };
     if constexpr (kZero) {
         mid();
 #pragma unroll
         for (int k = 0; k < kF32LeavesPerThread; ++k) {
+            int n = 6;
+            bool z_missing = false;
+            if constexpr (kWalls) {
+                const int* nb = nb8 + 8 * (own[k] >> 9);
+                n = neighbours((uint32_t)__ldg(nb + sx), (uint32_t)__ldg(nb + sy));
+                z_missing = __ldg(nb + sz) == num_leaves;
+            }
             float v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = relax_f32(0.f, 0.f, 0.f, 0.f, 0.f, 0.f, at4(B[k], j), 0.f, omega, dx2);
+            for (int j = 0; j < 4; ++j)
+                v[j] = relax_f32<kWalls>(0.f, 0.f, 0.f, 0.f, 0.f, 0.f, at4(B[k], j), 0.f, omega, dx2,
+                                         n - (z_missing && j == (p ? 3 : 0) ? 1 : 0));
             out[k] = make_float4(v[0], v[1], v[2], v[3]);
             if (live[k]) *reinterpret_cast<float4*>(e + (own[k] ^ 256u)) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     } else {
         const uint32_t co = ((uint32_t)(colour ^ 1) << 8) | (uint32_t)(128 * (w ^ 1));
         auto row = [&](uint32_t n, int a2, int b2) { return (n << 9) | co | (uint32_t)(16 * a2 + 4 * (b2 >> 1)); };
-        const int sx = a == 7 ? 0 : a == 0 ? 1 : 6, sy = b == 7 ? 2 : b == 0 ? 3 : 6, sz = 5 - p;
         uint32_t nx[kF32LeavesPerThread], ny[kF32LeavesPerThread], nz[kF32LeavesPerThread];
 #pragma unroll
         for (int k = 0; k < kF32LeavesPerThread; ++k) {
@@ -319,8 +339,12 @@ __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, con
         mid();  // every load of the pass is in flight
 #pragma unroll
         for (int k = 0; k < kF32LeavesPerThread; ++k)
-            out[k] = p ? relax_row_f32<1>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega, dx2)
-                       : relax_row_f32<0>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega, dx2);
+        {
+            const int n = kWalls ? neighbours(nx[k], ny[k]) : 6;
+            const bool zm = kWalls && nz[k] == (uint32_t)num_leaves;
+            out[k] = p ? relax_row_f32<1, kWalls>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega, dx2, n, zm)
+                       : relax_row_f32<0, kWalls>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega, dx2, n, zm);
+        }
     }
 #pragma unroll
     for (int k = 0; k < kF32LeavesPerThread; ++k)
@@ -328,7 +352,7 @@ __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, con
 }
 
 // rbgs_split_half_kernel on FP32 (see there).
-template <bool kZero>
+template <bool kZero, bool kWalls>
 __global__ void __launch_bounds__(kF32Threads, kF32ShortGridCtasPerSm)
     rbgs_split_half_f32_kernel(const int* __restrict__ nb8, const float* __restrict__ rhs, float* e, int num_leaves,
                                int colour, float omega, float dx2, const double* __restrict__ check, double tol2,
@@ -338,7 +362,7 @@ __global__ void __launch_bounds__(kF32Threads, kF32ShortGridCtasPerSm)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int groups = (num_leaves + kF32LeavesPerGroup - 1) / kF32LeavesPerGroup;
     for (int g = blockIdx.x; g < groups; g += gridDim.x)
-        relax_group_f32<kZero, false, true>(nb8, rhs, e, num_leaves, g, colour, omega, dx2, [] {});
+        relax_group_f32<kZero, false, true, kWalls>(nb8, rhs, e, num_leaves, g, colour, omega, dx2, [] {});
 }
 
 // ---- The persistent solve -------------------------------------------------------------------
@@ -460,9 +484,9 @@ __global__ void __launch_bounds__(kThreads, kShortGridCtasPerSm) rbgs_split_solv
                 relax_group<false, true, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, mid);
         } else {
             if (kZeroFirst && h == 0)
-                relax_group_f32<true, true, false>(nb8, rhs, e, num_leaves, g, 0, omega, dx2, mid);
+                relax_group_f32<true, true, false, false>(nb8, rhs, e, num_leaves, g, 0, omega, dx2, mid);
             else
-                relax_group_f32<false, true, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, dx2, mid);
+                relax_group_f32<false, true, false, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, dx2, mid);
         }
         ph = h, pg = g;
         h = nh, g = ng, x = nx, ok = nok;
@@ -506,7 +530,8 @@ __global__ void __launch_bounds__(256) from_split_f32_kernel(const float* __rest
 // The FP64 residual {sum r^2, sum b^2} of the iterate e (FP32, colour-split), r = div dx^2 -
 // (x+ + x- + y+ + y- + z+ + z- - 6 p), the staged kernel's residual per voxel, into acc. One
 // thread per row of a leaf (both colours, 8 voxels), 2 leaves per CTA, one wave looping; returns
-// at once when `check` has passed.
+// at once when `check` has passed. kWalls: zero-gradient walls, the in-domain neighbours only.
+template <bool kWalls>
 __global__ void __launch_bounds__(128) split_residual_f32_kernel(const int* __restrict__ nb8, const float* __restrict__ rhs,
                                                                  const float* __restrict__ e, int num_leaves, double h2,
                                                                  const double* __restrict__ check, double tol2,
@@ -533,7 +558,7 @@ __global__ void __launch_bounds__(128) split_residual_f32_kernel(const int* __re
         const uint32_t lf = (uint32_t)leaf;
         const uint32_t nxp = a == 7 ? (uint32_t)__ldg(nb + 0) : lf, nxm = a == 0 ? (uint32_t)__ldg(nb + 1) : lf;
         const uint32_t nyp = b == 7 ? (uint32_t)__ldg(nb + 2) : lf, nym = b == 0 ? (uint32_t)__ldg(nb + 3) : lf;
-        const uint32_t nzp = (uint32_t)__ldg(nb + 4), nzm = (uint32_t)__ldg(nb + 5);
+        const uint32_t nzp = (uint32_t)__ldg(nb + 4), nzm = (uint32_t)__ldg(nb + 5), L = (uint32_t)num_leaves;
         float c[8], xp[8], xm[8], yp[8], ym[8], bv[8];
         row8(lf, rp, par, c);
         row8(nxp, rowpos((a + 1) & 7, b), par ^ 1, xp);
@@ -551,8 +576,11 @@ __global__ void __launch_bounds__(128) split_residual_f32_kernel(const int* __re
         const float zhi = __ldg(e + (nzp << 9) + ((uint32_t)par << 8) + rp);
 #pragma unroll
         for (int z = 0; z < 8; ++z) {
+            const int n = 6 - (kWalls ? (nxp == L) + (nxm == L) + (nyp == L) + (nym == L) + (z == 7 && nzp == L) +
+                                            (z == 0 && nzm == L)
+                                      : 0);
             const double lap = (double)xp[z] + (double)xm[z] + (double)yp[z] + (double)ym[z] +
-                               (double)(z < 7 ? c[z + 1] : zhi) + (double)(z > 0 ? c[z - 1] : zlo) - 6.0 * (double)c[z];
+                               (double)(z < 7 ? c[z + 1] : zhi) + (double)(z > 0 ? c[z - 1] : zlo) - (double)n * (double)c[z];
             const double bb = (double)bv[z] * h2;
             r2 += (bb - lap) * (bb - lap);
             b2 += bb * bb;
@@ -700,7 +728,10 @@ void launch_rbgs_split_solve_f32(Context& c, const int* nb8, const float* rhs, f
 namespace hns {
 
 void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* rhs, float* e, int colour, bool e_zero,
-                                float omega, float dx2, const double* check, double tol2, bool short_grid, bool pdl) {
+                                float omega, float dx2, const double* check, double tol2, bool short_grid, bool pdl,
+                                bool walls) {
+    auto first = walls ? rbgs_split_half_f32_kernel<true, true> : rbgs_split_half_f32_kernel<true, false>;
+    auto later = walls ? rbgs_split_half_f32_kernel<false, true> : rbgs_split_half_f32_kernel<false, false>;
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     if (L >= (int64_t(1) << 22)) fail(HNS_ERR_INVALID_ARG, "too many leaves for the colour-split solve");
@@ -712,14 +743,12 @@ void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* r
     cfg.blockDim = dim3(kF32Threads);
     cfg.stream = c.stream;
     if (e_zero) {
-        HNS_CUDA(cudaLaunchKernelEx(&cfg, rbgs_split_half_f32_kernel<true>, nb8, rhs, e, (int)L, colour, omega, dx2, check,
-                                    tol2, c.counters));
+        HNS_CUDA(cudaLaunchKernelEx(&cfg, first, nb8, rhs, e, (int)L, colour, omega, dx2, check, tol2, c.counters));
         HNS_LAUNCHED();
         return;
     }
     if (!pdl) {
-        HNS_CUDA(cudaLaunchKernelEx(&cfg, rbgs_split_half_f32_kernel<false>, nb8, rhs, e, (int)L, colour, omega, dx2, check,
-                                    tol2, c.counters));
+        HNS_CUDA(cudaLaunchKernelEx(&cfg, later, nb8, rhs, e, (int)L, colour, omega, dx2, check, tol2, c.counters));
         HNS_LAUNCHED();
         return;
     }
@@ -729,8 +758,7 @@ void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* r
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HNS_CUDA(cudaLaunchKernelEx(&cfg, rbgs_split_half_f32_kernel<false>, nb8, rhs, e, (int)L, colour, omega, dx2, check,
-                                tol2, c.counters));
+    HNS_CUDA(cudaLaunchKernelEx(&cfg, later, nb8, rhs, e, (int)L, colour, omega, dx2, check, tol2, c.counters));
     HNS_LAUNCHED();
 }
 
@@ -746,11 +774,14 @@ void convert_split_f32(const Context& c, const float* src, float* dst, bool to_s
 }
 
 void launch_split_residual_f32(const Context& c, const int* nb8, const float* rhs, const float* e, double h2,
-                               const double* check, double tol2, double* acc) {
+                               const double* check, double tol2, double* acc, bool walls) {
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     const unsigned g = (unsigned)std::min<int64_t>((L + 1) / 2, (int64_t)c.sm_count() * 8);
-    split_residual_f32_kernel<<<g, 128, 0, c.stream>>>(nb8, rhs, e, (int)L, h2, check, tol2, acc);
+    if (walls)
+        split_residual_f32_kernel<true><<<g, 128, 0, c.stream>>>(nb8, rhs, e, (int)L, h2, check, tol2, acc);
+    else
+        split_residual_f32_kernel<false><<<g, 128, 0, c.stream>>>(nb8, rhs, e, (int)L, h2, check, tol2, acc);
     HNS_LAUNCHED();
 }
 

@@ -37,6 +37,7 @@ Split32 split32_workspace(Context& c) {
 void split32_solve(Context& c, const float* div, float* p, int K, float omega, unsigned flags, const SolvePlan* plan) {
     const float dx2 = c.dx * c.dx;
     const bool zero = (flags & HNS_SOLVE_ZERO_INIT) != 0;
+    const bool walls = (flags & HNS_SOLVE_NEUMANN) != 0;
     if (plan == nullptr && use_chip(c, 2 * K) && chip_fits(c, sizeof(float), false)) {
         // The whole solve in one launch, p in and out in slot order; the divergence too where it is
         // held on the chip, else it is streamed in the split layout.
@@ -47,14 +48,15 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
             convert_split_f32(c, div, s, true);
             rhs = s;
         }
-        launch_chip_solve_f32(c, c.split_faces(), rhs, held, p, true, 2 * K, zero, omega, dx2, false, nullptr, nullptr, 0, 0.0);
+        launch_chip_solve_f32(c, c.split_faces(), rhs, held, p, true, 2 * K, zero, omega, dx2, walls, nullptr, nullptr, 0,
+                              0.0);
         return;
     }
     const Split32 w = split32_workspace(c);
     convert_split_f32(c, div, w.rhs, true);
     if (!zero) convert_split_f32(c, p, w.e, true);
     const double tol2 = plan ? plan->tol * plan->tol : 0.0;
-    if (c.split_solve == HNS_SPLIT_PERSISTENT) {
+    if (c.split_solve == HNS_SPLIT_PERSISTENT && !walls) {
         // Persistent launches over the runs of iterations that share a check slot and have no
         // residual evaluation inside: [cE, (c+1)E - 1) and the single iteration (c+1)E - 1.
         for (int it = 0; it < K;) {
@@ -87,9 +89,9 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
             const bool eval = (it + 1) % E == 0;
             const double* chk = q >= 0 ? plan->slots + 2 * q : nullptr;
             double* next = eval ? plan->slots + 2 * (q + 1) : nullptr;
-            if (eval) launch_split_residual_f32(c, w.nb8, w.rhs, w.e, (double)dx2, chk, tol2, next);
+            if (eval) launch_split_residual_f32(c, w.nb8, w.rhs, w.e, (double)dx2, chk, tol2, next, walls);
             const int end = std::min(K, eval ? it + E : E - 1);
-            launch_chip_solve_f32(c, w.nb8, w.rhs, false, w.e, false, 2 * (end - it), zero && it == 0, omega, dx2, false, chk,
+            launch_chip_solve_f32(c, w.nb8, w.rhs, false, w.e, false, 2 * (end - it), zero && it == 0, omega, dx2, walls, chk,
                                   next, 2, tol2);
             it = end;
         }
@@ -104,21 +106,22 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
             const int last_check = it / E - 1;
             chk = last_check >= 0 ? plan->slots + 2 * last_check : nullptr;
             if ((it + 1) % E == 0) {
-                launch_split_residual_f32(c, w.nb8, w.rhs, w.e, (double)dx2, chk, tol2, plan->slots + 2 * ((it + 1) / E - 1));
+                launch_split_residual_f32(c, w.nb8, w.rhs, w.e, (double)dx2, chk, tol2, plan->slots + 2 * ((it + 1) / E - 1),
+                                          walls);
                 after_half = false;
             }
         }
-        launch_rbgs_split_half_f32(c, w.nb8, w.rhs, w.e, 0, zero && it == 0, omega, dx2, chk, tol2, false, after_half);
-        launch_rbgs_split_half_f32(c, w.nb8, w.rhs, w.e, 1, false, omega, dx2, chk, tol2, false, true);
+        launch_rbgs_split_half_f32(c, w.nb8, w.rhs, w.e, 0, zero && it == 0, omega, dx2, chk, tol2, false, after_half, walls);
+        launch_rbgs_split_half_f32(c, w.nb8, w.rhs, w.e, 1, false, omega, dx2, chk, tol2, false, true, walls);
         after_half = true;
     }
     convert_split_f32(c, w.e, p, false);
 }
 
-bool use_split32(const Context& c, unsigned flags, const float* div, const float* p) {
+bool use_split32(const Context& c, const float* div, const float* p) {
     // The layout conversions move 16-byte vectors of div and p.
     auto a16 = [](const float* q) { return ((uintptr_t)q & 15u) == 0; };
-    return c.rbgs_kernel == HNS_RBGS_SPLIT && !(flags & HNS_SOLVE_NEUMANN) && c.topo.num_leaves < (int64_t(1) << 22) &&
+    return c.rbgs_kernel == HNS_RBGS_SPLIT && c.topo.num_leaves < (int64_t(1) << 22) &&
            a16(div) && a16(p);
 }
 
@@ -144,7 +147,7 @@ SolvePlan rbgs_solve_checked(Context& c, const float* div, float* p, int max_ite
     plan.tol = tol;
     plan.slots = c.reduce_slots(8 + 2 * std::max(1, plan.num_checks)) + 8;  // first 8 doubles: exact residuals
     HNS_CUDA(cudaMemsetAsync(plan.slots, 0, sizeof(double) * 2 * (size_t)std::max(1, plan.num_checks), c.stream));
-    if (use_split32(c, flags, div, p)) {
+    if (use_split32(c, div, p)) {
         split32_solve(c, div, p, K, omega, flags, &plan);
         log_solve(c, plan.slots, plan.num_checks, tol, E, 1, K);
         return plan;

@@ -472,7 +472,7 @@ HNS_API hns_status hns_adjoint_advance_mixed(hns_ctx* ctx, const hns_fire_fields
 
 /* ---- options ----------------------------------------------------------------------------- */
 #define HNS_OPT_RBGS_KERNEL 1 /* which red-black kernel: */
-#define HNS_RBGS_PLAIN 0      /*   plain loads into a padded halo tile (also the zero-gradient walls' kernel) */
+#define HNS_RBGS_PLAIN 0      /*   plain loads into a padded halo tile (both kinds of wall) */
 #define HNS_RBGS_BULK 1       /*   bulk async copies of the contiguous leaf payload into a staged tile, both
                                    colours per launch (used when div and p are 16-byte aligned) */
 #define HNS_RBGS_SPLIT 2      /*   the solve on colour-split leaves, one in-place launch per colour, no
