@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "hns_confine.cuh"
 #include "hns_internal.cuh"
 #include "hns_stencil.cuh"
 
@@ -443,6 +444,119 @@ __global__ void __launch_bounds__(kThreads) adj_confinement_kernel(TopoView t, c
     }
 }
 
+// The same for fs = 1 or -1 as gathers, in three passes without atomics (the scatter form above
+// makes 84 of them a voxel). With w_bar(t) the adjoint of the curl at t,
+//   1. per voxel s: gb(s), the adjoint of the gradient of |omega|, and wb(s) = fb x N, the part of
+//      w_bar(s) that comes from N x omega;
+//   2. per voxel t: w_bar(t) = wb(t) + f omega(t) / |omega(t)| sum over the axes of
+//      gb_d(t - fs e_d) - gb_d(t + fs e_d), the adjoint of |omega(t)| as its neighbours read it;
+//   3. per voxel u: vel_bar(u) += out_bar(u) + the transpose of the curl at u's face neighbours.
+// A face neighbour outside the domain has a curl too (its own neighbours inside make it), with
+// wb = 0: pass 3 computes its w_bar from gb where it meets one.
+// 28,103 leaves: 3.0 -> 1.0 ms.
+__global__ void __launch_bounds__(kThreads) adj_confine_force_kernel(TopoView t, const float* __restrict__ vel,
+                                                                     const float* __restrict__ out_bar,
+                                                                     float* __restrict__ wb_out, float* __restrict__ gb_out,
+                                                                     float dt, float inv_dx, float scale, int fs) {
+    __shared__ dev::LeafNbhd L;
+    __shared__ dev::ConfineTile T;
+    const int64_t leaf = blockIdx.x;
+    dev::load_nbhd(L, t, leaf);
+    __syncthreads();
+    const float f = 0.5f * inv_dx;
+    dev::confine_tile(L, vel, T, f);
+    for (int n = threadIdx.x; n < 512; n += kThreads) {
+        const int a = n >> 6, b = (n >> 3) & 7, d = n & 7, c = dev::conf_wi(a, b, d);
+        const int64_t s = (leaf << 9) + n;
+        const float3 ob = dev::ld3(out_bar, s);
+        const float3 w = make_float3(T.w[0][c], T.w[1][c], T.w[2][c]);
+        const float3 g = make_float3((T.m[dev::conf_wi(a + fs, b, d)] - T.m[dev::conf_wi(a - fs, b, d)]) * f,
+                                     (T.m[dev::conf_wi(a, b + fs, d)] - T.m[dev::conf_wi(a, b - fs, d)]) * f,
+                                     (T.m[dev::conf_wi(a, b, d + fs)] - T.m[dev::conf_wi(a, b, d - fs)]) * f);
+        const float gn = sqrtf(dot3(g, g)), glen = gn + 1e-5f;
+        const float3 N = make_float3(g.x / glen, g.y / glen, g.z / glen);
+        const float3 fb = make_float3(ob.x * dt * scale, ob.y * dt * scale, ob.z * dt * scale);
+        const float3 Nb = make_float3(w.y * fb.z - w.z * fb.y, w.z * fb.x - w.x * fb.z, w.x * fb.y - w.y * fb.x);
+        dev::st3(wb_out, s, make_float3(fb.y * N.z - fb.z * N.y, fb.z * N.x - fb.x * N.z, fb.x * N.y - fb.y * N.x));
+        float3 gb = make_float3(Nb.x / glen, Nb.y / glen, Nb.z / glen);
+        if (gn > 0.f) {
+            const float q = dot3(Nb, g) / (glen * glen * gn);
+            gb.x -= q * g.x, gb.y -= q * g.y, gb.z -= q * g.z;
+        }
+        dev::st3(gb_out, s, gb);
+    }
+}
+
+// omega / |omega| times the adjoint of |omega|, from the six face neighbours' slots (-x, +x, ...; -1
+// outside): pass 2's second term.
+__device__ __forceinline__ float3 magnitude_part(const float* __restrict__ vel, const float* __restrict__ gb,
+                                                 const int64_t ns[6], float f, int fs) {
+    float3 v[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) v[q] = ldv(vel, ns[q]);
+    const float3 w = make_float3(((v[3].z - v[2].z) - (v[5].y - v[4].y)) * f, ((v[5].x - v[4].x) - (v[1].z - v[0].z)) * f,
+                                 ((v[1].y - v[0].y) - (v[3].x - v[2].x)) * f);
+    const float m = sqrtf(dot3(w, w));
+    if (m <= 0.f) return make_float3(0.f, 0.f, 0.f);
+    auto at = [&](int64_t q, int c) { return q < 0 ? 0.f : __ldg(gb + 3 * q + c); };
+    const float sum = (at(ns[0], 0) - at(ns[1], 0)) + (at(ns[2], 1) - at(ns[3], 1)) + (at(ns[4], 2) - at(ns[5], 2));
+    const float r = (fs > 0 ? sum : -sum) * f / m;
+    return make_float3(r * w.x, r * w.y, r * w.z);
+}
+
+__global__ void __launch_bounds__(kThreads) adj_confine_curl_kernel(TopoView t, const float* __restrict__ vel,
+                                                                    const float* __restrict__ gb, float* __restrict__ wb,
+                                                                    float f, int fs) {
+    __shared__ dev::LeafNbhd L;
+    const dev::VoxelIdx v = dev::voxel_of_block();
+    dev::load_nbhd(L, t, v.leaf);
+    __syncthreads();
+    const int64_t s = (v.leaf << 9) + v.n;
+    int64_t ns[6];
+    dev::face_slots(L, s, v.n, ns);
+    const float3 r = magnitude_part(vel, gb, ns, f, fs);
+    wb[3 * s] += r.x;
+    wb[3 * s + 1] += r.y;
+    wb[3 * s + 2] += r.z;
+}
+
+__global__ void __launch_bounds__(kThreads) adj_confine_gather_kernel(TopoView t, const float* __restrict__ vel,
+                                                                      const float* __restrict__ out_bar,
+                                                                      const float* __restrict__ gb,
+                                                                      const float* __restrict__ wb,
+                                                                      float* __restrict__ vel_bar, float f, int fs) {
+    __shared__ dev::LeafNbhd L;
+    const dev::VoxelIdx v = dev::voxel_of_block();
+    dev::load_nbhd(L, t, v.leaf);
+    __syncthreads();
+    const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
+    const int64_t s = (v.leaf << 9) + v.n;
+    int64_t ns[6];
+    dev::face_slots(L, s, v.n, ns);
+    float3 w[6];  // w_bar at -x, +x, -y, +y, -z, +z
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        if (ns[q] >= 0) {
+            w[q] = dev::ld3(wb, ns[q]);
+            continue;
+        }
+        int di, dj, dk;
+        face_offset(q ^ 1, di, dj, dk);  // face_offset's order is +x, -x, ...
+        int64_t around[6];
+#pragma unroll
+        for (int o = 0; o < 6; ++o) {
+            int ei, ej, ek;
+            face_offset(o ^ 1, ei, ej, ek);
+            around[o] = slot_at(t, i + di + ei, j + dj + ej, k + dk + ek);
+        }
+        w[q] = magnitude_part(vel, gb, around, f, fs);
+    }
+    const float3 ob = dev::ld3(out_bar, s);
+    vel_bar[3 * s] += ob.x + f * ((w[4].y - w[5].y) - (w[2].z - w[3].z));
+    vel_bar[3 * s + 1] += ob.y + f * ((w[0].z - w[1].z) - (w[4].x - w[5].x));
+    vel_bar[3 * s + 2] += ob.z + f * ((w[2].x - w[3].x) - (w[0].y - w[1].y));
+}
+
 __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __restrict__ src, float* __restrict__ dst,
                                                               int64_t n) {
     const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -511,12 +625,27 @@ void launch_adj_rbgs_colour(const Context& c, float* lam, float* div_bar, int co
     HNS_LAUNCHED();
 }
 
-void launch_adj_confinement(const Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt,
-                            float scale, float factor_scale) {
+void launch_adj_confinement(Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt, float scale,
+                            float factor_scale, float* work) {
     const int64_t n = c.num_voxels();
     if (n == 0) return;
+    const int fs = (int)factor_scale;
+    if (fs == 1 || fs == -1) {
+        if (work == nullptr) work = c.scratch_f32("adjoint_work", 8 * (size_t)n);
+        float *wb = work, *gb = work + 3 * n;
+        const float f = 0.5f * (1.0f / c.dx);
+        adj_confine_force_kernel<<<(unsigned)c.topo.num_leaves, kThreads, 0, c.stream>>>(c.topo.view, vel, out_bar, wb, gb, dt,
+                                                                                         1.0f / c.dx, scale, fs);
+        HNS_LAUNCHED();
+        adj_confine_curl_kernel<<<(unsigned)(2 * c.topo.num_leaves), kThreads, 0, c.stream>>>(c.topo.view, vel, gb, wb, f, fs);
+        HNS_LAUNCHED();
+        adj_confine_gather_kernel<<<(unsigned)(2 * c.topo.num_leaves), kThreads, 0, c.stream>>>(c.topo.view, vel, out_bar, gb,
+                                                                                                wb, vel_bar, f, fs);
+        HNS_LAUNCHED();
+        return;
+    }
     adj_confinement_kernel<<<blocks_for(n), kThreads, 0, c.stream>>>(c.topo.view, vel, out_bar, vel_bar, dt, 1.0f / c.dx,
-                                                                     scale, (int)factor_scale, n);
+                                                                     scale, fs, n);
     HNS_LAUNCHED();
 }
 

@@ -438,7 +438,7 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
     // Confinement and the velocity's self-advection.
     float* advb = arena + 5 * n;
     HNS_CUDA(cudaMemsetAsync(advb, 0, 3 * n * sizeof(float), c.stream));
-    launch_adj_confinement(c, adv, adv2b, advb, dt, P.vorticityScale, P.factorScale);
+    launch_adj_confinement(c, adv, adv2b, advb, dt, P.vorticityScale, P.factorScale, arena + 8 * n);
     launch_adj_advect(c, in.velocity, advb, nullptr, nullptr, nullptr, 0, in_bar.velocity, dt, arena + 8 * n);
 }
 

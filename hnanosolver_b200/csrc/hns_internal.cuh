@@ -389,8 +389,9 @@ void launch_adj_advect(Context& c, const float* vel, const float* vel_out_bar, c
 void launch_adj_divergence(const Context& c, const float* div_bar, float* vel_bar);
 void launch_adj_gradient(const Context& c, const float* out_bar, float* p_bar);
 void launch_adj_rbgs_colour(const Context& c, float* lam, float* div_bar, int colour, float keep, float nbr, float dmul);
-void launch_adj_confinement(const Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt,
-                            float scale, float factor_scale);
+// work: 6 floats per voxel of scratch (null: the context's).
+void launch_adj_confinement(Context& c, const float* vel, const float* out_bar, float* vel_bar, float dt, float scale,
+                            float factor_scale, float* work = nullptr);
 void launch_adj_accumulate(const Context& c, const float* src, float* dst, int64_t n);
 // div_bar += M^T p_bar for `iterations` red-black iterations from p = 0 (p = M div). lam: n floats
 // of scratch (null: the context's).

@@ -125,3 +125,28 @@ def test_wait_gives_up_then_recovers(dev):
         g.device_status()
     assert torch.equal(pa, pb)
     a.close(), b.close()
+
+
+@pytest.mark.parametrize("name", GRIDS)
+def test_walls_per_colour_bit_exact(dev, name):
+    """Zero-gradient walls, one launch per half-sweep on colour-split leaves against the staged
+    kernel: fixed iterations from zero and from given values, and a checked solve's iterates."""
+    from hnanosolver_b200 import lib as hl
+
+    a, b = (hl.Grid(_origins(name), voxel_size=0.1) for _ in range(2))
+    a.set_option(hl.OPT_SPLIT_SOLVE, hl.SPLIT_PER_COLOUR)
+    b.set_option(hl.OPT_RBGS_KERNEL, hl.RBGS_PLAIN)
+    n = a.num_voxels
+    div, p0, vel = _field(n, dev, 8), _field(n, dev, 9), _field(n, dev, 10, 3)
+    step = hl.StepDesc(dt=0.05, max_iterations=60, omega=1.5, tolerance=1e-2, check_every=10, flags=hl.SOLVE_NEUMANN)
+    got = []
+    for g in (a, b):
+        p, q, vo = p0.clone(), torch.empty_like(p0), torch.empty_like(vel)
+        torch.cuda.synchronize()
+        g.rbgs(div, p, 5, 1.6, hl.SOLVE_NEUMANN)
+        g.rbgs(div, q, 5, 1.6, hl.SOLVE_NEUMANN | hl.SOLVE_ZERO_INIT)
+        g.step_plain(vel, vo, [], [], step)
+        got.append((p, q, vo, g.last_solve().iterations))
+    for x, y in zip(*got):
+        assert x == y if isinstance(x, int) else torch.equal(x, y)
+    a.close(), b.close()
