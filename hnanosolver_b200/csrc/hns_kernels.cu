@@ -11,6 +11,10 @@
 // that one pass reads p and div once and writes p once (ping-pong buffers).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
+#include "hns_advect_tile.cuh"
+#include "hns_scalars_tile.cuh"
 #include "hns_internal.cuh"
 #include "hns_stencil.cuh"
 
@@ -472,14 +476,65 @@ unsigned leaf_blocks(const Context& c) { return (unsigned)(c.topo.num_leaves * 2
 }  // namespace
 
 void launch_advect_fused(const Context& c, const float* vel, float* vel_out, const FieldSet& f, float dt, const float* sdf) {
-    advect_fused_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, vel_out, f, dt * (1.0f / c.dx), sdf,
-                                                                   1.0f / c.dx);
+    const float sdt = dt * (1.0f / c.dx);
+    auto tile = [&](float* vo, const float* in, float* out) {
+        if (c.topo.num_leaves < (int64_t(1) << 22))
+            advect_tile_kernel<TileF32, int32_t><<<(unsigned)c.topo.num_leaves, kTileThreads, 0, c.stream>>>(
+                c.topo.view, vel, in, vo, out, sdt, 1.0f);
+        else
+            advect_tile_kernel<TileF32, int64_t><<<(unsigned)c.topo.num_leaves, kTileThreads, 0, c.stream>>>(
+                c.topo.view, vel, in, vo, out, sdt, 1.0f);
+        HNS_LAUNCHED();
+    };
+    // Without a collider: the leaf tile for the velocity and the first scalar, and for one scalar
+    // more; two or more further scalars share one trace in the gather kernel.
+    FieldSet rest = f;
+    if (sdf == nullptr && (vel_out != nullptr || f.count == 1)) {
+        tile(vel_out, f.count > 0 ? f.in[0] : nullptr, f.count > 0 ? f.out[0] : nullptr);
+        if (f.count == 2) tile(nullptr, f.in[1], f.out[1]);
+        if (f.count <= 2) return;
+        rest.count = f.count - 1;
+        for (int q = 0; q < rest.count; ++q) rest.in[q] = f.in[q + 1], rest.out[q] = f.out[q + 1];
+        vel_out = nullptr;
+    }
+    advect_fused_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, vel_out, rest, sdt, sdf, 1.0f / c.dx);
     HNS_LAUNCHED();
 }
 
-void launch_advect_scalars(const Context& c, const float* vel, const FieldSet& f, float dt, const float* sdf) {
-    advect_scalars_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, f, dt * (1.0f / c.dx), sdf);
+namespace {
+
+template <int kCount>
+void launch_scalars_tile(const Context& c, const float* vel, const ScalarPass& P, float sdt) {
+    constexpr size_t bytes = 2 * sizeof(float4) * kTileSide * TileF32::kSX;
+    auto kern = c.topo.num_leaves < (int64_t(1) << 22) ? advect_scalars_tile_kernel<kCount, int32_t>
+                                                       : advect_scalars_tile_kernel<kCount, int64_t>;
+    // The same limit for every context of the process.
+    HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    kern<<<(unsigned)c.topo.num_leaves, kTileThreads, bytes, c.stream>>>(c.topo.view, vel, P, sdt);
     HNS_LAUNCHED();
+}
+
+}  // namespace
+
+void launch_advect_scalars(const Context& c, const float* vel, const FieldSet& f, float dt, const float* sdf) {
+    const float sdt = dt * (1.0f / c.dx);
+    if (sdf != nullptr) {
+        advect_scalars_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, f, sdt, sdf);
+        HNS_LAUNCHED();
+        return;
+    }
+    for (int base = 0; base < f.count; base += kScalarsPerPass) {
+        ScalarPass P{};
+        const int m = std::min(kScalarsPerPass, f.count - base);
+        for (int q = 0; q < m; ++q) P.in[q] = f.in[base + q], P.out[q] = f.out[base + q];
+        switch (m) {
+            case 1: launch_scalars_tile<1>(c, vel, P, sdt); break;
+            case 2: launch_scalars_tile<2>(c, vel, P, sdt); break;
+            case 3: launch_scalars_tile<3>(c, vel, P, sdt); break;
+            case 4: launch_scalars_tile<4>(c, vel, P, sdt); break;
+            default: launch_scalars_tile<5>(c, vel, P, sdt); break;
+        }
+    }
 }
 
 void launch_collision_enforce(const Context& c, float* vel, const float* sdf) {

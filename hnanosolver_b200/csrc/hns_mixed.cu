@@ -26,6 +26,7 @@
 #include <string>
 #include <vector>
 
+#include "hns_advect_tile.cuh"
 #include "hns_internal.cuh"
 #include "hns_stencil.cuh"
 #include "hns_types.cuh"
@@ -1105,148 +1106,6 @@ __global__ void __launch_bounds__(kThreads, 4) advect_records_kernel(TopoView t,
     }
 }
 
-// ---- advection from a leaf tile in shared memory --------------------------------------------
-// The advection of the velocity and at most one scalar (advect_records_kernel's arithmetic)
-// with the leaf's voxels and a kTileHalo-voxel halo around it read once from the BF16 velocity
-// and FP16 scalar arrays into shared memory as FP32 (u, v, w, s), a tile of kTileSide^3 cells
-// at local coordinates [-kTileHalo, 8 + kTileHalo), with no record-packing pass. A trace cell
-// whose eight corners lie in the tile is eight shared-memory loads at fixed offsets from one
-// base index (a back trace shorter than a voxel per axis, and a forward trace that ends within
-// a voxel of the start); other cells take the leaf-table path, reading the arrays. The clamp's
-// six face neighbours always lie in the tile. Same values, same lerps in the same order, same
-// clamps: the records kernel's results to the bit. One CTA of 256 threads per leaf, two voxels
-// per thread (x and x + 4), four CTAs per SM so that one CTA's tile fill overlaps the others'
-// sampling; cells of missing leaves hold 0, as the records kernel reads outside the domain.
-//
-// Tile layout: cell (x, y, z) at x * kTileSX + y * kTileSY + z, both strides multiples of 8 cells
-// (16-byte cells): the 8 lanes of a quarter-warp, one z-row of voxels, then read cells whose
-// bank group is set by z alone, so a row whose traces straddle a y or x cell boundary still
-// reads distinct bank groups (an unpadded 10-cell stride measured 38 % bank conflicts).
-constexpr int kTileHalo = 1;
-constexpr int kTileSide = 8 + 2 * kTileHalo;
-constexpr int kTileSY = 16, kTileSX = kTileSide * kTileSY;
-constexpr int kTileCells = kTileSide * kTileSide * kTileSide;  // cells filled
-constexpr int kTileStore = kTileSide * kTileSX;                // cells allocated (padding included)
-constexpr int kTileThreads = 256;
-constexpr int kTileFill = (kTileCells + kTileThreads - 1) / kTileThreads;  // cells a thread fills
-
-// Trilinear sample of the four channels at (x, y, z) (global voxel units), lerps along z, then
-// y, then x (tri_lerp's order).
-// The FP32 (u, v, w, s) of the voxel at slot s from the BF16 velocity and FP16 scalar arrays
-// (s0 null: s = 0).
-__device__ __forceinline__ float4 voxel4(const __nv_bfloat16* __restrict__ vel, const __half* __restrict__ s0, uint32_t s) {
-    const unsigned short* v = reinterpret_cast<const unsigned short*>(vel) + 3 * (size_t)s;
-    return make_float4(__uint_as_float((uint32_t)__ldg(v) << 16), __uint_as_float((uint32_t)__ldg(v + 1) << 16),
-                       __uint_as_float((uint32_t)__ldg(v + 2) << 16), s0 != nullptr ? __half2float(__ldg(s0 + s)) : 0.f);
-}
-
-__device__ __forceinline__ float4 tile_sample(const float4* __restrict__ tile, const TopoView& t, const LeafNbhd& L,
-                                              const __nv_bfloat16* __restrict__ vel, const __half* __restrict__ s0,
-                                              float x, float y, float z) {
-    const int i = __float2int_rd(x), j = __float2int_rd(y), k = __float2int_rd(z);
-    const float tx = x - (float)i, ty = y - (float)j, tz = z - (float)k;
-    const int cx = i - (L.lx << 3) + kTileHalo, cy = j - (L.ly << 3) + kTileHalo, cz = k - (L.lz << 3) + kTileHalo;
-    float4 c[8];
-    if ((unsigned)cx <= (unsigned)(kTileSide - 2) && (unsigned)cy <= (unsigned)(kTileSide - 2) &&
-        (unsigned)cz <= (unsigned)(kTileSide - 2)) {
-        const float4* b = tile + cx * kTileSX + cy * kTileSY + cz;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) c[q] = b[(q >> 2) * kTileSX + ((q >> 1) & 1) * kTileSY + (q & 1)];
-    } else {
-        TapsT<int32_t> tp;
-        taps_at(tp, t, L, x, y, z);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) c[q] = tp.s[q] < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : voxel4(vel, s0, (uint32_t)tp.s[q]);
-    }
-    auto tri = [&](float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7) {
-        const float z0 = lerp1(v0, v1, tz), z1 = lerp1(v2, v3, tz), z2 = lerp1(v4, v5, tz), z3 = lerp1(v6, v7, tz);
-        return lerp1(lerp1(z0, z1, ty), lerp1(z2, z3, ty), tx);
-    };
-    return make_float4(tri(c[0].x, c[1].x, c[2].x, c[3].x, c[4].x, c[5].x, c[6].x, c[7].x),
-                       tri(c[0].y, c[1].y, c[2].y, c[3].y, c[4].y, c[5].y, c[6].y, c[7].y),
-                       tri(c[0].z, c[1].z, c[2].z, c[3].z, c[4].z, c[5].z, c[6].z, c[7].z),
-                       tri(c[0].w, c[1].w, c[2].w, c[3].w, c[4].w, c[5].w, c[6].w, c[7].w));
-}
-
-__global__ void __launch_bounds__(kTileThreads, 4) advect_tile_kernel(TopoView t, const __nv_bfloat16* __restrict__ vel,
-                                                                       const __half* __restrict__ s0,
-                                                                       __nv_bfloat16* __restrict__ vel_out,
-                                                                       __half* __restrict__ s0_out, float sdt) {
-    __shared__ float4 tile[kTileStore];
-    __shared__ LeafNbhd L;
-    const int64_t leaf = blockIdx.x;
-    load_nbhd(L, t, leaf);
-    __syncthreads();
-    // The fill: every load of the thread's cells is issued before any is unpacked.
-    const unsigned short* vb = reinterpret_cast<const unsigned short*>(vel);
-    const unsigned short* sb = reinterpret_cast<const unsigned short*>(s0);
-    uint32_t raw[kTileFill][4];
-#pragma unroll
-    for (int m = 0; m < kTileFill; ++m) {
-        const int q = threadIdx.x + m * kTileThreads;
-        raw[m][0] = raw[m][1] = raw[m][2] = raw[m][3] = 0u;
-        if (q < kTileCells) {
-            const int lx = q / (kTileSide * kTileSide) - kTileHalo, ly = (q / kTileSide) % kTileSide - kTileHalo,
-                      lz = q % kTileSide - kTileHalo;
-            const int r = (lx < 0 ? 0 : lx > 7 ? 18 : 9) + (ly < 0 ? 0 : ly > 7 ? 6 : 3) + (lz < 0 ? 0 : lz > 7 ? 2 : 1);
-            const int l = L.nb[r];
-            if (l >= 0) {
-                const uint32_t sl = ((uint32_t)l << 9) | (uint32_t)(((lx & 7) << 6) | ((ly & 7) << 3) | (lz & 7));
-                raw[m][0] = __ldg(vb + 3 * (size_t)sl);
-                raw[m][1] = __ldg(vb + 3 * (size_t)sl + 1);
-                raw[m][2] = __ldg(vb + 3 * (size_t)sl + 2);
-                if (sb != nullptr) raw[m][3] = __ldg(sb + sl);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < kTileFill; ++m) {
-        const int q = threadIdx.x + m * kTileThreads;
-        if (q < kTileCells) {
-            const int at = (q / (kTileSide * kTileSide)) * kTileSX + ((q / kTileSide) % kTileSide) * kTileSY + q % kTileSide;
-            tile[at] = make_float4(__uint_as_float(raw[m][0] << 16), __uint_as_float(raw[m][1] << 16),
-                                   __uint_as_float(raw[m][2] << 16), __half2float(__ushort_as_half((unsigned short)raw[m][3])));
-        }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-        const int n = (int)threadIdx.x + half * kTileThreads;
-        const int a = n >> 6, b = (n >> 3) & 7, cz = n & 7;
-        const int i = (L.lx << 3) + a, j = (L.ly << 3) + b, k = (L.lz << 3) + cz;
-        const float4* centre = tile + (a + kTileHalo) * kTileSX + (b + kTileHalo) * kTileSY + (cz + kTileHalo);
-        const float4 o = *centre;
-        const float bx = (float)i - o.x * sdt, by = (float)j - o.y * sdt, bz = (float)k - o.z * sdt;
-        const float4 f = tile_sample(tile, t, L, vel, s0, bx, by, bz);
-        const float4 g = tile_sample(tile, t, L, vel, s0, bx + f.x * sdt, by + f.y * sdt, bz + f.z * sdt);
-        float3 corr = make_float3(f.x + 0.5f * (o.x - g.x), f.y + 0.5f * (o.y - g.y), f.z + 0.5f * (o.z - g.z));
-        float3 mn = make_float3(o.x, o.y, o.z), mx = mn;
-        float dmn = o.w, dmx = o.w;
-        constexpr int kOff[6] = {-kTileSX, kTileSX, -kTileSY, kTileSY, -1, 1};
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float4 e = centre[kOff[q]];
-            mn.x = fminf(mn.x, e.x), mn.y = fminf(mn.y, e.y), mn.z = fminf(mn.z, e.z);
-            mx.x = fmaxf(mx.x, e.x), mx.y = fmaxf(mx.y, e.y), mx.z = fmaxf(mx.z, e.z);
-            dmn = fminf(dmn, e.w);
-            dmx = fmaxf(dmx, e.w);
-        }
-        mn.x = fminf(mn.x, f.x), mn.y = fminf(mn.y, f.y), mn.z = fminf(mn.z, f.z);
-        mx.x = fmaxf(mx.x, f.x), mx.y = fmaxf(mx.y, f.y), mx.z = fmaxf(mx.z, f.z);
-        corr.x = fmaxf(mn.x, fminf(corr.x, mx.x));
-        corr.y = fmaxf(mn.y, fminf(corr.y, mx.y));
-        corr.z = fmaxf(mn.z, fminf(corr.z, mx.z));
-        const int64_t s = (leaf << 9) + n;
-        if (vel_out != nullptr) vstore(vel_out, s, corr);
-        if (s0_out != nullptr) {
-            const float dcorr = f.w + 0.5f * (o.w - g.w);
-            dmn = fminf(dmn, f.w);
-            dmx = fmaxf(dmx, f.w);
-            sstore(s0_out, s, fmaxf(dmn, fminf(dcorr, dmx)));
-        }
-    }
-}
-
 }  // namespace
 
 void launch_advect_mixed(Context& c, const void* vel, void* vel_out, const void* const* sin, void* const* sout, int ns,
@@ -1256,9 +1115,9 @@ void launch_advect_mixed(Context& c, const void* vel, void* vel_out, const void*
     auto aligned8 = [](const void* q) { return ((uintptr_t)q & 7u) == 0; };
     if (n > 0 && c.topo.num_leaves < (int64_t(1) << 22) && ns <= 1) {
         // Velocity and at most one scalar: the shared-memory leaf tile, filled from the arrays.
-        advect_tile_kernel<<<(unsigned)c.topo.num_leaves, kTileThreads, 0, c.stream>>>(
+        advect_tile_kernel<TileHalf, int32_t><<<(unsigned)c.topo.num_leaves, kTileThreads, 0, c.stream>>>(
             c.topo.view, static_cast<const __nv_bfloat16*>(vel), ns > 0 ? static_cast<const __half*>(sin[0]) : nullptr,
-            static_cast<__nv_bfloat16*>(vel_out), ns > 0 ? static_cast<__half*>(sout[0]) : nullptr, sdt);
+            static_cast<__nv_bfloat16*>(vel_out), ns > 0 ? static_cast<__half*>(sout[0]) : nullptr, sdt, 1.0f);
         HNS_LAUNCHED();
         return;
     }
