@@ -351,10 +351,11 @@ void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* r
                                 bool pdl = true, bool walls = false);
 // The solve held in the SMs' shared memory (hns_rbgs_chip.cu): `half_sweeps` half-sweeps (red
 // first) in one cooperative launch, the values of the launch-per-colour kernels to the bit.
-// chip_fits: whether the grid's values of `bytes` each fit, in_place_slots with their right-hand
-// side (needed where the right-hand side is in slot order). walls: zero-gradient walls. The launch
-// does nothing when `check` has passed, and ends before half-sweep mid_half when check_mid has.
-bool chip_fits(const Context& c, size_t bytes, bool in_place_slots);
+// chip_fits: whether a grid of values of `bytes` each fits and is faster there (transpose: for
+// launch_chip_transpose). The slots flags: the array is in slot order, else colour-split. walls:
+// zero-gradient walls. The launch does nothing when `check` has passed, and ends before half-sweep
+// mid_half when check_mid has.
+bool chip_fits(const Context& c, size_t bytes, bool transpose = false);
 void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,
                            int half_sweeps, bool e_zero, float omega, float dx2, bool walls, const double* check,
                            const double* check_mid, int mid_half, double tol2);

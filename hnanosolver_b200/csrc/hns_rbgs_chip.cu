@@ -1,20 +1,20 @@
 // The red-black SOR solve held on the chip: every half-sweep of a solve in one cooperative launch
-// whose CTAs, one per SM, keep their leaves' values in shared memory from the first half-sweep to
+// whose CTAs, all resident, keep their leaves' values in shared memory from the first half-sweep to
 // the last and exchange only the faces between CTAs.
 //
 // Why. A half-sweep of a grid of a few million voxels is bound by its launch, by L2 latency and by
 // the drain between the colours, not by bytes. The 148 SMs hold 33 MB of shared memory between
-// them; the values and the right-hand side of 3.5M FP32 voxels (6.9M in FP16, and 1.7 times as many
-// without the right-hand side, which then streams from L2) fit there with a halo.
+// them, where the values and the right-hand side of a few million voxels fit with a halo.
 //
 // Measured, us per half-sweep of a box of leaves, one launch per colour -> here:
-//   leaves           59          512         1,493        3,300        6,594        10,000
-//   FP32         3.2 -> 1.1  2.3 -> 1.6   3.0 -> 2.2   3.9 -> 3.5   5.4 -> 4.6   7.3 -> 6.1
-//   walls        4.6 -> 1.2  7.2 -> 1.7    15 -> 2.5    28 -> 3.5    52 -> 4.7  (staged kernel)
-//   transpose    4.1 -> 1.1  4.5 -> 1.6   6.2 -> 2.3    10 -> 3.4    16 -> 5.1
-//   FP16         2.3 -> 1.1  2.1 -> 1.7   3.4 -> 2.1   2.8 -> 3.0   3.6 -> 4.0   4.8 -> 4.8
-// What is left is instruction issue and the shared-memory pipe (each about half busy on 6,594
-// leaves) behind the exchange's L2 round trip (1.1 us with nothing else to do).
+//   leaves           59          512         1,493        3,300        5,300        6,594
+//   FP32         3.0 -> 1.1  2.1 -> 1.2   2.3 -> 1.7   2.7 -> 2.8   3.7 -> 3.8      4.3
+//   walls        3.0 -> 1.2  2.1 -> 1.3   2.8 -> 1.9   3.0 -> 3.0   4.2 -> 4.1      4.8
+//   transpose    4.1 -> 1.1  4.5 -> 1.2   6.2 -> 1.8    10 -> 3.0    14 -> 4.0   16 -> 5.0
+//   FP16         1.8 -> 1.1  2.1 -> 1.2   3.4 -> 1.7   2.8 -> 2.7   3.6 -> 3.5      3.6
+// From 3,300 leaves on the gain is the host's: one launch in place of hundreds. What is left is the
+// shared-memory pipe and instruction issue, and for small grids the exchange's L2 round trip (1.1 us
+// with nothing else to do).
 //
 // Partition. CTA k owns the P leaves from k P (the caller's leaf order, which is spatially compact
 // for NanoVDB-ordered grids; any order is correct). Leaves are stored colour-split, as in
@@ -50,8 +50,9 @@ namespace hns {
 namespace {
 
 constexpr uint32_t kChipMaxPolls = 1u << 20;
+constexpr size_t kChipSmSmem = 233472;   // an SM's shared memory, 228 KB
 constexpr size_t kChipMaxSmem = 232448;  // 227 KB, the most one CTA can have
-constexpr size_t kChipReserve = 2048;    // static shared memory and slack
+constexpr size_t kChipReserve = 1536;    // of each CTA: 1 KB of the system's, its static shared memory
 
 enum ChipMode { kDirichlet = 0, kWalls = 1, kTranspose = 2 };
 
@@ -214,9 +215,7 @@ __device__ __forceinline__ uint2 update(const uint2& XP, const uint2& XM, const 
     return make_uint2(r[0], r[1]);
 }
 
-// kRhsSmem: the right-hand side (kTranspose: the divergence's adjoint) is held in shared memory too;
-// otherwise it is read from global memory in every half-sweep (colour-split order required).
-template <typename T, ChipMode kMode, bool kRhsSmem, int kChipThreads>
+template <typename T, ChipMode kMode, int kChipThreads>
 __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_kernel(ChipArgs<T> A) {
     using V = typename Row<T>::V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -229,8 +228,8 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
     T* es = reinterpret_cast<T*>(smem_raw);
     const int halo0 = (P + 1) * 512;
     T* bs = es + halo0 + (size_t)P * 6 * 32;
-    int* nbs = reinterpret_cast<int*>(bs + (kRhsSmem ? (size_t)P * 512 : 0));  // face table, 8 per leaf
-    int* foreign = nbs + 8 * P;                                                // 8 l + f of each foreign face
+    int* nbs = reinterpret_cast<int*>(bs + (size_t)P * 512);  // face table, 8 per leaf
+    int* foreign = nbs + 8 * P;                               // 8 l + f of each foreign face
     if (tid == 0) num_foreign = 0;
     __syncthreads();
     // Face table: a local leaf 0 .. P - 1, P for a missing neighbour, -1 - g for leaf g of another CTA.
@@ -254,14 +253,12 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
         V c0 = Row<T>::zero(), c1 = c0;
         if (!A.zero_init) load_row(A.e, A.e_slots, leaf0 + l, a, b, 4 * r, c0, c1);
         store_row(es, false, l, a, b, 4 * r, c0, c1);
-        if constexpr (kRhsSmem) {
-            if constexpr (kMode == kTranspose)
-                load_row(A.bar, A.rhs_slots, leaf0 + l, a, b, 4 * r, c0, c1);
-            else
-                load_row(A.rhs, A.rhs_slots, leaf0 + l, a, b, 4 * r, c0, c1);
-            if constexpr (kMode != kTranspose) c0 = scaled(c0, A.dx2), c1 = scaled(c1, A.dx2);
-            store_row(bs, false, l, a, b, 4 * r, c0, c1);
-        }
+        if constexpr (kMode == kTranspose)
+            load_row(A.bar, A.rhs_slots, leaf0 + l, a, b, 4 * r, c0, c1);
+        else
+            load_row(A.rhs, A.rhs_slots, leaf0 + l, a, b, 4 * r, c0, c1);
+        if constexpr (kMode != kTranspose) c0 = scaled(c0, A.dx2), c1 = scaled(c1, A.dx2);
+        store_row(bs, false, l, a, b, 4 * r, c0, c1);
     }
     __syncthreads();
     const int nf = num_foreign;
@@ -369,10 +366,8 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
                 V B;
                 if constexpr (kMode == kTranspose)
                     B = Row<T>::zero();
-                else if constexpr (kRhsSmem)
-                    B = *reinterpret_cast<const V*>(bs + own);
                 else
-                    B = scaled(__ldg(reinterpret_cast<const V*>(A.rhs + ((int64_t)leaf0 << 9) + own)), A.dx2);
+                    B = *reinterpret_cast<const V*>(bs + own);
                 const V C = *reinterpret_cast<const V*>(es + own), K = *reinterpret_cast<const V*>(es + (own ^ 256));
                 const V XP = *reinterpret_cast<const V*>(es + (a == 7 ? ax : leaf + ixp));
                 const V XM = *reinterpret_cast<const V*>(es + (a == 0 ? ax : leaf + ixm));
@@ -421,27 +416,47 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
 // Shared memory of a CTA of per_cta leaves: values, the zero leaf, six halo faces a leaf, the
 // right-hand side, the face table and the list of foreign faces.
 template <typename T>
-size_t chip_smem(int64_t per_cta, bool rhs) {
-    return (((size_t)per_cta * (rhs ? 2 : 1) + 1) * 512 + (size_t)per_cta * 6 * 32) * sizeof(T) +
-           (size_t)per_cta * 14 * sizeof(int);
+size_t chip_smem(int64_t per_cta) {
+    return ((2 * (size_t)per_cta + 1) * 512 + (size_t)per_cta * 6 * 32) * sizeof(T) + (size_t)per_cta * 14 * sizeof(int);
 }
 
-template <typename T, ChipMode kMode, bool kRhsSmem>
+// How a launch divides the grid: four CTAs an SM, so that one CTA's exchange overlaps the others'
+// updates, where their shared memory fits; else one of 1,024 threads. us per half-sweep (FP32, open
+// walls) with one CTA an SM -> four of 256 threads:
+//   leaves  512: 1.61 -> 1.23   1,493: 2.26 -> 1.71   3,300: 3.46 -> 2.84   5,300: 3.92 -> 3.83
+// Up to four leaves a CTA 128 threads: 256 fill the SM's registers, so that solves of other streams
+// wait. HNS_Advance on 1,493 leaves, us alone / with three contexts taking turns: 788 / 626 with
+// 256 threads, 835 / 513 with 128.
+// FP16 conversions make its update issue-bound: beyond kChipMaxHalfLeaves leaves a CTA full grids
+// launched per colour issue it as fast (5,300 leaves 3.6 -> 3.5 us, 6,500 3.6 -> 4.0).
+constexpr int64_t kChipMaxHalfLeaves = 9;
+struct ChipShape {
+    int64_t per_cta;  // 0: the grid does not fit
+    int threads;
+};
+template <typename T>
+ChipShape chip_shape(const Context& c) {
+    const int64_t L = c.topo.num_leaves, sms = c.sm_count();
+    if (L <= 0) return {0, 0};
+    const int64_t quarter = (L + 4 * sms - 1) / (4 * sms), whole = (L + sms - 1) / sms;
+    if (sizeof(T) == 2 && quarter > kChipMaxHalfLeaves) return {0, 0};
+    if (chip_smem<T>(quarter) <= kChipSmSmem / 4 - kChipReserve) return {quarter, quarter <= 4 ? 128 : 256};
+    if (chip_smem<T>(whole) <= kChipMaxSmem - kChipReserve) return {whole, 1024};
+    return {0, 0};
+}
+
+template <typename T, ChipMode kMode>
 void launch_chip(Context& c, ChipArgs<T> A) {
     const int64_t L = c.topo.num_leaves;
-    const int sms = c.sm_count();
+    const ChipShape shape = chip_shape<T>(c);
     A.num_leaves = (int)L;
-    A.per_cta = (int)((L + sms - 1) / sms);
-    // Threads for one to three tasks a warp: more would wait at the barrier for nothing, and a small
-    // CTA leaves room on its SM for the solves of other streams.
-    const int threads = A.per_cta > 24 ? 1024 : A.per_cta > 8 ? 512 : A.per_cta > 2 ? 256 : 128;
-    auto kern = threads == 1024 ? rbgs_chip_kernel<T, kMode, kRhsSmem, 1024>
-                : threads == 512 ? rbgs_chip_kernel<T, kMode, kRhsSmem, 512>
-                : threads == 256 ? rbgs_chip_kernel<T, kMode, kRhsSmem, 256>
-                                 : rbgs_chip_kernel<T, kMode, kRhsSmem, 128>;
+    A.per_cta = (int)shape.per_cta;
+    auto kern = shape.threads == 1024  ? rbgs_chip_kernel<T, kMode, 1024>
+                : shape.threads == 256 ? rbgs_chip_kernel<T, kMode, 256>
+                                       : rbgs_chip_kernel<T, kMode, 128>;
     const unsigned blocks = (unsigned)((L + A.per_cta - 1) / A.per_cta);
     // The same limit for every context of the process, so none lowers another's.
-    HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kChipMaxSmem - 1024)));
+    HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kChipMaxSmem - kChipReserve)));
     // Face words and the abort word, cleared once. Each launch takes tags that no earlier launch of
     // the context has used, so nothing is cleared between launches; a captured launch runs with the
     // same tags at every replay, so the words are cleared before it.
@@ -463,8 +478,8 @@ void launch_chip(Context& c, ChipArgs<T> A) {
     A.counters = c.counters;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = chip_smem<T>(A.per_cta, kRhsSmem);
+    cfg.blockDim = dim3((unsigned)shape.threads);
+    cfg.dynamicSmemBytes = chip_smem<T>(A.per_cta);
     cfg.stream = c.stream;
     // Cooperative: every CTA resident at once, which the waits rely on.
     cudaLaunchAttribute attr[1];
@@ -476,24 +491,13 @@ void launch_chip(Context& c, ChipArgs<T> A) {
     HNS_LAUNCHED();
 }
 
-// Whether the grid's values (and with rhs, the right-hand side) fit the SMs' shared memory.
-// FP16 beyond kChipMaxHalfLeaves leaves an SM launches per colour: conversions make its update
-// issue-bound, and 148 CTAs of 32 warps issue it no faster than full grids do (4.0 against 3.6 us on
-// 6,594 leaves, 45 an SM; 3.3 against 3.6 on 5,300, 36 an SM).
-constexpr int64_t kChipMaxHalfLeaves = 36;
-template <typename T>
-bool fits(const Context& c, bool rhs) {
-    const int64_t L = c.topo.num_leaves;
-    const int sms = c.sm_count();
-    if (sizeof(T) == 2 && (L + sms - 1) / sms > kChipMaxHalfLeaves) return false;
-    return L > 0 && chip_smem<T>((L + sms - 1) / sms, rhs) <= kChipMaxSmem - kChipReserve;
-}
-
 }  // namespace
 
-bool chip_fits(const Context& c, size_t bytes, bool in_place_slots) {
-    // Slot-order arrays are read once, so their right-hand side has to be held.
-    return bytes == 2 ? fits<__half>(c, in_place_slots) : fits<float>(c, in_place_slots);
+bool chip_fits(const Context& c, size_t bytes, bool transpose) {
+    const ChipShape s = bytes == 2 ? chip_shape<__half>(c) : chip_shape<float>(c);
+    // One CTA an SM is no faster than full grids launched per colour, but for the transpose, which
+    // has no such form on colour-split leaves.
+    return s.per_cta > 0 && (transpose || s.threads < 1024);
 }
 
 void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,
@@ -503,14 +507,8 @@ void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rh
     A.nb8 = nb8, A.rhs = rhs, A.e = e, A.rhs_slots = rhs_slots, A.e_slots = e_slots;
     A.half_sweeps = half_sweeps, A.zero_init = e_zero, A.omega = omega, A.dx2 = dx2;
     A.check = check, A.check_mid = check_mid, A.mid_half = mid_half, A.tol2 = tol2;
-    if (fits<float>(c, true)) {
-        if (walls) launch_chip<float, kWalls, true>(c, A);
-        else launch_chip<float, kDirichlet, true>(c, A);
-    } else {
-        if (rhs_slots) fail(HNS_ERR_INVALID_ARG, "a streamed right-hand side has to be colour-split");
-        if (walls) launch_chip<float, kWalls, false>(c, A);
-        else launch_chip<float, kDirichlet, false>(c, A);
-    }
+    if (walls) launch_chip<float, kWalls>(c, A);
+    else launch_chip<float, kDirichlet>(c, A);
 }
 
 void launch_chip_solve_f16(Context& c, const int* nb8, const void* rhs, void* e, int half_sweeps, bool e_zero, float omega,
@@ -518,14 +516,14 @@ void launch_chip_solve_f16(Context& c, const int* nb8, const void* rhs, void* e,
     ChipArgs<__half> A = {};
     A.nb8 = nb8, A.rhs = static_cast<const __half*>(rhs), A.e = static_cast<__half*>(e);
     A.half_sweeps = half_sweeps, A.zero_init = e_zero, A.omega = omega, A.dx2 = 1.0f, A.check = check, A.tol2 = tol2;
-    launch_chip<__half, kDirichlet, true>(c, A);
+    launch_chip<__half, kDirichlet>(c, A);
 }
 
 void launch_chip_transpose(Context& c, const int* nb8, const float* p_bar, float* div_bar, int iterations, float omega) {
     ChipArgs<float> A = {};
     A.nb8 = nb8, A.e = const_cast<float*>(p_bar), A.bar = div_bar, A.rhs_slots = true, A.e_slots = true;
     A.half_sweeps = 2 * iterations, A.omega = omega, A.dx2 = c.dx * c.dx;
-    launch_chip<float, kTranspose, true>(c, A);
+    launch_chip<float, kTranspose>(c, A);
 }
 
 }  // namespace hns

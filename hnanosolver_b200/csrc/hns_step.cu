@@ -38,18 +38,9 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
     const float dx2 = c.dx * c.dx;
     const bool zero = (flags & HNS_SOLVE_ZERO_INIT) != 0;
     const bool walls = (flags & HNS_SOLVE_NEUMANN) != 0;
-    if (plan == nullptr && use_chip(c, 2 * K) && chip_fits(c, sizeof(float), false)) {
-        // The whole solve in one launch, p in and out in slot order; the divergence too where it is
-        // held on the chip, else it is streamed in the split layout.
-        const bool held = chip_fits(c, sizeof(float), true);
-        const float* rhs = div;
-        if (!held) {
-            float* s = c.scratch_f32("split32_rhs", (size_t)c.num_voxels());
-            convert_split_f32(c, div, s, true);
-            rhs = s;
-        }
-        launch_chip_solve_f32(c, c.split_faces(), rhs, held, p, true, 2 * K, zero, omega, dx2, walls, nullptr, nullptr, 0,
-                              0.0);
+    if (plan == nullptr && use_chip(c, 2 * K) && chip_fits(c, sizeof(float))) {
+        // The whole solve in one launch, from and to the caller's slot order.
+        launch_chip_solve_f32(c, c.split_faces(), div, true, p, true, 2 * K, zero, omega, dx2, walls, nullptr, nullptr, 0, 0.0);
         return;
     }
     const Split32 w = split32_workspace(c);
@@ -80,7 +71,7 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
         convert_split_f32(c, w.e, p, false);
         return;
     }
-    if (plan != nullptr && use_chip(c, 2 * plan->check_every) && chip_fits(c, sizeof(float), false)) {
+    if (plan != nullptr && use_chip(c, 2 * plan->check_every) && chip_fits(c, sizeof(float))) {
         // One launch from each residual evaluation to the next: iteration (c + 1) E - 1, which tests
         // the check before it, and from the second iteration on the check just evaluated.
         const int E = plan->check_every;
