@@ -206,6 +206,12 @@ void Context::release_spare_graphs() {
     spare_graphs.clear();
 }
 
+Context::SpareGraph* Context::find_graph(const std::vector<uintptr_t>& key) {
+    for (auto& g : spare_graphs)
+        if (g.key == key) return &g;
+    return nullptr;
+}
+
 double* Context::reduce_slots(int count) {
     if (count > kReduceSlots) fail(HNS_ERR_UNSUPPORTED, "more than " + std::to_string(kMaxChecks) + " convergence checks");
     if (!d_reduce.ptr) d_reduce.alloc(sizeof(double) * kReduceSlots);

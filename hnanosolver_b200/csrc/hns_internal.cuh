@@ -201,9 +201,11 @@ struct Context {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
     };
-    std::vector<SpareGraph> spare_graphs;
+    std::vector<SpareGraph> spare_graphs;  // at most kMaxSpareGraphs
+    static constexpr size_t kMaxSpareGraphs = 64;
     int spare_graph_ok = -1;
     void release_spare_graphs();
+    SpareGraph* find_graph(const std::vector<uintptr_t>& key);
     // Whether the context's stream is being captured into a graph (work enqueued now runs only
     // when the graph does: a table built under capture is not marked built).
     bool stream_capturing() const;

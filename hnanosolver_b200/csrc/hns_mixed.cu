@@ -597,8 +597,6 @@ bool capturing(const Context& c) {
     return st != cudaStreamCaptureStatusNone;
 }
 
-constexpr size_t kMaxSpareGraphs = 64;
-
 // Condition of a spare outer iteration's graph: 1 while the refinement has not converged (the
 // test every kernel of the iteration makes before it does anything).
 __global__ void spare_gate_kernel(cudaGraphConditionalHandle h, const double* __restrict__ check, double tol2) {
@@ -613,14 +611,12 @@ __global__ void spare_gate_kernel(cudaGraphConditionalHandle h, const double* __
 bool run_spare_graph(Context& c, const std::vector<uintptr_t>& key, const double* check, double tol2,
                      const std::function<void()>& body) {
     if (c.spare_graph_ok == 0) return false;
-    Context::SpareGraph* found = nullptr;
-    for (auto& g : c.spare_graphs)
-        if (g.key == key) found = &g;
+    Context::SpareGraph* found = c.find_graph(key);
     if (found == nullptr) {
         // Bounded: a step's one or two solves have at most max_outer - 1 spare iterations each. At 16
         // graphs the two solves of the fire adjoint (11 each) released and made them anew on every
         // call, 10 ms of host time a call on a 28,103-leaf grid.
-        if (c.spare_graphs.size() >= kMaxSpareGraphs) c.release_spare_graphs();
+        if (c.spare_graphs.size() >= Context::kMaxSpareGraphs) c.release_spare_graphs();
         Context::SpareGraph sg;
         sg.key = key;
         bool ok = cudaGraphCreate(&sg.graph, 0) == cudaSuccess;
