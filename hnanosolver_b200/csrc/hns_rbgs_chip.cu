@@ -11,7 +11,7 @@
 //   FP32         3.0 -> 1.1  2.1 -> 1.2   2.3 -> 1.7   2.7 -> 2.8   3.7 -> 3.8      4.3
 //   walls        3.0 -> 1.2  2.1 -> 1.3   2.8 -> 1.9   3.0 -> 3.0   4.2 -> 4.1      4.8
 //   transpose    4.1 -> 1.1  4.5 -> 1.2   6.2 -> 1.8    10 -> 3.0    14 -> 4.0   16 -> 5.0
-//   FP16         1.8 -> 1.1  2.1 -> 1.2   3.4 -> 1.7   2.8 -> 2.7   3.6 -> 3.5      3.6
+//   FP16         1.8 -> 1.1  2.1 -> 1.2   2.3 -> 1.7      2.7          3.0          3.5
 // From 3,300 leaves on the gain is the host's: one launch in place of hundreds. What is left is the
 // shared-memory pipe and instruction issue, and for small grids the exchange's L2 round trip (1.1 us
 // with nothing else to do).
@@ -428,8 +428,8 @@ size_t chip_smem(int64_t per_cta) {
 // wait. HNS_Advance on 1,493 leaves, us alone / with three contexts taking turns: 788 / 626 with
 // 256 threads, 835 / 513 with 128.
 // FP16 conversions make its update issue-bound: beyond kChipMaxHalfLeaves leaves a CTA full grids
-// launched per colour issue it as fast (5,300 leaves 3.6 -> 3.5 us, 6,500 3.6 -> 4.0).
-constexpr int64_t kChipMaxHalfLeaves = 9;
+// launched per colour issue it as fast (2,400 leaves 2.4 us either way, 4,096 2.7 against 2.9 here).
+constexpr int64_t kChipMaxHalfLeaves = 4;
 struct ChipShape {
     int64_t per_cta;  // 0: the grid does not fit
     int threads;

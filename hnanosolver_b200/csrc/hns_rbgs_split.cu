@@ -51,6 +51,11 @@ constexpr int kLeavesPerThread = 4;  // leaves a thread relaxes its row in
 constexpr int kThreads = 64 * kLeavesPerBlock;
 constexpr int kShortGridCtasPerSm = 6;  // the register limit at 80 registers and 128 threads
 constexpr int kHalfCtasPerSm = 6;       // the half-sweep kernel's launch bound
+// Grids of up to kTwoLeafLimit leaves take two leaves per thread at eight CTAs per SM: with four, less
+// than a wave of CTAs is spread unevenly over the SMs. us per half-sweep, four -> two: 1,493 leaves
+// 3.4 -> 2.3, 3,300 2.8 -> 2.7, 4,096 3.5 -> 2.7, 5,300 3.5 -> 3.0, 6,594 3.5 -> 3.8, 10,000 4.75 -> 4.8.
+constexpr int kHalfCtasPerSm2 = 8;
+constexpr int64_t kTwoLeafLimit = 6000;
 
 // nbr27 indices of the six face neighbours: (dx+1)*9 + (dy+1)*3 + (dz+1).
 constexpr int kNbXp = 22, kNbXm = 4, kNbYp = 16, kNbYm = 10, kNbZp = 14, kNbZm = 12;
@@ -120,7 +125,7 @@ __device__ __forceinline__ uint2 relax_row(uint2 XP, uint2 XM, uint2 YP, uint2 Y
 // zero leaf. Offsets are 32-bit element counts (fewer than 2^22 leaves).
 constexpr int kLeavesPerGroup = kLeavesPerBlock * kLeavesPerThread;
 
-template <bool kZero, bool kShared, bool kPdl, typename Mid>
+template <bool kZero, bool kShared, bool kPdl, int kLeaves, typename Mid>
 __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const __half* __restrict__ rhs, __half* e,
                                             int num_leaves, int g, int colour, float omega, Mid&& mid) {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;
@@ -128,22 +133,22 @@ __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const _
     const int p = (w + colour) & 1;  // z parity of this colour in the warp's rows
     const uint32_t rowc = ((uint32_t)colour << 8) | (uint32_t)(4 * (32 * w + lane));  // own entries within a leaf
     auto lde = [](const __half* q) { return kShared ? ld8_rw(q) : ld8(q); };
-    const int leaf0 = g * kLeavesPerGroup + (int)(threadIdx.x >> 6);
-    uint32_t own[kLeavesPerThread];
-    bool live[kLeavesPerThread];
+    const int leaf0 = g * (kLeavesPerBlock * kLeaves) + (int)(threadIdx.x >> 6);
+    uint32_t own[kLeaves];
+    bool live[kLeaves];
 #pragma unroll
-    for (int k = 0; k < kLeavesPerThread; ++k) {
+    for (int k = 0; k < kLeaves; ++k) {
         const int leaf = leaf0 + k * kLeavesPerBlock;
         live[k] = leaf < num_leaves;
         own[k] = ((uint32_t)(live[k] ? leaf : 0) << 9) | rowc;  // a dead slot reads leaf 0 and stores nothing
     }
-    uint2 B[kLeavesPerThread], out[kLeavesPerThread];
+    uint2 B[kLeaves], out[kLeaves];
 #pragma unroll
-    for (int k = 0; k < kLeavesPerThread; ++k) B[k] = ld8(rhs + own[k]);
+    for (int k = 0; k < kLeaves; ++k) B[k] = ld8(rhs + own[k]);
     if constexpr (kZero) {
         mid();
 #pragma unroll
-        for (int k = 0; k < kLeavesPerThread; ++k) {
+        for (int k = 0; k < kLeaves; ++k) {
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = relax1(0u, 0u, 0u, 0u, 0u, 0u, half_at(B[k], j), 0u, omega);
@@ -155,9 +160,9 @@ __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const _
         const uint32_t co = ((uint32_t)(colour ^ 1) << 8) | (uint32_t)(128 * (w ^ 1));
         auto row = [&](uint32_t n, int a2, int b2) { return (n << 9) | co | (uint32_t)(16 * a2 + 4 * (b2 >> 1)); };
         const int sx = a == 7 ? 0 : a == 0 ? 1 : 6, sy = b == 7 ? 2 : b == 0 ? 3 : 6, sz = 5 - p;
-        uint32_t nx[kLeavesPerThread], ny[kLeavesPerThread], nz[kLeavesPerThread];
+        uint32_t nx[kLeaves], ny[kLeaves], nz[kLeaves];
 #pragma unroll
-        for (int k = 0; k < kLeavesPerThread; ++k) {
+        for (int k = 0; k < kLeaves; ++k) {
             const int* nb = nb8 + 8 * (own[k] >> 9);
             nx[k] = (uint32_t)__ldg(nb + sx);
             ny[k] = (uint32_t)__ldg(nb + sy);
@@ -166,16 +171,16 @@ __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const _
         // e is written by the preceding half-sweep: wait until it has finished (a no-op for a
         // launch without the programmatic-serialization attribute).
         if constexpr (kPdl) asm volatile("griddepcontrol.wait;" ::: "memory");
-        uint2 C[kLeavesPerThread], K[kLeavesPerThread], XP[kLeavesPerThread], XM[kLeavesPerThread],
-            YP[kLeavesPerThread], YM[kLeavesPerThread];
-        uint32_t ZC[kLeavesPerThread];
+        uint2 C[kLeaves], K[kLeaves], XP[kLeaves], XM[kLeaves],
+            YP[kLeaves], YM[kLeaves];
+        uint32_t ZC[kLeaves];
 #pragma unroll
-        for (int k = 0; k < kLeavesPerThread; ++k) {
+        for (int k = 0; k < kLeaves; ++k) {
             C[k] = ld8_rw(e + own[k]);
             K[k] = lde(e + (own[k] ^ 256u));
         }
 #pragma unroll
-        for (int k = 0; k < kLeavesPerThread; ++k) {
+        for (int k = 0; k < kLeaves; ++k) {
             const uint32_t lf = own[k] >> 9;
             XP[k] = lde(e + row(a == 7 ? nx[k] : lf, (a + 1) & 7, b));
             XM[k] = lde(e + row(a == 0 ? nx[k] : lf, (a - 1) & 7, b));
@@ -186,20 +191,20 @@ __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const _
         }
         mid();  // every load of the pass is in flight
 #pragma unroll
-        for (int k = 0; k < kLeavesPerThread; ++k)
+        for (int k = 0; k < kLeaves; ++k)
             out[k] = p ? relax_row<1>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega)
                        : relax_row<0>(XP[k], XM[k], YP[k], YM[k], K[k], ZC[k], B[k], C[k], omega);
     }
 #pragma unroll
-    for (int k = 0; k < kLeavesPerThread; ++k)
+    for (int k = 0; k < kLeaves; ++k)
         if (live[k]) *reinterpret_cast<uint2*>(e + own[k]) = out[k];
 }
 
 // One half-sweep per launch. Leaf groups: one per CTA in a full grid; a short grid loops. Within
 // a launch a thread reads and writes only its own rows of the launch's colour and only reads the
 // other colour, so the passes of a CTA are independent.
-template <bool kZero>
-__global__ void __launch_bounds__(kThreads, kHalfCtasPerSm) rbgs_split_half_kernel(const int* __restrict__ nb8,
+template <bool kZero, int kLeaves>
+__global__ void __launch_bounds__(kThreads, kLeaves == 4 ? kHalfCtasPerSm : kHalfCtasPerSm2) rbgs_split_half_kernel(const int* __restrict__ nb8,
                                                                     const __half* __restrict__ rhs, __half* e,
                                                                     int num_leaves, int colour, float omega,
                                                                     const double* __restrict__ check, double tol2,
@@ -210,9 +215,10 @@ __global__ void __launch_bounds__(kThreads, kHalfCtasPerSm) rbgs_split_half_kern
     // blocks take the SM slots this launch's last wave frees and load what no sweep writes
     // before they wait for this launch to finish.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int groups = (num_leaves + kLeavesPerGroup - 1) / kLeavesPerGroup;
+    constexpr int kPerGroup = kLeavesPerBlock * kLeaves;
+    const int groups = (num_leaves + kPerGroup - 1) / kPerGroup;
     for (int g = blockIdx.x; g < groups; g += gridDim.x)
-        relax_group<kZero, false, true>(nb8, rhs, e, num_leaves, g, colour, omega, [] {});
+        relax_group<kZero, false, true, kLeaves>(nb8, rhs, e, num_leaves, g, colour, omega, [] {});
 }
 
 // ---- FP32 ---------------------------------------------------------------------------------
@@ -387,6 +393,7 @@ __global__ void __launch_bounds__(kF32Threads, kF32ShortGridCtasPerSm)
 // other wait watches, and every CTA returns, leaving e unfinished. `unreachable` (0 but in the
 // test of that path) raises every wait's target out of reach.
 constexpr uint32_t kSolveMaxPolls = 1u << 20;
+static_assert(kLeavesPerThread == 4, "the half-sweep kernel's forms");
 static_assert(kThreads == kF32Threads, "one block shape for both precisions");
 static_assert(64 + 6 * kLeavesPerGroup + 1 <= kThreads, "dependency threads");
 
@@ -479,9 +486,9 @@ __global__ void __launch_bounds__(kThreads, kShortGridCtasPerSm) rbgs_split_solv
         };
         if constexpr (kHalf) {
             if (kZeroFirst && h == 0)
-                relax_group<true, true, false>(nb8, rhs, e, num_leaves, g, 0, omega, mid);
+                relax_group<true, true, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, 0, omega, mid);
             else
-                relax_group<false, true, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, mid);
+                relax_group<false, true, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, h & 1, omega, mid);
         } else {
             if (kZeroFirst && h == 0)
                 relax_group_f32<true, true, false, false>(nb8, rhs, e, num_leaves, g, 0, omega, dx2, mid);
@@ -644,7 +651,8 @@ void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, v
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     if (L >= (int64_t(1) << 22)) fail(HNS_ERR_INVALID_ARG, "too many leaves for the colour-split inner solve");
-    const int per_block = kLeavesPerBlock * kLeavesPerThread;
+    const bool two = L <= kTwoLeafLimit;
+    const int per_block = kLeavesPerBlock * (two ? 2 : kLeavesPerThread);
     unsigned blocks = (unsigned)((L + per_block - 1) / per_block);
     // A launch that will most likely return at once (the refinement expected to have converged)
     // uses one wave of CTAs: its cost is then the launch, not the scheduling of every CTA.
@@ -661,7 +669,7 @@ void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, v
     if (e_zero) {
         cfg.numAttrs = c.add_inner_window(attr, 0);
         cfg.attrs = attr;
-        HNS_CUDA(cudaLaunchKernelEx(&cfg, rbgs_split_half_kernel<true>, nb8, r, x, (int)L, colour, omega, check, tol2,
+        HNS_CUDA(cudaLaunchKernelEx(&cfg, two ? rbgs_split_half_kernel<true, 2> : rbgs_split_half_kernel<true, 4>, nb8, r, x, (int)L, colour, omega, check, tol2,
                                     c.counters));
         HNS_LAUNCHED();
         return;
@@ -676,7 +684,7 @@ void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, v
     na = c.add_inner_window(attr, na);
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    HNS_CUDA(cudaLaunchKernelEx(&cfg, rbgs_split_half_kernel<false>, nb8, r, x, (int)L, colour, omega, check, tol2,
+    HNS_CUDA(cudaLaunchKernelEx(&cfg, two ? rbgs_split_half_kernel<false, 2> : rbgs_split_half_kernel<false, 4>, nb8, r, x, (int)L, colour, omega, check, tol2,
                                 c.counters));
     HNS_LAUNCHED();
 }

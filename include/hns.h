@@ -502,7 +502,7 @@ HNS_API hns_status hns_adjoint_advance_mixed(hns_ctx* ctx, const hns_fire_fields
                                      between convergence checks, leaf groups ordered by per-group
                                      progress counters instead of launch boundaries. */
 #define HNS_SPLIT_AUTO 2        /*   default: where the grid's values fit the SMs' shared memory (FP32 up
-                                     to about 3.3M voxels; FP16 up to 2.7M), one cooperative launch per
+                                     to about 3.3M voxels; FP16 up to 1.2M), one cooperative launch per
                                      solve that keeps them there from the first half-sweep to the last,
                                      else one launch per half-sweep. All three give the same results to
                                      the bit. */
