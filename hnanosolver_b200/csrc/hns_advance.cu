@@ -26,10 +26,12 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hns_confine.cuh"
 #include "hns_internal.cuh"
+#include "hns_rows.cuh"
 #include "hns_stencil.cuh"
 
 namespace hns {
@@ -144,66 +146,85 @@ struct Burn {
 // temperature_buoyancy (Kernel.cu:546-563) from the burned temperature, with the density term
 // v.y -= alpha density dt when alpha != 0, into a separate velocity buffer (neighbouring
 // threads still read `vel`).
-template <int kModel>
-__global__ void __launch_bounds__(kThreads) div_combust_buoy_kernel(TopoView t, const float* __restrict__ vel,
-                                                                     float* __restrict__ vel_out, float* __restrict__ div,
-                                                                     float inv_dx, float* __restrict__ fuel,
-                                                                     float* __restrict__ waste, float* __restrict__ temp,
-                                                                     float* __restrict__ flame,
-                                                                     const float* __restrict__ density, Burn B, float dt,
-                                                                     float ambient, float strength) {
-    __shared__ LeafNbhd L;
-    const VoxelIdx v = voxel_of_block();
-    load_nbhd(L, t, v.leaf);
-    __syncthreads();
-    const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
-    const int64_t s = (v.leaf << 9) + v.n;
-    const float3 c = ld3(vel, s);
-    const float xp = (c.x + near_v(t, L, vel, i + 1, j, k).x) * 0.5f;
-    const float xm = (c.x + near_v(t, L, vel, i - 1, j, k).x) * 0.5f;
-    const float yp = (c.y + near_v(t, L, vel, i, j + 1, k).y) * 0.5f;
-    const float ym = (c.y + near_v(t, L, vel, i, j - 1, k).y) * 0.5f;
-    const float zp = (c.z + near_v(t, L, vel, i, j, k + 1).z) * 0.5f;
-    const float zm = (c.z + near_v(t, L, vel, i, j, k - 1).z) * 0.5f;
-    float dv = (xp - xm + yp - ym + zp - zm) * inv_dx;
-
-    float Tn = temp[s];
-    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) {
-        float f = fuel[s];
-        const float w = waste[s], T = Tn, fl = flame[s];
-        if (f < 0.001f) f = 0.0f;
-        const float oxy = 1.0f - f - w;
-        if (oxy < 0.0f) {
-            fuel[s] = f;
+// Half z-rows (hns_rows.cuh): four voxels a thread, each array as vector loads; kVec false where one
+// of them is not aligned for that.
+template <int kModel, bool kVec>
+__global__ void __launch_bounds__(kRowThreads) div_combust_buoy_kernel(TopoView t, const float* __restrict__ vel,
+                                                                       float* __restrict__ vel_out, float* __restrict__ div,
+                                                                       float inv_dx, float* __restrict__ fuel,
+                                                                       float* __restrict__ waste, float* __restrict__ temp,
+                                                                       float* __restrict__ flame,
+                                                                       const float* __restrict__ density, Burn B, float dt,
+                                                                       float ambient, float strength) {
+    HalfRow row;
+    if (!half_row(t, row, blockIdx.x)) return;
+    const int64_t s = row.own;
+    float3 c[4];
+    float dv[4], T4[4], f4[4], w4[4], fl4[4], d4[4];
+    half_row_divergence<kVec>(row, vel, inv_dx, c, dv);
+    // In-place fields: read and written by this thread alone.
+    auto get = [&](const float* p, float v[4]) {
+        if constexpr (kVec) {
+            const float4 q = *reinterpret_cast<const float4*>(p + s);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
         } else {
-            const float burn = fminf(oxy, f);
-            fuel[s] = f - burn;
-            waste[s] = w + burn * 2.0f;
-            Tn = T + burn * B.gain;
-            temp[s] = Tn;
-            dv += burn * B.expansion;
-            flame[s] = fmaxf(fl, fminf(1.0f, burn * 10.0f));
+#pragma unroll
+            for (int z = 0; z < 4; ++z) v[z] = p[s + z];
         }
-    } else if constexpr (kModel == HNS_COMBUSTION_RATE) {
-        const float f = fuel[s];
-        if (f > 0.0f && Tn >= B.ignition) {
-            const float burned = fminf(f, B.rate * dt);
-            fuel[s] = f - burned;
-            Tn = Tn + burned * B.heat;
-            temp[s] = Tn;
+    };
+    get(temp, T4);
+    if constexpr (kModel != HNS_COMBUSTION_NONE) get(fuel, f4);
+    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) get(waste, w4), get(flame, fl4);
+    if (B.alpha != 0.0f && density != nullptr) scalar_row<kVec>(density, s, d4);
+    float3 u[4];
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        float Tn = T4[z];
+        if constexpr (kModel == HNS_COMBUSTION_OXYGEN) {
+            float f = f4[z];
+            const float w = w4[z], T = Tn, fl = fl4[z];
+            if (f < 0.001f) f = 0.0f;
+            const float oxy = 1.0f - f - w;
+            if (oxy < 0.0f) {
+                f4[z] = f;
+            } else {
+                const float burn = fminf(oxy, f);
+                f4[z] = f - burn;
+                w4[z] = w + burn * 2.0f;
+                Tn = T + burn * B.gain;
+                dv[z] += burn * B.expansion;
+                fl4[z] = fmaxf(fl, fminf(1.0f, burn * 10.0f));
+            }
+        } else if constexpr (kModel == HNS_COMBUSTION_RATE) {
+            const float f = f4[z];
+            if (f > 0.0f && Tn >= B.ignition) {
+                const float burned = fminf(f, B.rate * dt);
+                f4[z] = f - burned;
+                Tn = Tn + burned * B.heat;
+            }
+        }
+        T4[z] = Tn;
+        if (B.alpha != 0.0f) {
+            const float bt = Tn > ambient ? fmaxf(0.0f, (Tn - ambient) * strength) : 0.0f;
+            const float fy = bt - B.alpha * (density != nullptr ? d4[z] : 0.0f);
+            u[z] = make_float3(c[z].x, c[z].y + fy * dt, c[z].z);
+        } else if (Tn <= ambient) {
+            u[z] = c[z];
+        } else {
+            const float by = fmaxf(0.0f, (Tn - ambient) * strength);
+            u[z] = make_float3(c[z].x + 0.0f * dt, c[z].y + by * dt, c[z].z + 0.0f * dt);
         }
     }
-    div[s] = dv;
-    if (B.alpha != 0.0f) {
-        const float bt = Tn > ambient ? fmaxf(0.0f, (Tn - ambient) * strength) : 0.0f;
-        const float fy = bt - B.alpha * (density != nullptr ? __ldg(density + s) : 0.0f);
-        st3(vel_out, s, make_float3(c.x, c.y + fy * dt, c.z));
-    } else if (Tn <= ambient) {
-        st3(vel_out, s, c);
-    } else {
-        const float by = fmaxf(0.0f, (Tn - ambient) * strength);
-        st3(vel_out, s, make_float3(c.x + 0.0f * dt, c.y + by * dt, c.z + 0.0f * dt));
+    store_scalar_row<kVec>(div, s, dv);
+    if constexpr (kModel != HNS_COMBUSTION_NONE) {
+        store_scalar_row<kVec>(fuel, s, f4);
+        store_scalar_row<kVec>(temp, s, T4);
     }
+    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) {
+        store_scalar_row<kVec>(waste, s, w4);
+        store_scalar_row<kVec>(flame, s, fl4);
+    }
+    store_vel_row<kVec>(vel_out, s, u);
 }
 
 unsigned leaf_blocks(const Context& c) { return (unsigned)(c.topo.num_leaves * 2); }
@@ -215,18 +236,19 @@ void launch_div_combust_buoy(const Context& c, const float* vel, float* vel_out,
                              const hns_force_model& M, float dt) {
     const Burn B{P.temperatureRelease, P.expansionRate, M.burn_rate, M.heat_release, M.ignition_temp, M.density_buoyancy};
     const float inv_dx = 1.0f / c.dx;
-    if (M.combustion == HNS_COMBUSTION_OXYGEN)
-        div_combust_buoy_kernel<HNS_COMBUSTION_OXYGEN><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-            c.topo.view, vel, vel_out, div, inv_dx, fuel, waste, temp, flame, density, B, dt, P.ambientTemp,
-            P.buoyancyStrength);
-    else if (M.combustion == HNS_COMBUSTION_RATE)
-        div_combust_buoy_kernel<HNS_COMBUSTION_RATE><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-            c.topo.view, vel, vel_out, div, inv_dx, fuel, waste, temp, flame, density, B, dt, P.ambientTemp,
-            P.buoyancyStrength);
-    else
-        div_combust_buoy_kernel<HNS_COMBUSTION_NONE><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-            c.topo.view, vel, vel_out, div, inv_dx, fuel, waste, temp, flame, density, B, dt, P.ambientTemp,
-            P.buoyancyStrength);
+    bool vec = true;
+    for (const float* p : {vel, (const float*)vel_out, (const float*)div, (const float*)fuel, (const float*)waste,
+                           (const float*)temp, (const float*)flame, density})
+        vec = vec && row_aligned(p, sizeof(float));
+    auto pick = [&](auto model) {
+        constexpr int m = decltype(model)::value;
+        return vec ? div_combust_buoy_kernel<m, true> : div_combust_buoy_kernel<m, false>;
+    };
+    auto kern = M.combustion == HNS_COMBUSTION_OXYGEN ? pick(std::integral_constant<int, HNS_COMBUSTION_OXYGEN>{})
+                : M.combustion == HNS_COMBUSTION_RATE ? pick(std::integral_constant<int, HNS_COMBUSTION_RATE>{})
+                                                      : pick(std::integral_constant<int, HNS_COMBUSTION_NONE>{});
+    kern<<<row_blocks(c), kRowThreads, 0, c.stream>>>(c.topo.view, vel, vel_out, div, inv_dx, fuel, waste, temp, flame,
+                                                      density, B, dt, P.ambientTemp, P.buoyancyStrength);
     HNS_LAUNCHED();
 }
 

@@ -28,9 +28,11 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
 #include "hns_confine.cuh"
 #include "hns_internal.cuh"
+#include "hns_rows.cuh"
 #include "hns_stencil.cuh"
 #include "hns_types.cuh"
 
@@ -155,72 +157,82 @@ struct BurnParams {
     float alpha;                 // density buoyancy; 0: the reference's temperature_buoyancy
 };
 
-__device__ __forceinline__ float opt_load(const __half* p, int64_t s) { return p != nullptr ? sload(p, s) : 0.0f; }
-
 // divergence (Kernel.cu:432-453) of the forced velocity; the scalar sources (add_scalar_source,
 // Kernel.cu:732-737: temperature, density, fuel); the force model's burn (combustion_oxygen,
 // Kernel.cu:641-677, with the expansion added to the divergence; combustion, Kernel.cu:568-588;
 // or none); then temperature_buoyancy (Kernel.cu:546-563) from the burned temperature, with the
 // density term when alpha != 0, into vel_out (neighbouring threads still read vel).
-template <int kModel>
-__global__ void __launch_bounds__(kThreads) div_burn_buoy_mixed_kernel(TopoView t, const bf16* __restrict__ vel,
-                                                                        bf16* __restrict__ vel_out, float* __restrict__ div,
-                                                                        float inv_dx, FireScalars S, BurnParams B, float dt,
-                                                                        float ambient, float strength) {
-    __shared__ LeafNbhd L;
-    const VoxelIdx v = voxel_of_block();
-    load_nbhd(L, t, v.leaf);
-    __syncthreads();
-    const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
-    const int64_t s = (v.leaf << 9) + v.n;
-    const float3 c = vload(vel, s);
-    const float xp = (c.x + near_b(t, L, vel, i + 1, j, k).x) * 0.5f;
-    const float xm = (c.x + near_b(t, L, vel, i - 1, j, k).x) * 0.5f;
-    const float yp = (c.y + near_b(t, L, vel, i, j + 1, k).y) * 0.5f;
-    const float ym = (c.y + near_b(t, L, vel, i, j - 1, k).y) * 0.5f;
-    const float zp = (c.z + near_b(t, L, vel, i, j, k + 1).z) * 0.5f;
-    const float zm = (c.z + near_b(t, L, vel, i, j, k - 1).z) * 0.5f;
-    float dv = (xp - xm + yp - ym + zp - zm) * inv_dx;
-
-    float T = opt_load(S.temp_in, s);
-    if (S.src_temp != nullptr) T += dt * sload(S.src_temp, s);
-    float D = opt_load(S.dens_in, s);
-    if (S.src_dens != nullptr) D += dt * sload(S.src_dens, s);
-    float F = opt_load(S.fuel_in, s);
-    if (S.src_fuel != nullptr) F += dt * sload(S.src_fuel, s);
-    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) {
-        float W = sload(S.waste_in, s), FL = sload(S.flame_in, s);
-        if (F < 0.001f) F = 0.0f;
-        const float oxy = 1.0f - F - W;
-        if (oxy >= 0.0f) {
-            const float burn = fminf(oxy, F);
-            F = F - burn;
-            W = W + burn * 2.0f;
-            T = T + burn * B.gain;
-            dv += burn * B.expansion;
-            FL = fmaxf(FL, fminf(1.0f, burn * 10.0f));
+// Half z-rows (hns_rows.cuh): four voxels a thread, each array as vector loads; kVec false where one
+// of them is not aligned for that.
+template <int kModel, bool kVec>
+__global__ void __launch_bounds__(kRowThreads) div_burn_buoy_mixed_kernel(TopoView t, const bf16* __restrict__ vel,
+                                                                          bf16* __restrict__ vel_out,
+                                                                          float* __restrict__ div, float inv_dx,
+                                                                          FireScalars S, BurnParams B, float dt,
+                                                                          float ambient, float strength) {
+    HalfRow row;
+    if (!half_row(t, row, blockIdx.x)) return;
+    const int64_t s = row.own;
+    float3 c[4];
+    float dv[4], T4[4], D4[4], F4[4], W4[4], FL4[4];
+    half_row_divergence<kVec>(row, vel, inv_dx, c, dv);
+    auto field = [&](const __half* in, const __half* src, float v[4]) {
+        if (in != nullptr) {
+            scalar_row<kVec>(in, s, v);
+        } else {
+#pragma unroll
+            for (int z = 0; z < 4; ++z) v[z] = 0.0f;
         }
-        sstore(S.waste_out, s, W);
-        sstore(S.flame_out, s, FL);
-    } else if constexpr (kModel == HNS_COMBUSTION_RATE) {
-        if (F > 0.0f && T >= B.ignition) {
-            const float burned = fminf(F, B.rate * dt);
-            F = F - burned;
-            T = T + burned * B.heat;
+        if (src != nullptr) {
+            float a[4];
+            scalar_row<kVec>(src, s, a);
+#pragma unroll
+            for (int z = 0; z < 4; ++z) v[z] += dt * a[z];
+        }
+    };
+    field(S.temp_in, S.src_temp, T4);
+    field(S.dens_in, S.src_dens, D4);
+    field(S.fuel_in, S.src_fuel, F4);
+    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) field(S.waste_in, nullptr, W4), field(S.flame_in, nullptr, FL4);
+    float3 u[4];
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        float T = T4[z], F = F4[z];
+        if constexpr (kModel == HNS_COMBUSTION_OXYGEN) {
+            float W = W4[z], FL = FL4[z];
+            if (F < 0.001f) F = 0.0f;
+            const float oxy = 1.0f - F - W;
+            if (oxy >= 0.0f) {
+                const float burn = fminf(oxy, F);
+                F = F - burn;
+                W = W + burn * 2.0f;
+                T = T + burn * B.gain;
+                dv[z] += burn * B.expansion;
+                FL = fmaxf(FL, fminf(1.0f, burn * 10.0f));
+            }
+            W4[z] = W, FL4[z] = FL;
+        } else if constexpr (kModel == HNS_COMBUSTION_RATE) {
+            if (F > 0.0f && T >= B.ignition) {
+                const float burned = fminf(F, B.rate * dt);
+                F = F - burned;
+                T = T + burned * B.heat;
+            }
+        }
+        T4[z] = T, F4[z] = F;
+        u[z] = c[z];
+        if (B.alpha != 0.0f) {
+            const float bt = T > ambient ? fmaxf(0.0f, (T - ambient) * strength) : 0.0f;
+            u[z].y = c[z].y + (bt - B.alpha * D4[z]) * dt;
+        } else if (T > ambient) {
+            u[z].y = c[z].y + fmaxf(0.0f, (T - ambient) * strength) * dt;
         }
     }
-    div[s] = dv;
-    if (S.temp_out != nullptr) sstore(S.temp_out, s, T);
-    if (S.fuel_out != nullptr) sstore(S.fuel_out, s, F);
-    if (S.dens_out != nullptr) sstore(S.dens_out, s, D);
-    float3 r = c;
-    if (B.alpha != 0.0f) {
-        const float bt = T > ambient ? fmaxf(0.0f, (T - ambient) * strength) : 0.0f;
-        r.y = c.y + (bt - B.alpha * D) * dt;
-    } else if (T > ambient) {
-        r.y = c.y + fmaxf(0.0f, (T - ambient) * strength) * dt;
-    }
-    vstore(vel_out, s, r);
+    store_scalar_row<true>(div, s, dv);
+    if constexpr (kModel == HNS_COMBUSTION_OXYGEN) store_scalar_row<kVec>(S.waste_out, s, W4), store_scalar_row<kVec>(S.flame_out, s, FL4);
+    if (S.temp_out != nullptr) store_scalar_row<kVec>(S.temp_out, s, T4);
+    if (S.fuel_out != nullptr) store_scalar_row<kVec>(S.fuel_out, s, F4);
+    if (S.dens_out != nullptr) store_scalar_row<kVec>(S.dens_out, s, D4);
+    store_vel_row<kVec>(vel_out, s, u);
 }
 
 constexpr int kFireFields = 5;  // density, temperature, fuel, waste, flame
@@ -424,15 +436,20 @@ RefinePlan run_advance_mixed(Context& c, const hns_fire_fields& in, const hns_fi
             adv_in[kWaste] = S.waste_out;
             adv_in[kFlame] = S.flame_out;
         }
-        if (M.combustion == HNS_COMBUSTION_OXYGEN)
-            div_burn_buoy_mixed_kernel<HNS_COMBUSTION_OXYGEN><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-                c.topo.view, adv2, nxt.vel, div, inv_dx, S, B, dt_sub, P.ambientTemp, P.buoyancyStrength);
-        else if (M.combustion == HNS_COMBUSTION_RATE)
-            div_burn_buoy_mixed_kernel<HNS_COMBUSTION_RATE><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-                c.topo.view, adv2, nxt.vel, div, inv_dx, S, B, dt_sub, P.ambientTemp, P.buoyancyStrength);
-        else
-            div_burn_buoy_mixed_kernel<HNS_COMBUSTION_NONE><<<leaf_blocks(c), kThreads, 0, c.stream>>>(
-                c.topo.view, adv2, nxt.vel, div, inv_dx, S, B, dt_sub, P.ambientTemp, P.buoyancyStrength);
+        bool vec = true;
+        for (const void* q : {(const void*)adv2, (const void*)nxt.vel, (const void*)S.temp_in, (const void*)S.fuel_in,
+                              (const void*)S.waste_in, (const void*)S.flame_in, (const void*)S.dens_in,
+                              (const void*)S.src_temp, (const void*)S.src_fuel, (const void*)S.src_dens})
+            vec = vec && row_aligned(q, 2);
+        auto pick = [&](auto model) {
+            constexpr int m = decltype(model)::value;
+            return vec ? div_burn_buoy_mixed_kernel<m, true> : div_burn_buoy_mixed_kernel<m, false>;
+        };
+        auto kern = M.combustion == HNS_COMBUSTION_OXYGEN ? pick(std::integral_constant<int, HNS_COMBUSTION_OXYGEN>{})
+                    : M.combustion == HNS_COMBUSTION_RATE ? pick(std::integral_constant<int, HNS_COMBUSTION_RATE>{})
+                                                          : pick(std::integral_constant<int, HNS_COMBUSTION_NONE>{});
+        kern<<<row_blocks(c), kRowThreads, 0, c.stream>>>(c.topo.view, adv2, nxt.vel, div, inv_dx, S, B, dt_sub, P.ambientTemp,
+                                                          P.buoyancyStrength);
         HNS_LAUNCHED();
         c.phase_end();
 

@@ -12,10 +12,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "hns_advect_tile.cuh"
 #include "hns_scalars_tile.cuh"
 #include "hns_internal.cuh"
+#include "hns_rows.cuh"
 #include "hns_stencil.cuh"
 
 namespace hns {
@@ -152,25 +154,6 @@ __global__ void __launch_bounds__(kThreads) advect_scalars_kernel(TopoView t, co
 }
 
 // ---- projection -----------------------------------------------------------------------------
-
-// divergence (src/Cuda/Kernel.cu:432-453).
-__global__ void __launch_bounds__(kThreads) divergence_kernel(TopoView t, const float* __restrict__ vel,
-                                                               float* __restrict__ div, float inv_dx) {
-    __shared__ LeafNbhd L;
-    const VoxelIdx v = voxel_of_block();
-    load_nbhd(L, t, v.leaf);
-    __syncthreads();
-    const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
-    const int64_t s = (v.leaf << 9) + v.n;
-    const float3 c = ld3(vel, s);
-    const float xp = (c.x + near_v(t, L, vel, i + 1, j, k).x) * 0.5f;
-    const float xm = (c.x + near_v(t, L, vel, i - 1, j, k).x) * 0.5f;
-    const float yp = (c.y + near_v(t, L, vel, i, j + 1, k).y) * 0.5f;
-    const float ym = (c.y + near_v(t, L, vel, i, j - 1, k).y) * 0.5f;
-    const float zp = (c.z + near_v(t, L, vel, i, j, k + 1).z) * 0.5f;
-    const float zm = (c.z + near_v(t, L, vel, i, j, k - 1).z) * 0.5f;
-    div[s] = (xp - xm + yp - ym + zp - zm) * inv_dx;
-}
 
 constexpr int PT = 12;  // pressure tile edge: leaf + two-voxel halo (local -2..9)
 constexpr int RT = 10;  // divergence tile edge: leaf + one-voxel halo (local -1..8)
@@ -329,10 +312,8 @@ __global__ void __launch_bounds__(kThreads) rbgs_iteration_kernel(TopoView t, co
     }
 }
 
-// subtractPressureGradient (src/Cuda/Kernel.cu:495-541); sdf (or null): the collision
-// treatment of the result (Kernel.cu:528-538).
-// kNeumann: zero-gradient walls, a missing neighbour's pressure is the voxel's own.
-template <bool kNeumann>
+// subtractPressureGradient (src/Cuda/Kernel.cu:495-541) with the collision treatment of the result
+// (Kernel.cu:528-538); without a collider, gradient_rows_kernel.
 __global__ void __launch_bounds__(kThreads) subtract_gradient_kernel(TopoView t, const float* __restrict__ vel,
                                                                       const float* __restrict__ p,
                                                                       float* __restrict__ out, float inv_dx,
@@ -344,20 +325,12 @@ __global__ void __launch_bounds__(kThreads) subtract_gradient_kernel(TopoView t,
     const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
     const int64_t s = (v.leaf << 9) + v.n;
     const float h = 0.5f * inv_dx;
-    auto pn = [&](int x, int y, int z) {
-        if constexpr (kNeumann) {
-            const int64_t q = slot_of(t, L, x, y, z);
-            return q < 0 ? __ldg(p + s) : __ldg(p + q);
-        } else {
-            return near_s(t, L, p, x, y, z);
-        }
-    };
-    const float gx = (pn(i + 1, j, k) - pn(i - 1, j, k)) * h;
-    const float gy = (pn(i, j + 1, k) - pn(i, j - 1, k)) * h;
-    const float gz = (pn(i, j, k + 1) - pn(i, j, k - 1)) * h;
+    const float gx = (near_s(t, L, p, i + 1, j, k) - near_s(t, L, p, i - 1, j, k)) * h;
+    const float gy = (near_s(t, L, p, i, j + 1, k) - near_s(t, L, p, i, j - 1, k)) * h;
+    const float gz = (near_s(t, L, p, i, j, k + 1) - near_s(t, L, p, i, j, k - 1)) * h;
     const float3 u = ld3(vel, s);
     float3 r = make_float3(u.x - gx, u.y - gy, u.z - gz);
-    if (sdf != nullptr) collide(t, L, sdf, s, i, j, k, inv_dx, 0.1f, r);
+    collide(t, L, sdf, s, i, j, k, inv_dx, 0.1f, r);
     st3(out, s, r);
 }
 
@@ -543,7 +516,11 @@ void launch_collision_enforce(const Context& c, float* vel, const float* sdf) {
 }
 
 void launch_divergence(const Context& c, const float* vel, float* div) {
-    divergence_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, div, 1.0f / c.dx);
+    const float inv_dx = 1.0f / c.dx;
+    const bool v = row_aligned(vel, sizeof(float)), d = row_aligned(div, sizeof(float));
+    auto kern = v ? (d ? divergence_rows_kernel<float, true, true> : divergence_rows_kernel<float, true, false>)
+                  : (d ? divergence_rows_kernel<float, false, true> : divergence_rows_kernel<float, false, false>);
+    kern<<<row_blocks(c), kRowThreads, 0, c.stream>>>(c.topo.view, vel, div, inv_dx);
     HNS_LAUNCHED();
 }
 
@@ -567,14 +544,21 @@ void launch_rbgs_iteration(const Context& c, const float* div, const float* p_in
 
 void launch_subtract_gradient(const Context& c, const float* vel, const float* p, float* out, const float* sdf,
                               unsigned flags) {
-    if (flags & HNS_SOLVE_NEUMANN) {
-        if (sdf) fail(HNS_ERR_UNSUPPORTED, "zero-gradient walls do not take a collider");
-        subtract_gradient_kernel<true><<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, p, out, 1.0f / c.dx,
-                                                                                    nullptr);
-    } else {
-        subtract_gradient_kernel<false><<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, p, out,
-                                                                                     1.0f / c.dx, sdf);
+    const bool walls = (flags & HNS_SOLVE_NEUMANN) != 0;
+    if (walls && sdf) fail(HNS_ERR_UNSUPPORTED, "zero-gradient walls do not take a collider");
+    if (sdf != nullptr) {
+        subtract_gradient_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(c.topo.view, vel, p, out, 1.0f / c.dx, sdf);
+        HNS_LAUNCHED();
+        return;
     }
+    const bool v = row_aligned(vel, sizeof(float)) && row_aligned(out, sizeof(float)), q = row_aligned(p, sizeof(float));
+    auto pick = [&](auto w) {
+        constexpr bool kW = decltype(w)::value;
+        return v ? (q ? gradient_rows_kernel<kW, true, true> : gradient_rows_kernel<kW, true, false>)
+                 : (q ? gradient_rows_kernel<kW, false, true> : gradient_rows_kernel<kW, false, false>);
+    };
+    auto kern = walls ? pick(std::true_type{}) : pick(std::false_type{});
+    kern<<<row_blocks(c), kRowThreads, 0, c.stream>>>(c.topo.view, vel, p, out, 1.0f / c.dx);
     HNS_LAUNCHED();
 }
 
