@@ -30,7 +30,7 @@
 #include <string>
 #include <type_traits>
 
-#include "hns_confine.cuh"
+#include "hns_confine_rows.cuh"
 #include "hns_internal.cuh"
 #include "hns_rows.cuh"
 #include "hns_stencil.cuh"
@@ -107,31 +107,23 @@ __global__ void __launch_bounds__(kThreads) confine_mixed_kernel(TopoView t, con
     vstore(out, s, r);
 }
 
-// confine_mixed_kernel on a shared-memory leaf tile (hns_confine.cuh), for |fs| <= 1: one CTA
-// per leaf, the same values.
-__global__ void __launch_bounds__(kThreads) confine_tile_mixed_kernel(TopoView t, const bf16* __restrict__ vel,
-                                                                       bf16* __restrict__ out, float dt, float inv_dx,
-                                                                       float scale, int fs, const bf16* __restrict__ src_v3,
-                                                                       float gravity) {
-    __shared__ LeafNbhd L;
-    __shared__ ConfineTile T;
-    const int64_t leaf = blockIdx.x;
-    load_nbhd(L, t, leaf);
-    __syncthreads();
-    confine_tile(L, vel, T, 0.5f * inv_dx);
-    for (int n = threadIdx.x; n < 512; n += blockDim.x) {
-        const int64_t s = (leaf << 9) + n;
-        float3 r = confine_at(T, n >> 6, (n >> 3) & 7, n & 7, fs, inv_dx, dt, scale);
-        if (src_v3 != nullptr) {
-            const float3 a = vload(src_v3, s);
-            r.x += a.x * dt;
-            r.y += a.y * dt;
-            r.z += a.z * dt;
+// What follows the confinement of a half row: the velocity source and gravity.
+struct AfterConfinementMixed {
+    const bf16* src_v3;
+    float dt, gravity;
+    __device__ __forceinline__ void operator()(int64_t s0, float3 u[4]) const {
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+            if (src_v3 != nullptr) {
+                const float3 a = vload(src_v3, s0 + z);
+                u[z].x += a.x * dt;
+                u[z].y += a.y * dt;
+                u[z].z += a.z * dt;
+            }
+            if (gravity != 0.0f) u[z].y -= gravity * dt;
         }
-        if (gravity != 0.0f) r.y -= gravity * dt;
-        vstore(out, s, r);
     }
-}
+};
 
 // The scalar fields of one pass (FP16; null: absent) and the burned outputs (null: the pass
 // leaves that field unchanged and writes nothing).
@@ -399,15 +391,16 @@ RefinePlan run_advance_mixed(Context& c, const hns_fire_fields& in, const hns_fi
 
         c.phase_begin(HNS_PHASE_FORCES);
         const int fs = (int)P.factorScale;
-        if (fs >= -1 && fs <= 1)
-            confine_tile_mixed_kernel<<<(unsigned)c.topo.num_leaves, kThreads, 0, c.stream>>>(
-                c.topo.view, adv, adv2, dt_sub, inv_dx, P.vorticityScale, fs, static_cast<const bf16*>(src.velocity),
-                P.gravity);
-        else
+        if (fs >= -1 && fs <= 1) {
+            // div is not written yet: the pass's scratch.
+            launch_confine_rows(c, adv, adv2, div, dt_sub, P.vorticityScale, fs,
+                                AfterConfinementMixed{static_cast<const bf16*>(src.velocity), dt_sub, P.gravity});
+        } else {
             confine_mixed_kernel<<<leaf_blocks(c), kThreads, 0, c.stream>>>(
                 c.topo.view, adv, adv2, dt_sub, inv_dx, P.vorticityScale, fs, static_cast<const bf16*>(src.velocity),
                 P.gravity);
-        HNS_LAUNCHED();
+            HNS_LAUNCHED();
+        }
         // The burned scalars: the fields this pass changes go to solver-owned arrays, which the
         // scalar advection then reads; the others are advected from the substep's input.
         FireScalars S{};

@@ -332,7 +332,7 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
     float* div = arena + 6 * n;
     FieldSet none{};
     launch_advect_fused(c, in.velocity, adv, none, dt);
-    launch_confine_sources(c, adv, adv2, dt, P.vorticityScale, P.factorScale, src.velocity, P.gravity);
+    launch_confine_sources(c, adv, adv2, div, dt, P.vorticityScale, P.factorScale, src.velocity, P.gravity);
     float* s1[kFields] = {};
     float* s2[kFields] = {};
     for (int f = 0; f < kFields; ++f) {

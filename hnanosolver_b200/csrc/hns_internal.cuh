@@ -428,10 +428,11 @@ void launch_gradient_f64(const Context& c, float* vel, const double* p);
 void run_advance(Context& c, int iterations, float dt, const hns_combustion_params& params, const hns_force_model& model,
                  const hns_step_desc* solve, hns_solve_info* info);
 void check_force_model(const hns_force_model& m);
-// The step's force kernels (hns_advance.cu): confinement + velocity source + gravity, vel -> out;
+// The step's force kernels (hns_advance.cu): confinement + velocity source + gravity, vel -> out,
+// with mag (a float per voxel, 16-byte aligned) as scratch;
 // divergence + burn (in place on its fields) + buoyancy, vel -> vel_out.
-void launch_confine_sources(const Context& c, const float* vel, float* out, float dt, float scale, float factor_scale,
-                            const float* src_v3, float gravity);
+void launch_confine_sources(const Context& c, const float* vel, float* out, float* mag, float dt, float scale,
+                            float factor_scale, const float* src_v3, float gravity);
 void launch_div_combust_buoy(const Context& c, const float* vel, float* vel_out, float* div, float* fuel, float* waste,
                              float* temp, float* flame, const float* density, const hns_combustion_params& P,
                              const hns_force_model& M, float dt);
