@@ -3,8 +3,8 @@
 // arithmetic, and the pressure solves as the FP64 iterative refinement of hns_step_mixed.
 //
 // Per substep:
-//   advect_records / advect_mixed   velocity -> adv                     (advect_vector)
-//   confine_mixed                   adv -> adv2, + velocity source,     (vorticityConfinement out
+//   advect_tile                     velocity -> adv                     (advect_vector)
+//   curl_rows + confine_rows        adv -> adv2, + velocity source,     (vorticityConfinement out
 //                                   gravity                              of place, add_velocity_source,
 //                                                                        add_gravity)
 //   div_burn_buoy_mixed             adv2 -> div, adv3 (= out velocity);  (divergence, add_scalar_source,
@@ -13,8 +13,8 @@
 //   refined solve                   div -> p (FP64)                      (redBlackGaussSeidelUpdate loop,
 //   [divergence of adv3, refined solve]  disturbanceEnable > 0           to a tolerance)
 //   gradient_mixed                  out velocity -= grad p, in place     (subtractPressureGradient)
-//   pack_fire_records +             scalars -> out scalars along the     (advect_scalars)
-//   advect_scalars_records          projected velocity
+//   advect_scalars_half_tile        scalars -> out scalars along the     (advect_scalars)
+//                                   projected velocity
 // The scalar sources are pointwise and independent of the velocity, so adding them in the
 // divergence pass instead of the confinement pass (where HNS_Advance launches them) gives the
 // same values, and the sourced value feeds the burn in FP32 without an FP16 rounding between.
@@ -33,6 +33,7 @@
 #include "hns_confine_rows.cuh"
 #include "hns_internal.cuh"
 #include "hns_rows.cuh"
+#include "hns_scalars_tile.cuh"
 #include "hns_stencil.cuh"
 #include "hns_types.cuh"
 
@@ -229,111 +230,15 @@ __global__ void __launch_bounds__(kRowThreads) div_burn_buoy_mixed_kernel(TopoVi
 
 constexpr int kFireFields = 5;  // density, temperature, fuel, waste, flame
 
-struct HalfFields {
-    const __half* in[kFireFields];
-    __half* out[kFireFields];
-    int count;
-};
-
-// Voxel records for the scalar advection: the BF16 velocity and up to five FP16 scalars in 16
-// bytes (u | v << 16, w | s0 << 16, s1 | s2 << 16, s3 | s4 << 16; absent scalars 0), so that each
-// of the 2 x 8 trace taps and 6 clamp neighbours is one load instead of one per field.
-__global__ void __launch_bounds__(kThreads) pack_fire_records_kernel(const bf16* __restrict__ vel, HalfFields f,
-                                                                      uint4* __restrict__ rec, int64_t n) {
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned short* v = reinterpret_cast<const unsigned short*>(vel) + 3 * s;
-        uint32_t h[kFireFields] = {0u, 0u, 0u, 0u, 0u};
-#pragma unroll
-        for (int q = 0; q < kFireFields; ++q)
-            if (q < f.count) h[q] = __half_as_ushort(__ldg(f.in[q] + s));
-        rec[s] = make_uint4((uint32_t)__ldg(v) | ((uint32_t)__ldg(v + 1) << 16), (uint32_t)__ldg(v + 2) | (h[0] << 16),
-                            h[1] | (h[2] << 16), h[3] | (h[4] << 16));
-    }
-}
-
-__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-__device__ __forceinline__ float hf(uint32_t w, int hi) {
-    return __half2float(__ushort_as_half((unsigned short)(hi ? (w >> 16) : (w & 0xFFFFu))));
-}
-// Scalar q of a record (word 1 high half, then words 2 and 3).
-__device__ __forceinline__ float rec_s(const uint4& r, int q) {
-    return q == 0 ? hf(r.y, 1) : q == 1 ? hf(r.z, 0) : q == 2 ? hf(r.z, 1) : q == 3 ? hf(r.w, 0) : hf(r.w, 1);
-}
-
-// HNS_Advance's multi-field advection (advect_scalars, src/Cuda/Kernel.cu:163-289) on FP16
-// fields along a BF16 velocity, from voxel records: the back-trace uses the voxel's own
-// velocity, the taps' weight-sum trilinear (setupInterpolation, Kernel.cu:204-233) reads slot 0
-// outside the domain, and the MacCormack correction is clamped to the centre, its six face
-// neighbours and the forward sample; the FP32 step's operations in its order, one 16-byte load
-// per tap for the velocity and every field.
-// I: the slot type, int32_t where the grid has fewer than 2^22 leaves (32-bit addressing).
-template <int kCount, typename I>
-__global__ void __launch_bounds__(kThreads) advect_scalars_records_kernel(TopoView t, const uint4* __restrict__ rec,
-                                                                           HalfFields f, float sdt) {
-    __shared__ LeafNbhd L;
-    const VoxelIdx v = voxel_of_block();
-    load_nbhd(L, t, v.leaf);
-    __syncthreads();
-    const int i = (L.lx << 3) + (v.n >> 6), j = (L.ly << 3) + ((v.n >> 3) & 7), k = (L.lz << 3) + (v.n & 7);
-    const I s = (I(v.leaf) << 9) + I(v.n);
-    const uint4 o = __ldg(rec + s);
-    const float bx = (float)i - bf_lo(o.x) * sdt, by = (float)j - bf_hi(o.x) * sdt, bz = (float)k - bf_lo(o.y) * sdt;
-    I bi[8], fi[8], ni[6];
-    float bw[8], fw[8];
-    interp_setup_fast<I>(t, L, bx, by, bz, bi, bw);
-    float3 vf = make_float3(0.f, 0.f, 0.f);
-    float pf[kCount], pb[kCount];
-#pragma unroll
-    for (int c = 0; c < kCount; ++c) pf[c] = 0.f, pb[c] = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const uint4 a = __ldg(rec + bi[q]);
-        vf.x = vf.x + bf_lo(a.x) * bw[q];
-        vf.y = vf.y + bf_hi(a.x) * bw[q];
-        vf.z = vf.z + bf_lo(a.y) * bw[q];
-#pragma unroll
-        for (int c = 0; c < kCount; ++c) pf[c] = __fmaf_rn(rec_s(a, c), bw[q], pf[c]);
-    }
-    interp_setup_fast<I>(t, L, bx + vf.x * sdt, by + vf.y * sdt, bz + vf.z * sdt, fi, fw);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const uint4 a = __ldg(rec + fi[q]);
-#pragma unroll
-        for (int c = 0; c < kCount; ++c) pb[c] = __fmaf_rn(rec_s(a, c), fw[q], pb[c]);
-    }
-    face_slots(L, s, v.n, ni);  // x-1, x+1, y-1, y+1, z-1, z+1
-#pragma unroll
-    for (int q = 0; q < 6; ++q) ni[q] = ni[q] < 0 ? I(0) : ni[q];  // outside the domain: slot 0
-    float mn[kCount], mx[kCount], po[kCount];
-#pragma unroll
-    for (int c = 0; c < kCount; ++c) po[c] = rec_s(o, c), mn[c] = po[c], mx[c] = po[c];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const uint4 a = __ldg(rec + ni[q]);
-#pragma unroll
-        for (int c = 0; c < kCount; ++c) {
-            const float x = rec_s(a, c);
-            mn[c] = fminf(mn[c], x);
-            mx[c] = fmaxf(mx[c], x);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < kCount; ++c) {
-        const float corr = __fmaf_rn(0.5f, po[c] - pb[c], pf[c]);
-        sstore(f.out[c], (int64_t)s, fmaxf(fminf(mn[c], pf[c]), fminf(corr, fmaxf(mx[c], pf[c]))));
-    }
-}
-
 template <typename I>
-void launch_advect_scalars_records(const Context& c, const uint4* rec, const HalfFields& f, float sdt) {
-    const dim3 g = leaf_blocks(c);
-    switch (f.count) {
-        case 1: advect_scalars_records_kernel<1, I><<<g, kThreads, 0, c.stream>>>(c.topo.view, rec, f, sdt); break;
-        case 2: advect_scalars_records_kernel<2, I><<<g, kThreads, 0, c.stream>>>(c.topo.view, rec, f, sdt); break;
-        case 3: advect_scalars_records_kernel<3, I><<<g, kThreads, 0, c.stream>>>(c.topo.view, rec, f, sdt); break;
-        case 4: advect_scalars_records_kernel<4, I><<<g, kThreads, 0, c.stream>>>(c.topo.view, rec, f, sdt); break;
-        default: advect_scalars_records_kernel<5, I><<<g, kThreads, 0, c.stream>>>(c.topo.view, rec, f, sdt); break;
+void launch_scalars_half(const Context& c, const bf16* vel, const HalfScalarPass& P, float sdt) {
+    const unsigned g = (unsigned)c.topo.num_leaves;
+    switch (P.count) {
+        case 1: advect_scalars_half_tile_kernel<1, I><<<g, kTileThreads, 0, c.stream>>>(c.topo.view, vel, P, sdt); break;
+        case 2: advect_scalars_half_tile_kernel<2, I><<<g, kTileThreads, 0, c.stream>>>(c.topo.view, vel, P, sdt); break;
+        case 3: advect_scalars_half_tile_kernel<3, I><<<g, kTileThreads, 0, c.stream>>>(c.topo.view, vel, P, sdt); break;
+        case 4: advect_scalars_half_tile_kernel<4, I><<<g, kTileThreads, 0, c.stream>>>(c.topo.view, vel, P, sdt); break;
+        default: advect_scalars_half_tile_kernel<5, I><<<g, kTileThreads, 0, c.stream>>>(c.topo.view, vel, P, sdt); break;
     }
     HNS_LAUNCHED();
 }
@@ -461,25 +366,31 @@ RefinePlan run_advance_mixed(Context& c, const hns_fire_fields& in, const hns_fi
         c.phase_end();
 
         c.phase_begin(HNS_PHASE_ADVECT);
-        HalfFields f{};
+        HalfScalarPass f{};
         for (int q = 0; q < kFireFields; ++q)
             if (cur.s[q]) {
                 f.in[f.count] = adv_in[q];
                 f.out[f.count] = nxt.s[q];
                 ++f.count;
             }
+        // The advection reads its inputs while it writes: one that overlaps an output (a caller that
+        // passes a field's input as another field's output) is read from a copy.
+        for (int q = 0; q < f.count; ++q)
+            for (int r = 0; r < f.count; ++r) {
+                const uintptr_t i = reinterpret_cast<uintptr_t>(f.in[q]), o = reinterpret_cast<uintptr_t>(f.out[r]);
+                if (i < o + 2 * n && o < i + 2 * n) {
+                    __half* copy = half_scratch(c, "fire_copy_" + std::to_string(q), n);
+                    HNS_CUDA(cudaMemcpyAsync(copy, f.in[q], n * sizeof(__half), cudaMemcpyDeviceToDevice, c.stream));
+                    f.in[q] = copy;
+                    break;
+                }
+            }
         if (f.count > 0) {
-            // Voxel records of the projected velocity and the fields, then one load per tap.
-            uint4* rec = reinterpret_cast<uint4*>(c.scratch_f32("fire_records", 4 * n));
-            const unsigned pg = (unsigned)std::min<int64_t>((int64_t)(n + kThreads - 1) / kThreads,
-                                                            (int64_t)c.sm_count() * 8);
-            pack_fire_records_kernel<<<pg, kThreads, 0, c.stream>>>(nxt.vel, f, rec, (int64_t)n);
-            HNS_LAUNCHED();
             const float sdt = dt_sub * inv_dx;
             if (c.topo.num_leaves < (int64_t(1) << 22))
-                launch_advect_scalars_records<int32_t>(c, rec, f, sdt);
+                launch_scalars_half<int32_t>(c, nxt.vel, f, sdt);
             else
-                launch_advect_scalars_records<int64_t>(c, rec, f, sdt);
+                launch_scalars_half<int64_t>(c, nxt.vel, f, sdt);
         }
         c.phase_end();
         cur = nxt;
