@@ -157,3 +157,21 @@ def test_unaligned_fp32_arrays(dev, name, walls):
         got.append((div, out, sv, sd))
     for x, y in zip(*got):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["one", "corner", "spheres"])
+def test_multigrid_on_small_and_shuffled_grids(dev, name):
+    """The level transfers where every side of a leaf is missing, where two leaves touch at a corner only,
+    and where neighbours lie anywhere in the order: a transfer that reads a wrong cell does not
+    converge in the cycles that the sorted grids need (at most 12 refinements of two)."""
+    from hnanosolver_b200 import lib as hl
+
+    o = np.array([[0, 0, 0], [8, 8, 8]], np.int32) if name == "corner" else _origins(name)
+    grid = hl.Grid(o, voxel_size=0.1)
+    vel, (d,) = _fields(grid.num_voxels, dev, 1, 2.0)
+    v, d = vel.bfloat16(), d.half()
+    vo, do = torch.empty_like(v), torch.empty_like(d)
+    torch.cuda.synchronize()
+    info = grid.step_mixed(v, vo, [d], [do], hl.MixedDesc(dt=0.1, omega=1.9, tolerance=1e-5, max_outer=12, inner_iterations=2,
+                                                          flags=hl.SOLVE_MULTIGRID), info=True)
+    assert info.residual <= 1e-5
