@@ -169,19 +169,26 @@ void Topology::build(const int32_t* leaf_origins, int64_t n, cudaStream_t stream
             nbr[(size_t)l * 27 + q] = v;
         }
     }
-    d_origin.alloc(sizeof(int4) * (size_t)n);
-    d_nbr27.alloc(sizeof(int32_t) * nbr.size());
+    int4* d_origin;
+    int* d_nbr27;
+    alloc_leaves(n, d_origin, d_nbr27);
     d_lookup.alloc(sizeof(int32_t) * lookup.size());
-    HNS_CUDA(cudaMemcpyAsync(d_origin.ptr, org.data(), d_origin.bytes, cudaMemcpyHostToDevice, stream));
-    HNS_CUDA(cudaMemcpyAsync(d_nbr27.ptr, nbr.data(), d_nbr27.bytes, cudaMemcpyHostToDevice, stream));
+    HNS_CUDA(cudaMemcpyAsync(d_origin, org.data(), sizeof(int4) * (size_t)n, cudaMemcpyHostToDevice, stream));
+    HNS_CUDA(cudaMemcpyAsync(d_nbr27, nbr.data(), sizeof(int32_t) * nbr.size(), cudaMemcpyHostToDevice, stream));
     HNS_CUDA(cudaMemcpyAsync(d_lookup.ptr, lookup.data(), d_lookup.bytes, cudaMemcpyHostToDevice, stream));
     HNS_CUDA(cudaStreamSynchronize(stream));  // host vectors go out of scope
-    view.num_leaves = n;
-    view.origin = d_origin.as<int4>();
-    view.nbr27 = d_nbr27.as<int>();
     view.lookup = d_lookup.as<int>();
     view.lo_x = lo[0], view.lo_y = lo[1], view.lo_z = lo[2];
     view.dim_x = (int)dims[0], view.dim_y = (int)dims[1], view.dim_z = (int)dims[2];
+}
+
+void Topology::alloc_leaves(int64_t n, int4*& origin, int*& nbr27) {
+    d_leaves.alloc((sizeof(int4) + 27 * sizeof(int32_t)) * (size_t)n);
+    origin = d_leaves.as<int4>();
+    nbr27 = reinterpret_cast<int*>(origin + n);
+    view.num_leaves = n;
+    view.origin = origin;
+    view.nbr27 = nbr27;
 }
 
 // ---- context ---------------------------------------------------------------------------------

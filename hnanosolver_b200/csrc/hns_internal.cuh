@@ -91,8 +91,12 @@ struct TopoView {
 struct Topology {
     int64_t num_leaves = 0;
     std::vector<int32_t> origins;  // host copy, 3 per leaf
-    DeviceBuffer d_origin, d_nbr27, d_lookup;
+    // The leaf tables: origins and 27-neighbour table in one block (an allocation of its own costs the
+    // host 0.3 ms, and as much again when it is freed), the lookup table.
+    DeviceBuffer d_leaves, d_lookup;
     TopoView view{};
+    // Allocates d_leaves for n leaves and points the view into it.
+    void alloc_leaves(int64_t n, int4*& origin, int*& nbr27);
     bool nanovdb_order = false;
     void build(const int32_t* leaf_origins, int64_t n, cudaStream_t stream);
     // The leaves that the active voxels ijk (int32 [3 n], host or device) touch after a

@@ -8,7 +8,7 @@
 //   1. The voxels' bounding box (and the check of their range): one read of the list.
 //   2. A flag per leaf of the dilated bounding box, in the leaf lookup table that the grid needs
 //      anyway: per voxel the leaves its dilation box reaches (per axis: -1 when z & 7 < padding,
-//      +1 when (z & 7) + padding >= 8), found once per warp where its voxels share a leaf.
+//      +1 when (z & 7) + padding >= 8), found once per warp for its voxels of one leaf.
 //   3. NanoVDB leaf order is root tile, then upper-node child, then lower-node child, each in
 //      x, y, z order (PointsToGrid orders leaves this way). A lower node is 16^3 leaves, so the flags
 //      are counted and then numbered node by node, the nodes in that order: one CTA per node of
@@ -17,7 +17,9 @@
 //      only the origins go back to the host (the context keeps a host copy).
 // Bound by the two reads of the voxel list and by the call's allocations and three host waits: the
 // band of a 512^3 shell (12M voxels, padding 2, 46,000 leaves), context made and destroyed, took
-// 8.7 ms with a radix sort of one key per voxel (1.4 ms of kernels, 300 MB of temporary arrays).
+// 8.7 ms with a radix sort of one key per voxel (1.4 ms of kernels, 300 MB of temporary arrays), 2.1 ms
+// with the tables in three allocations, and takes 1.7 ms with them in two (0.23 ms of kernels; an
+// allocation and its release cost the host 0.6 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -86,30 +88,25 @@ __global__ void __launch_bounds__(kTopoThreads) flag_kernel(const int32_t* __res
             c[d] = (v >> 3) - box.lo[d];
             reach[d] = 2u | ((v & 7) < padding ? 1u : 0u) | ((v & 7) + padding >= 8 ? 4u : 0u);
         }
-    uint32_t m = 0;
-#pragma unroll
-    for (int k = 0; k < 27; ++k)
-        if (((reach[0] >> (k / 9)) & 1u) && ((reach[1] >> ((k / 3) % 3)) & 1u) && ((reach[2] >> (k % 3)) & 1u)) m |= 1u << k;
-    auto at = [&](int k) {
-        return ((int64_t)(c[0] + k / 9 - 1) * box.dim[1] + (c[1] + (k / 3) % 3 - 1)) * box.dim[2] + (c[2] + k % 3 - 1);
-    };
-    // A flag already set is not written again: the list's voxels set few flags many times.
-    auto set = [&](int k) {
-        int* f = flags + at(k);
-        if (*reinterpret_cast<volatile int*>(f) == 0) *f = 1;
-    };
-    const int64_t leaf = ((int64_t)c[0] * box.dim[1] + c[1]) * box.dim[2] + c[2];
-    const int64_t first = __shfl_sync(0xffffffffu, leaf, 0);
-    if (__all_sync(0xffffffffu, live && leaf == first)) {
-        const uint32_t all = __reduce_or_sync(0xffffffffu, m);
-        const int lane = threadIdx.x & 31;
-        if (lane < 27 && ((all >> lane) & 1u)) set(lane);
-    } else {
-        while (m) {
-            const int k = __ffs(m) - 1;
-            m &= m - 1;
-            set(k);
-        }
+    const uint32_t row = ((reach[1] & 1u) ? reach[2] : 0u) | ((reach[1] & 2u) ? reach[2] << 3 : 0u) | ((reach[1] & 4u) ? reach[2] << 6 : 0u);
+    const uint32_t m = ((reach[0] & 1u) ? row : 0u) | ((reach[0] & 2u) ? row << 9 : 0u) | ((reach[0] & 4u) ? row << 18 : 0u);
+    // The warp's voxels by leaf: the lanes of one leaf share its reached neighbours out. (Bit k of m:
+    // neighbour (k / 9, k / 3 % 3, k % 3) - 1; at most 2^28 leaves in the box.)
+    const int leaf = live ? (int)(((int64_t)c[0] * box.dim[1] + c[1]) * box.dim[2] + c[2]) : -1;
+    const unsigned mates = __match_any_sync(0xffffffffu, leaf);
+    uint32_t all = __reduce_or_sync(mates, m);
+    if (!live) return;
+    unsigned below;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(below));
+    const int size = __popc(mates);
+    int turn = __popc(mates & below);
+    for (; all; all &= all - 1, turn = turn == 0 ? size - 1 : turn - 1) {
+        if (turn != 0) continue;
+        const int k = __ffs(all) - 1;
+        int* f = flags + ((int64_t)(c[0] + k / 9 - 1) * box.dim[1] + (c[1] + k / 3 % 3 - 1)) * box.dim[2] + (c[2] + k % 3 - 1);
+        // A flag already set is not written again: the list's voxels set few flags many times (a stale 0
+        // from this SM's cache costs a write).
+        if (*f == 0) *f = 1;
     }
 }
 
@@ -291,23 +288,21 @@ void Topology::build_from_voxels(const int32_t* ijk, int64_t n, bool ijk_on_devi
     HNS_CUDA(cudaStreamSynchronize(s));
 
     num_leaves = L;
-    d_origin.alloc(sizeof(int4) * (size_t)L);
-    d_nbr27.alloc(sizeof(int32_t) * 27 * (size_t)L);
+    int4* d_origin;
+    int* d_nbr27;
+    alloc_leaves(L, d_origin, d_nbr27);
     // The origins for the host pass through the neighbour table's memory, which is written after.
-    int* org3 = d_nbr27.as<int>();
+    int* org3 = d_nbr27;
     number_kernel<<<(unsigned)num_nodes, kTopoThreads, 0, s>>>(d_nodes.as<int3>(), box, first.as<int>(), d_lookup.as<int>(),
-                                                               d_origin.as<int4>(), org3);
+                                                               d_origin, org3);
     HNS_LAUNCHED();
     origins.resize((size_t)L * 3);
     HNS_CUDA(cudaMemcpyAsync(origins.data(), org3, sizeof(int32_t) * origins.size(), cudaMemcpyDeviceToHost, s));
     nanovdb_order = true;
-    view.num_leaves = L;
-    view.origin = d_origin.as<int4>();
-    view.nbr27 = d_nbr27.as<int>();
     view.lookup = d_lookup.as<int>();
     view.lo_x = box.lo[0], view.lo_y = box.lo[1], view.lo_z = box.lo[2];
     view.dim_x = box.dim[0], view.dim_y = box.dim[1], view.dim_z = box.dim[2];
-    nbr27_kernel<<<grid_for(L), kTopoThreads, 0, s>>>(d_origin.as<int4>(), L, view, d_nbr27.as<int>());
+    nbr27_kernel<<<grid_for(L), kTopoThreads, 0, s>>>(d_origin, L, view, d_nbr27);
     HNS_LAUNCHED();
     HNS_CUDA(cudaStreamSynchronize(s));
 }
