@@ -351,7 +351,7 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
         p64 = reinterpret_cast<double*>(sf(c, "p64", 2 * n));
         const float om = S.refined->omega > 0.f ? S.refined->omega : 1.9f;
         refine_solve<__half>(c, div, p64, S.refined->max_outer, S.refined->inner_iterations, om, S.refined->tolerance,
-                             S.refined->flags | kSolvePlainSmoothing);
+                             S.refined->flags);
         HNS_CUDA(cudaMemcpyAsync(velp, adv3, 3 * n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
         launch_gradient_f64(c, velp, p64);
     } else {
@@ -405,7 +405,7 @@ void adjoint_fire(Context& c, const hns_fire_f32& in, const hns_fire_sources_f32
         // div_bar = dx^2 L^-1 p_bar: the refined solve of p_bar as a divergence.
         const float om = S.refined->omega > 0.f ? S.refined->omega : 1.9f;
         refine_solve<__half>(c, pbar, p64, S.refined->max_outer, S.refined->inner_iterations, om, S.refined->tolerance,
-                             S.refined->flags | kSolvePlainSmoothing);
+                             S.refined->flags);
         convert_array(c, p64, HNS_DTYPE_F64, dbar, HNS_DTYPE_F32, nn);
     } else {
         adj_rbgs(c, pbar, dbar, S.iterations, S.omega, arena + 8 * n);

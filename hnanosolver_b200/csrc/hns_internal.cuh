@@ -328,14 +328,7 @@ int max_leaf_depth(Context& c);
 // memory limit, 1 the persisting-L2 limit. Returns the value now in force (>= value).
 size_t raise_device_setting(int device, int which, size_t value);
 // One V-cycle of the FP16 inner solve on the colour-split layout (e in place; e_zero: e = 0 before).
-// plain: two Gauss-Seidel iterations at every level instead of the over-relaxed schedule.
-void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_zero, const double* check, double tol2,
-                 bool plain);
-// A refine_solve flag: multigrid cycles with plain smoothing. The adjoints' solves take it: a
-// gradient's branches (clamps, trace cells) follow the recomputed forward, and another iterate within
-// the same tolerance flips some of them, moving single voxels of the gradient by up to 6.5e-3 of its
-// rms on fire512.
-constexpr unsigned kSolvePlainSmoothing = 1u << 30;
+void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_zero, const double* check, double tol2);
 // The FP16 inner solve on colour-split leaves (hns_rbgs_split.cu): the face-neighbour table
 // (8 ints per leaf, missing neighbours = the zero leaf L) and one in-place half-sweep (colour 0
 // red, 1 black). e holds L + 1 leaves, the last all zeros. e_zero: e = 0 before this red

@@ -644,14 +644,13 @@ RefinePlan refine_solve(Context& c, const float* div, double* p, int max_outer, 
     // colour-split half-sweep as the fine smoother (mg16_vcycle); other layouts and the FP32
     // inner solve take the FP32 V-cycle in slot order below.
     const bool mg16 = (flags & HNS_SOLVE_MULTIGRID) && sizeof(TI) == 2 && layout == HNS_INNER_SPLIT;
-    const bool plain = (flags & kSolvePlainSmoothing) != 0;
     auto mg16_iteration = [&](int k, unsigned gk) {
         const double* chk = plan.slots + 2 * k;
         refine_scale_split_kernel<<<gk, kThreads, 0, c.stream>>>(r, reinterpret_cast<__half*>(rhat), n, chk, tol2,
                                                                  scales + k);
         HNS_LAUNCHED();
         c.phase_begin(HNS_PHASE_INNER);
-        for (int cyc = 0; cyc < plan.inner; ++cyc) mg16_vcycle(c, nb8, rhat, e_split, cyc == 0, chk, tol2, plain);
+        for (int cyc = 0; cyc < plan.inner; ++cyc) mg16_vcycle(c, nb8, rhat, e_split, cyc == 0, chk, tol2);
         c.phase_end();
         refine_update_split_kernel<<<gk, kThreads, 0, c.stream>>>(p, reinterpret_cast<const __half*>(e_split), n,
                                                                   scales + k, chk, tol2, k == 0);
@@ -676,8 +675,7 @@ RefinePlan refine_solve(Context& c, const float* div, double* p, int max_outer, 
                     (uintptr_t)rhat, (uintptr_t)e_split, (uintptr_t)nb8, (uintptr_t)plan.slots, (uintptr_t)scales,
                     (uintptr_t)plan.max_outer, (uintptr_t)n,
                     (uintptr_t)c.coarse_solve, (uintptr_t)c.coarse_cluster_ok, (uintptr_t)c.split_solve,
-                    (uintptr_t)c.first_wait_polls, (uintptr_t)c.inner_window.num_bytes, (uintptr_t)tol_bits,
-                    (uintptr_t)plain};
+                    (uintptr_t)c.first_wait_polls, (uintptr_t)c.inner_window.num_bytes, (uintptr_t)tol_bits};
                 if (run_spare_graph(c, key, chk, tol2, [&] { mg16_iteration(k, gk); })) continue;
             }
             mg16_iteration(k, gk);

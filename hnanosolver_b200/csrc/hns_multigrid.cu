@@ -945,22 +945,12 @@ void mg_vcycle(Context& c, const float* b0, float* u0, const double* check, doub
 }
 
 // One V-cycle of the FP16 inner solve L e = r^ (unit spacing) on the colour-split layout: e is
-// refined in place (e_zero: e = 0 before the cycle). Fine level: kMgNuFine red-black iterations of
-// the colour-split half-sweep before and after the coarse correction; levels with
+// refined in place (e_zero: e = 0 before the cycle). Fine level: kMgNu red-black iterations of
+// the colour-split half-sweep at omega = 1 before and after the coarse correction; levels with
 // 4, 2 and 1 cells per leaf side in FP32 with the wall-corrected operator, kMgNu iterations
 // before and after at the first two, SOR sweeps at the last (coarsest_schedule).
 namespace {
-// Over-relaxed red-black smoothing: in three dimensions a factor near 1.2 smooths about twice as
-// well per sweep as 1 (Yavneh, "On red-black SOR smoothing in multigrid", SIAM J. Sci. Comput. 17,
-// 1996), so one fine iteration before and after takes the place of two. Residual after six cycles
-// (three refinements of two), fine iterations / factor fine and coarse: 2 + 2 / 1, 1; 1 + 1 / 1.2, 1.2;
-// 1 + 1 / 1.15, 1.25; 1 + 1 with 1 + 2 coarse / 1.15, 1.25:
-//   shell512 2.3e-6, 3.2e-6, 2.9e-6, 1.2e-5     fire1024 1.8e-6, 1.9e-6, 1.7e-6, 6.9e-6
-//   plume256 1.4e-6, 1.3e-6, 1.2e-6, 5.8e-6     256^3 box 9.7e-6, 9.9e-6, 9.4e-6, 1.0e-5
-// and on 14 more boxes, shells and unions of spheres at most 2.3e-6, 2.9e-6, 2.6e-6, 1.1e-5. A fine
-// half-sweep is 16 of a cycle's 380 us on shell512; the cycle had eight.
-constexpr int kMgNuFine = 1, kMgNu = 2;
-constexpr float kMgOmegaFine = 1.15f, kMgOmega = 1.25f;
+constexpr int kMgNu = 2;
 
 // SOR sweeps and factor at the coarsest level (one cell per leaf), from how many leaves deep the
 // domain is (D, max_leaf_depth): clamp(2 D + 2, 10, 20) sweeps at clamp(2 / (1 + sin(pi / 2 D)),
@@ -1110,8 +1100,7 @@ void coarsest_solve(Context& c, const int4* nb8, float* u, const float* b, int s
 }
 }  // namespace
 
-void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_zero, const double* check, double tol2,
-                 bool plain) {
+void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_zero, const double* check, double tol2) {
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     const TopoView t = c.topo.view;
@@ -1125,21 +1114,19 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
         u[l] = c.scratch_f32("mg16_u" + std::to_string(l), cells);
         b[l] = c.scratch_f32("mg16_b" + std::to_string(l), cells);
     }
-    const int nu = plain ? kMgNu : kMgNuFine;
-    const float omega_fine = plain ? 1.0f : kMgOmegaFine, omega_coarse = plain ? 1.0f : kMgOmega;
     auto fine = [&](bool zero_first) {
-        for (int it = 0; it < nu; ++it) {
-            launch_rbgs_split_half(c, nb8, rhat, e, 0, zero_first && it == 0, omega_fine, check, tol2, false);
-            launch_rbgs_split_half(c, nb8, rhat, e, 1, false, omega_fine, check, tol2, false);
+        for (int it = 0; it < kMgNu; ++it) {
+            launch_rbgs_split_half(c, nb8, rhat, e, 0, zero_first && it == 0, 1.0f, check, tol2, false);
+            launch_rbgs_split_half(c, nb8, rhat, e, 1, false, 1.0f, check, tol2, false);
         }
     };
     fine(e_zero);
-    launch_pdl(c, mg16_restrict_kernel, L << 4, f8, (const __half*)eh, r, b[1], u[1], (int)L, omega_coarse,
+    launch_pdl(c, mg16_restrict_kernel, L << 4, f8, (const __half*)eh, r, b[1], u[1], (int)L, 1.0f,
                level_h2(1), level_gamma(1), check, tol2);
-    smooth_level<2>(c, f8, u[1], b[1], kMgNu, omega_coarse, 1, true, check, tol2);
+    smooth_level<2>(c, f8, u[1], b[1], kMgNu, 1.0f, 1, true, check, tol2);
     launch_pdl(c, restrict_level1_kernel, L << 2, f8, (const float*)u[1], (const float*)b[1], b[2], u[2], (int)L, 0.25f,
-               level_gamma(1), omega_coarse, level_h2(2), level_gamma(2), check, tol2);
-    smooth_level<1>(c, f8, u[2], b[2], kMgNu, omega_coarse, 2, true, check, tol2);
+               level_gamma(1), 1.0f, level_h2(2), level_gamma(2), check, tol2);
+    smooth_level<1>(c, f8, u[2], b[2], kMgNu, 1.0f, 2, true, check, tol2);
     launch_pdl(c, mgl_restrict_kernel<1>, L, f8, (const float*)u[2], (const float*)b[2], b[3], (int)L, 1.0f / 16.0f,
                0.6f, check, tol2);
     int coarse_sweeps;
@@ -1147,9 +1134,9 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
     coarsest_schedule(c, coarse_sweeps, coarse_omega);
     coarsest_solve(c, f8, u[3], b[3], coarse_sweeps, coarse_omega, check, tol2);
     launch_pdl(c, mgl_prolong_kernel<1>, L, t, (const float*)u[3], u[2], check, tol2);
-    smooth_level<1>(c, f8, u[2], b[2], kMgNu, omega_coarse, 2, false, check, tol2);
+    smooth_level<1>(c, f8, u[2], b[2], kMgNu, 1.0f, 2, false, check, tol2);
     launch_pdl(c, prolong_level2_kernel, L << 2, t, (const float*)u[2], u[1], check, tol2);
-    smooth_level<2>(c, f8, u[1], b[1], kMgNu, omega_coarse, 1, false, check, tol2);
+    smooth_level<2>(c, f8, u[1], b[1], kMgNu, 1.0f, 1, false, check, tol2);
     launch_pdl(c, mg16_prolong_kernel, L << 4, t, (const float*)u[1], eh, check, tol2);
     fine(false);
 }
