@@ -207,56 +207,37 @@ __device__ __forceinline__ float level_nsum(const int4* __restrict__ nb8, const 
     return sum;
 }
 
-// One colour of SOR at level LG: u += omega ((sum - h2 b) / (6 + gamma missing) - u). Colour:
-// the global cell parity, which for LG >= 1 is that of the local coordinates (leaf origins are
-// even in cells) and for LG = 0 that of the leaf.
-template <int LG>
-__global__ void __launch_bounds__(kThreads) mgl_smooth_kernel(TopoView t, const int4* __restrict__ nb8, float* u,
-                                                              const float* __restrict__ b, int colour, int zero,
-                                                              float omega, float h2, float gamma,
-                                                              const double* __restrict__ check, double tol2) {
+// One colour of SOR at the coarsest level (one cell per leaf): u += omega ((sum - h2 b) / (6 + gamma
+// missing) - u), the colour being the leaf's parity.
+__global__ void __launch_bounds__(kThreads) coarsest_sweep_kernel(TopoView t, const int4* __restrict__ nb8, float* u,
+                                                                  const float* __restrict__ b, int colour, int zero,
+                                                                  float omega, float h2, float gamma,
+                                                                  const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
     // Programmatic dependent launches: the next kernel of the cycle may be scheduled now; u and
     // b are read after griddepcontrol.wait (a no-op for an ordinary launch).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int num_leaves = (int)t.num_leaves;
-    const int64_t t0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    LevelCell<LG> c;
-    int64_t q;
-    if constexpr (LG == 0) {
-        // One cell per leaf: the leaf's parity decides; from u = 0 the other colour writes 0.
-        if (t0 >= num_leaves) return;
-        q = t0;
-        c = level_cell<0>(q);
-        const int4 o = t.origin[c.leaf];
-        if ((((o.x + o.y + o.z) >> 3) & 1) != colour) {
-            if (zero) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                u[q] = 0.f;
-            }
-            return;
+    const int64_t q = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (q >= num_leaves) return;
+    const int4 o = t.origin[q];
+    if ((((o.x + o.y + o.z) >> 3) & 1) != colour) {
+        if (zero) {  // from u = 0 the other colour writes 0
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            u[q] = 0.f;
         }
-    } else {
-        // One thread per cell of the colour: the z pair (2k, 2k + 1) of row (x, y) holds one.
-        constexpr int m = (1 << LG) - 1, hz = (1 << (LG - 1)) - 1;
-        if (t0 >= ((int64_t)num_leaves << (3 * LG - 1))) return;
-        c.leaf = (int)(t0 >> (3 * LG - 1));
-        c.x = (int)(t0 >> (2 * LG - 1)) & m;
-        c.y = (int)(t0 >> (LG - 1)) & m;
-        const int z0 = 2 * ((int)t0 & hz);
-        c.z = z0 + ((c.x + c.y + colour) & 1);
-        q = ((int64_t)c.leaf << (3 * LG)) + (((c.x << LG) + c.y) << LG) + c.z;
+        return;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     int missing;
-    if (LG == 0 && zero) {
+    if (zero) {
         // u = 0 before this sweep: no neighbour is read.
-        float unused = level_nsum<LG, false>(nb8, u, c.leaf, c.x, c.y, c.z, num_leaves, missing);
+        float unused = level_nsum<0, false>(nb8, u, (int)q, 0, 0, 0, num_leaves, missing);
         (void)unused;
         u[q] = omega * (-h2 * __ldg(b + q)) / (6.0f + gamma * (float)missing);
         return;
     }
-    const float sum = level_nsum<LG>(nb8, u, c.leaf, c.x, c.y, c.z, num_leaves, missing);
+    const float sum = level_nsum<0>(nb8, u, (int)q, 0, 0, 0, num_leaves, missing);
     const float uq = u[q];
     u[q] = uq + omega * ((sum - h2 * __ldg(b + q)) / (6.0f + gamma * (float)missing) - uq);
 }
@@ -269,7 +250,7 @@ __global__ void __launch_bounds__(kThreads) mgl_smooth_kernel(TopoView t, const 
 // the diagonal 6 + gamma missing, the cell's index; colour-0 records from the front of the
 // table, colour-1 records from the back. Neighbours' values are read through the cluster's
 // shared memory window (distributed shared memory), and a cluster barrier separates the
-// colours. The arithmetic is mgl_smooth_kernel<0>'s, in its order: the values are its values.
+// colours. The arithmetic is coarsest_sweep_kernel's, in its order: the values are its values.
 // The cluster has 16 CTAs (a non-portable size) where the device schedules that, else 8.
 constexpr int kCoarseThreads = 1024, kCoarseUnroll = 3;
 constexpr int kCoarseCellBytes = 32 + 4 + 4;  // the record, u, b (plus 4 bytes: u's zero)
@@ -430,8 +411,10 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
 // floats), which updates its 2 cells of the colour from 16-byte loads of the row, its right-hand
 // side and its 4 x/y neighbour rows (across a face, the neighbour leaf's row; a missing leaf adds
 // gamma to the diagonal) and the values past its z ends, and stores the row back whole (no other
-// thread writes it in this sweep). Neighbours are summed in mgl_smooth_kernel's order, so the
-// values are its values: 8 loads for 2 updates where it makes 20.
+// thread writes it in this sweep). Neighbours are summed in the order +x, -x, +y, -y, +z, -z:
+// 7 loads for 2 updates. Selects pick the colour's two cells
+// before the arithmetic: a loop over the four that skips two ran all four for half the lanes each (95.6M
+// voxels 19.5 -> 17.5 us).
 __global__ void __launch_bounds__(kThreads) level1_smooth_rows_kernel(const int4* __restrict__ nb8, float* u,
                                                                       const float* __restrict__ b, int num_leaves,
                                                                       int colour, float omega, float h2,
@@ -449,34 +432,73 @@ __global__ void __launch_bounds__(kThreads) level1_smooth_rows_kernel(const int4
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     auto ld4 = [&](int l, int64_t off) { return l < num_leaves ? __ldg(reinterpret_cast<const float4*>(u + off)) : z4; };
     const int64_t own = row_of(leaf, x, y);
-    const float4 bb = __ldg(reinterpret_cast<const float4*>(b + own));
-    const float4 c4 = __ldg(reinterpret_cast<const float4*>(u + own));
-    const float4 xp = ld4(lxp, row_of(lxp, (x + 1) & 3, y));
-    const float4 xm = ld4(lxm, row_of(lxm, (x - 1) & 3, y));
-    const float4 yp = ld4(lyp, row_of(lyp, x, (y + 1) & 3));
-    const float4 ym = ld4(lym, row_of(lym, x, (y - 1) & 3));
-    const float zhi = f1.x >= num_leaves ? 0.f : __ldg(u + row_of(f1.x, x, y));
-    const float zlo = f1.y >= num_leaves ? 0.f : __ldg(u + row_of(f1.y, x, y) + 3);
+    // The row's cells of the colour are z = p and p + 2: one of them lies at a z end of the leaf.
+    const bool p = ((x + y + colour) & 1) != 0;
+    const int lz = p ? f1.x : f1.y;
+    const float4 bb = __ldg(reinterpret_cast<const float4*>(b + own)), c = __ldg(reinterpret_cast<const float4*>(u + own));
+    const float4 xp = ld4(lxp, row_of(lxp, (x + 1) & 3, y)), xm = ld4(lxm, row_of(lxm, (x - 1) & 3, y));
+    const float4 yp = ld4(lyp, row_of(lyp, x, (y + 1) & 3)), ym = ld4(lym, row_of(lym, x, (y - 1) & 3));
+    const float end = lz < num_leaves ? __ldg(u + row_of(lz, x, y) + (p ? 0 : 3)) : 0.f;
     const int lateral = (lxp >= num_leaves) + (lxm >= num_leaves) + (lyp >= num_leaves) + (lym >= num_leaves);
-    float cv[4] = {c4.x, c4.y, c4.z, c4.w};
-    const float bv[4] = {bb.x, bb.y, bb.z, bb.w};
-    const float xpv[4] = {xp.x, xp.y, xp.z, xp.w}, xmv[4] = {xm.x, xm.y, xm.z, xm.w};
-    const float ypv[4] = {yp.x, yp.y, yp.z, yp.w}, ymv[4] = {ym.x, ym.y, ym.z, ym.w};
-    const float old[4] = {cv[0], cv[1], cv[2], cv[3]};
-#pragma unroll
-    for (int z = 0; z < 4; ++z) {
-        if (((x + y + z) & 1) != colour) continue;  // the other colour keeps its value
-        const int missing = lateral + (z == 3 && f1.x >= num_leaves) + (z == 0 && f1.y >= num_leaves);
-        const float diag = 6.0f + gamma * (float)missing;
-        float sum = xpv[z];
-        sum += xmv[z];
-        sum += ypv[z];
-        sum += ymv[z];
-        sum += z < 3 ? old[z < 3 ? z + 1 : 3] : zhi;
-        sum += z > 0 ? old[z > 0 ? z - 1 : 0] : zlo;
-        cv[z] = old[z] + omega * ((sum - h2 * bv[z]) / diag - old[z]);
-    }
-    *reinterpret_cast<float4*>(u + own) = make_float4(cv[0], cv[1], cv[2], cv[3]);
+    const int ends = lz >= num_leaves;
+    auto relax = [&](float vxp, float vxm, float vyp, float vym, float vzp, float vzm, float vb, float vc, int missing) {
+        float sum = vxp;
+        sum += vxm;
+        sum += vyp;
+        sum += vym;
+        sum += vzp;
+        sum += vzm;
+        return vc + omega * ((sum - h2 * vb) / (6.0f + gamma * (float)missing) - vc);
+    };
+    auto lo = [&](const float4& v) { return p ? v.y : v.x; };
+    auto hi = [&](const float4& v) { return p ? v.w : v.z; };
+    const float mid = p ? c.z : c.y;  // between the two
+    const float r0 = relax(lo(xp), lo(xm), lo(yp), lo(ym), mid, p ? c.x : end, lo(bb), lo(c), lateral + (p ? 0 : ends));
+    const float r1 = relax(hi(xp), hi(xm), hi(yp), hi(ym), p ? end : c.w, mid, hi(bb), hi(c), lateral + (p ? ends : 0));
+    *reinterpret_cast<float4*>(u + own) = p ? make_float4(c.x, r0, c.z, r1) : make_float4(r0, c.y, r1, c.w);
+}
+
+// The same at level 2 (2^3 cells per leaf): one thread per (leaf, x), whose four cells hold two of the
+// colour, (y, z) = (0, p) and (1, 1 - p); 8 loads for the two updates, where a thread per cell of the colour
+// made 16 (95.6M voxels 5.9 -> 4.9 us).
+__global__ void __launch_bounds__(kThreads) level2_smooth_kernel(const int4* __restrict__ nb8, float* u,
+                                                                 const float* __restrict__ b, int num_leaves, int colour,
+                                                                 float omega, float h2, float gamma,
+                                                                 const double* __restrict__ check, double tol2) {
+    if (done(check, tol2)) return;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (tid >= ((int64_t)num_leaves << 1)) return;
+    const int leaf = (int)(tid >> 1), x = (int)tid & 1;
+    const int4 f0 = __ldg(nb8 + 2 * leaf), f1 = __ldg(nb8 + 2 * leaf + 1);
+    const bool p = ((x + colour) & 1) != 0;
+    const int lx = x ? f0.x : f0.y, lza = p ? f1.x : f1.y, lzb = p ? f1.y : f1.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto quad = [&](const float* q, int l, int cx) { return __ldg(reinterpret_cast<const float4*>(q + ((int64_t)l << 3) + 4 * cx)); };
+    auto cell = [&](int l, int y, int z) { return l < num_leaves ? __ldg(u + ((int64_t)l << 3) + 4 * x + 2 * y + z) : 0.f; };
+    // A quad's cells: .x (0, 0), .y (0, 1), .z (1, 0), .w (1, 1).
+    const float4 c = quad(u, leaf, x), in = quad(u, leaf, x ^ 1), bb = quad(b, leaf, x);
+    const float4 out = lx < num_leaves ? quad(u, lx, x ^ 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float ym = cell(f0.w, 1, p ? 1 : 0), yp = cell(f0.z, 0, p ? 0 : 1);
+    const float za = cell(lza, 0, p ? 0 : 1), zb = cell(lzb, 1, p ? 1 : 0);
+    auto relax = [&](float vxp, float vxm, float vyp, float vym, float vzp, float vzm, float vb, float vc, int missing) {
+        float sum = vxp;
+        sum += vxm;
+        sum += vyp;
+        sum += vym;
+        sum += vzp;
+        sum += vzm;
+        return vc + omega * ((sum - h2 * vb) / (6.0f + gamma * (float)missing) - vc);
+    };
+    auto lo = [&](const float4& v) { return p ? v.y : v.x; };  // (0, p)
+    auto hi = [&](const float4& v) { return p ? v.z : v.w; };  // (1, 1 - p)
+    auto plus = [&](float i, float o) { return x ? o : i; };   // across +x: the other half inside, or the next leaf
+    const int mx = lx >= num_leaves;
+    const float ra = relax(plus(lo(in), lo(out)), plus(lo(out), lo(in)), p ? c.w : c.z, ym, p ? za : c.y, p ? c.x : za, lo(bb), lo(c),
+                           mx + (f0.w >= num_leaves) + (lza >= num_leaves));
+    const float rb = relax(plus(hi(in), hi(out)), plus(hi(out), hi(in)), yp, p ? c.x : c.y, p ? c.w : zb, p ? zb : c.z, hi(bb), hi(c),
+                           mx + (f0.z >= num_leaves) + (lzb >= num_leaves));
+    *reinterpret_cast<float4*>(u + ((int64_t)leaf << 3) + 4 * x) = p ? make_float4(c.x, ra, rb, c.w) : make_float4(ra, c.y, c.z, rb);
 }
 
 // bc (level LG - 1) = the mean of the residuals b - (sum - (6 + gamma missing) u) / h2 of each
@@ -506,7 +528,7 @@ __global__ void __launch_bounds__(kThreads) mgl_restrict_kernel(const int4* __re
 
 // The same from level 1 to level 2, one thread per level-2 column (X, Y) (two cells): the 2 x 2 rows of
 // level 1 under it and the 8 beside them as 16-byte loads. Each cell's children are added in the
-// order of mgl_restrict_kernel, each one's neighbours in the order of mgl_smooth_kernel. The first
+// order of mgl_restrict_kernel, each one's neighbours in the sweeps' order. The first
 // red sweep of level 2 from u = 0 is made in passing. 95.6M voxels: 34 -> 19 us.
 __global__ void __launch_bounds__(kThreads, 3) restrict_level1_kernel(const int4* __restrict__ nb8,
                                                                       const float* __restrict__ u,
@@ -985,26 +1007,19 @@ void launch_pdl(const Context& c, void (*kern)(KArgs...), int64_t threads, Args.
 float level_h2(int l) { return (float)(1 << (2 * l)); }
 float level_gamma(int l) { return (float)((1 << l) - 1) / (float)((1 << l) + 1); }
 
-// iters red-black iterations at level l (2^LG cells per leaf side). begun: the first red sweep, from
-// u = 0, is made already (by the restriction); for LG = 0 it is made here, over an u that need not
-// be 0 before.
-template <int LG>
-void smooth_level(Context& c, const int4* nb8, float* u, const float* b, int iters, float omega, int l, bool begun,
-                  const double* check, double tol2) {
-    const float h2 = level_h2(l), gamma = level_gamma(l);
-    int64_t threads = c.topo.num_leaves;  // LG = 0: one thread per leaf
-    if constexpr (LG > 0) threads <<= 3 * LG - 1;  // one thread per cell of the colour
-    for (int it = 0; it < iters; ++it)
-        for (int colour = 0; colour < 2; ++colour) {
-            if (begun && it == 0 && colour == 0) continue;
-            const int zero = (int)(LG == 0 && it == 0 && colour == 0);
-            if constexpr (LG == 2)
-                launch_pdl(c, level1_smooth_rows_kernel, c.topo.num_leaves << 4, nb8, u, b, (int)c.topo.num_leaves,
-                           colour, omega, h2, gamma, check, tol2);
-            else
-                launch_pdl(c, mgl_smooth_kernel<LG>, threads, c.topo.view, nb8, u, b, colour, zero, omega, h2, gamma,
-                           check, tol2);
-        }
+// kMgNu red-black iterations at level l = 1 or 2. begun: the first red sweep, from u = 0, is made
+// already (by the restriction).
+void smooth_level(Context& c, const int4* nb8, float* u, const float* b, int l, bool begun, const double* check,
+                  double tol2) {
+    const int L = (int)c.topo.num_leaves;
+    for (int s = begun ? 1 : 0; s < 2 * kMgNu; ++s) {
+        if (l == 1)
+            launch_pdl(c, level1_smooth_rows_kernel, (int64_t)L << 4, nb8, u, b, L, s & 1, 1.0f, level_h2(l), level_gamma(l),
+                       check, tol2);
+        else
+            launch_pdl(c, level2_smooth_kernel, (int64_t)L << 1, nb8, u, b, L, s & 1, 1.0f, level_h2(l), level_gamma(l), check,
+                       tol2);
+    }
 }
 
 }  // namespace
@@ -1084,7 +1099,8 @@ void coarsest_solve(Context& c, const int4* nb8, float* u, const float* b, int s
         }
     }
     if (c.coarse_solve != HNS_COARSE_CLUSTER || sweeps < 1 || c.coarse_cluster_ok <= 0) {
-        smooth_level<0>(c, nb8, u, b, sweeps, omega, 3, false, check, tol2);
+        for (int s = 0; s < 2 * sweeps; ++s)
+            launch_pdl(c, coarsest_sweep_kernel, L, c.topo.view, nb8, u, b, s & 1, (int)(s == 0), omega, h2, gamma, check, tol2);
         return;
     }
     const int ctas = c.coarse_cluster_ok;
@@ -1123,10 +1139,10 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
     fine(e_zero);
     launch_pdl(c, mg16_restrict_kernel, L << 4, f8, (const __half*)eh, r, b[1], u[1], (int)L, 1.0f,
                level_h2(1), level_gamma(1), check, tol2);
-    smooth_level<2>(c, f8, u[1], b[1], kMgNu, 1.0f, 1, true, check, tol2);
+    smooth_level(c, f8, u[1], b[1], 1, true, check, tol2);
     launch_pdl(c, restrict_level1_kernel, L << 2, f8, (const float*)u[1], (const float*)b[1], b[2], u[2], (int)L, 0.25f,
                level_gamma(1), 1.0f, level_h2(2), level_gamma(2), check, tol2);
-    smooth_level<1>(c, f8, u[2], b[2], kMgNu, 1.0f, 2, true, check, tol2);
+    smooth_level(c, f8, u[2], b[2], 2, true, check, tol2);
     launch_pdl(c, mgl_restrict_kernel<1>, L, f8, (const float*)u[2], (const float*)b[2], b[3], (int)L, 1.0f / 16.0f,
                0.6f, check, tol2);
     int coarse_sweeps;
@@ -1134,9 +1150,9 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
     coarsest_schedule(c, coarse_sweeps, coarse_omega);
     coarsest_solve(c, f8, u[3], b[3], coarse_sweeps, coarse_omega, check, tol2);
     launch_pdl(c, mgl_prolong_kernel<1>, L, t, (const float*)u[3], u[2], check, tol2);
-    smooth_level<1>(c, f8, u[2], b[2], kMgNu, 1.0f, 2, false, check, tol2);
+    smooth_level(c, f8, u[2], b[2], 2, false, check, tol2);
     launch_pdl(c, prolong_level2_kernel, L << 2, t, (const float*)u[2], u[1], check, tol2);
-    smooth_level<2>(c, f8, u[1], b[1], kMgNu, 1.0f, 1, false, check, tol2);
+    smooth_level(c, f8, u[1], b[1], 1, false, check, tol2);
     launch_pdl(c, mg16_prolong_kernel, L << 4, t, (const float*)u[1], eh, check, tol2);
     fine(false);
 }
