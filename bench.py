@@ -63,6 +63,10 @@ KERNELS = {("f32", "per-colour"): "rbgs_split_half_f32_kernel (FP32 solve, colou
                                   "launch per run of half-sweeps between checks)",
            ("f16", "persistent"): "rbgs_split_solve_kernel<__half> (FP16 inner solve, colour-split leaves, persistent: "
                                   "one launch per inner solve)"}
+# The library's default: one launch per colour, or the solve held in shared memory (rbgs_chip_kernel)
+# where the grid fits (box64).
+for _p in ("f32", "f16"):
+    KERNELS[(_p, "auto")] = KERNELS[(_p, "per-colour")]
 
 # The fire step (HNS_Advance with the configurations' forces): the sparse plume runs it in FP32
 # with a fixed 100 red-black iterations per step, the large sparse fire on BF16/FP16 storage with
@@ -101,8 +105,8 @@ def measured_peak_gbs():
 
 def apply_options(g, hl, args):
     """The library options the command line selects."""
-    form = getattr(args, "split_solve", "per-colour")
-    g.set_option(hl.OPT_SPLIT_SOLVE, hl.SPLIT_PERSISTENT if form == "persistent" else hl.SPLIT_PER_COLOUR)
+    form = getattr(args, "split_solve", "auto")
+    g.set_option(hl.OPT_SPLIT_SOLVE, {"persistent": hl.SPLIT_PERSISTENT, "per-colour": hl.SPLIT_PER_COLOUR}.get(form, hl.SPLIT_AUTO))
     coarse = getattr(args, "coarse_solve", "cluster")
     g.set_option(hl.OPT_COARSE_SOLVE, hl.COARSE_CLUSTER if coarse == "cluster" else hl.COARSE_LAUNCHES)
     g.set_option(hl.OPT_L2_PERSIST, 0 if getattr(args, "no_l2_persist", False) else 1)
@@ -1242,7 +1246,7 @@ def box64_ours(args):
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": z["ms_per_step"], "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
                 "config": box64_config(args), "details": {"walls": forms},
-                "roofline": {"kernel": "rbgs_iteration_kernel<true> (zero-gradient walls)", "bound": "hbm",
+                "roofline": {"kernel": "rbgs_chip_kernel (zero-gradient walls, the solve held in shared memory)", "bound": "hbm",
                              "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": None, "launch_ms": it_ms,
                              "note": "262,144 voxels sit in L2: launch-bound, the fraction is not an HBM bound"},
@@ -1276,8 +1280,9 @@ def main():
                     help="inner solve of the mixed-precision refinement: V-cycles with red-black smoothing "
                          "(HNS_SOLVE_MULTIGRID, default) or red-black SOR iterations")
     ap.add_argument("--cycles", type=int, default=2, help="V-cycles per outer refinement step (--inner multigrid)")
-    ap.add_argument("--split-solve", choices=["persistent", "per-colour"], default="per-colour",
-                    help="launch form of the colour-split red-black solves (same results to the bit)")
+    ap.add_argument("--split-solve", choices=["auto", "persistent", "per-colour"], default="auto",
+                    help="launch form of the colour-split red-black solves (same results to the bit); auto: the "
+                         "library's choice by size")
     ap.add_argument("--coarse-solve", choices=["cluster", "launches"], default="cluster",
                     help="the multigrid cycle's coarsest level: one thread-block cluster launch or two "
                          "launches per SOR sweep (same results to the bit)")
@@ -1289,6 +1294,14 @@ def main():
     args = ap.parse_args()
     if args.warmup < 3:
         ap.error("--warmup must be at least 3")
+    from oracle import binding
+
+    if not os.path.exists(binding.REF_SO):  # built from the reference's sources (oracle/Makefile)
+        if args.impl == "reference":
+            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libhns_ref.so is not built: no reference sources"}),
+                  flush=True)
+            return
+        args.no_cpu_baseline = True
     if args.workload == "box64":
         (box64_reference if args.impl == "reference" else box64_ours)(args)
         return

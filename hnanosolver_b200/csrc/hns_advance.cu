@@ -4,17 +4,17 @@
 //
 // Per substep the reference runs about 2*iterations + 15 launches, with cudaMalloc'd
 // temporaries, memsets and device-to-device copies. Here:
-//   advect_fused          velocity -> adv                       (advect_vector)
-//   confine_sources       adv -> adv2, + sources, gravity       (vorticityConfinement out of
-//                                                                place, add_velocity_source(_xyz),
+//   advect_tile           velocity -> adv                       (advect_vector)
+//   curl_rows +           adv -> adv2, + sources, gravity       (vorticityConfinement out of
+//   confine_rows                                                 place, add_velocity_source(_xyz),
 //                                                                add_scalar_source, add_gravity)
 //   div_combust_buoy      adv2 -> div, fields, adv3             (divergence, combustion_oxygen or
 //                                                                the force model's burn,
 //                                                                temperature_buoyancy [+ density])
 //   rbgs x iterations     div -> p                              (redBlackGaussSeidelUpdate)
 //   [divergence, rbgs x max(2, iterations/2)]  when disturbanceEnable > 0
-//   subtract_gradient     adv3, p -> velocity
-//   advect_scalars        the persistent scalars, with the projected velocity
+//   gradient_rows         adv3, p -> velocity
+//   advect_scalars_tile   the persistent scalars, with the projected velocity
 // With a "collision_sdf" field the collider enters as in the reference: enforced on the
 // velocity before the substeps and after each projection, trace points inside it pulled back
 // in both advections, and the near-wall blend after the velocity advection and the gradient.

@@ -1,23 +1,26 @@
 // Solver kernels for sm_100a: advection, divergence, red-black SOR, gradient subtraction,
 // vorticity confinement, FP64 residual norms.
 //
-// Work decomposition: every kernel is leaf-tiled. Stencil and advection kernels run two
-// 256-thread CTAs per 8^3 leaf, one thread per voxel, with the leaf's 27-leaf neighbourhood
-// staged in shared memory so that neighbour taps resolve without a tree walk (the
+// Work decomposition: every kernel is leaf-tiled. The advections take a leaf and a one-voxel halo
+// into shared memory, one CTA per 8^3 leaf (hns_advect_tile.cuh, hns_scalars_tile.cuh); divergence and
+// gradient take half a z-row a thread with vector loads (hns_rows.cuh); the forms with a collider and
+// the confinement run two 256-thread CTAs per leaf, one thread per voxel, with the leaf's 27-leaf
+// neighbourhood staged in shared memory so that neighbour taps resolve without a tree walk (the
 // reference walks a NanoVDB ReadAccessor per tap, src/Utils/Stencils.hpp:59-61). The
-// red-black solver runs one CTA per leaf and fuses both colours of an iteration: it stages
+// red-black iteration here runs one CTA per leaf and fuses both colours: it stages
 // the leaf with a two-voxel pressure halo and a one-voxel divergence halo, relaxes the red
 // voxels of the leaf and of its one-voxel face ring, then the black voxels of the leaf, so
-// that one pass reads p and div once and writes p once (ping-pong buffers).
+// that one pass reads p and div once and writes p once (ping-pong buffers); whole solves take the
+// colour-split forms (hns_rbgs_split.cu, hns_rbgs_chip.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <type_traits>
 
 #include "hns_advect_tile.cuh"
-#include "hns_scalars_tile.cuh"
 #include "hns_internal.cuh"
 #include "hns_rows.cuh"
+#include "hns_scalars_tile.cuh"
 #include "hns_stencil.cuh"
 
 namespace hns {
