@@ -469,6 +469,11 @@ __global__ void __launch_bounds__(kThreads) adj_confine_force_kernel(TopoView t,
         const int a = n >> 6, b = (n >> 3) & 7, d = n & 7, c = dev::conf_wi(a, b, d);
         const int64_t s = (leaf << 9) + n;
         const float3 ob = dev::ld3(out_bar, s);
+        if (ob.x == 0.f && ob.y == 0.f && ob.z == 0.f) {  // no adjoint, whatever the velocity (0 times infinity is not 0)
+            dev::st3(wb_out, s, make_float3(0.f, 0.f, 0.f));
+            dev::st3(gb_out, s, make_float3(0.f, 0.f, 0.f));
+            continue;
+        }
         const float3 w = make_float3(T.w[0][c], T.w[1][c], T.w[2][c]);
         const float3 g = make_float3((T.m[dev::conf_wi(a + fs, b, d)] - T.m[dev::conf_wi(a - fs, b, d)]) * f,
                                      (T.m[dev::conf_wi(a, b + fs, d)] - T.m[dev::conf_wi(a, b - fs, d)]) * f,
@@ -497,9 +502,9 @@ __device__ __forceinline__ float3 magnitude_part(const float* __restrict__ vel, 
     const float3 w = make_float3(((v[3].z - v[2].z) - (v[5].y - v[4].y)) * f, ((v[5].x - v[4].x) - (v[1].z - v[0].z)) * f,
                                  ((v[1].y - v[0].y) - (v[3].x - v[2].x)) * f);
     const float m = sqrtf(dot3(w, w));
-    if (m <= 0.f) return make_float3(0.f, 0.f, 0.f);
     auto at = [&](int64_t q, int c) { return q < 0 ? 0.f : __ldg(gb + 3 * q + c); };
     const float sum = (at(ns[0], 0) - at(ns[1], 0)) + (at(ns[2], 1) - at(ns[3], 1)) + (at(ns[4], 2) - at(ns[5], 2));
+    if (m <= 0.f || sum == 0.f) return make_float3(0.f, 0.f, 0.f);  // no neighbour has an adjoint: 0 for any omega
     const float r = (fs > 0 ? sum : -sum) * f / m;
     return make_float3(r * w.x, r * w.y, r * w.z);
 }

@@ -1,0 +1,53 @@
+"""Infinities and NaN that no adjoint reaches. Where the adjoint of an output is 0, the values that
+output was computed from do not enter the gradient, finite or not (a loss over part of a domain whose
+rest has blown up): the gradient is that of the same fields with the non-finite values replaced by 0."""
+import numpy as np
+import pytest
+
+from hnanosolver_b200 import synth
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch.device("cuda", 0)
+
+
+BAD = [float("nan"), float("inf"), -float("inf")]
+
+
+def _grid(dev):
+    """A grid, the slots of a few of its voxels and the mask of the voxels within 4 of one."""
+    from hnanosolver_b200 import lib as hl
+
+    o = synth.spheres_topology(64, 3, 6.0, 14.0, seed=9)
+    ijk = torch.from_numpy(synth.leaf_dense_coords(o)).to(dev)
+    slots = torch.from_numpy(np.random.default_rng(2).choice(len(ijk), 6, replace=False)).to(dev)
+    near = torch.zeros(len(ijk), dtype=torch.bool, device=dev)
+    for s in slots:
+        near |= (ijk - ijk[s]).abs().amax(dim=1) <= 4
+    return hl.Grid(o, voxel_size=0.1), slots, near
+
+
+@pytest.mark.parametrize("factor", [1.0, -1.0])
+@pytest.mark.parametrize("bad", BAD)
+def test_confinement(dev, bad, factor):
+    grid, slots, near = _grid(dev)
+    gen = torch.Generator(device=dev).manual_seed(4)
+    vel = torch.randn((grid.num_voxels, 3), device=dev, generator=gen)
+    out_bar = torch.randn(vel.shape, device=dev, generator=gen)
+    out_bar[near] = 0.0
+    got = []
+    for value in (bad, 0.0):
+        vel[slots, 1] = value
+        bar = torch.zeros_like(vel)
+        torch.cuda.synchronize()
+        grid.adjoint_vorticity_confinement(vel, out_bar, bar, 0.1, 0.4, factor)
+        grid.synchronize()
+        got.append(bar)
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
+    grid.close()
