@@ -673,7 +673,15 @@ float* adj_scratch(Context& c) { return c.scratch_f32("adjoint_work", 8 * (size_
 // to the initial p is not needed (p starts at 0), so lam is never rescaled at the end.
 void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, float omega, float* lam) {
     if (iterations <= 0) return;
-    if (use_chip(c, 2 * iterations) && aligned16(p_bar) && aligned16(div_bar) && chip_fits(c, sizeof(float), true)) {
+    if (!aligned16(div_bar)) {  // both forms move its rows as 16-byte vectors
+        const size_t bytes = (size_t)c.num_voxels() * sizeof(float);
+        float* d = c.scratch_f32("adjoint_div_aligned", (size_t)c.num_voxels());
+        HNS_CUDA(cudaMemcpyAsync(d, div_bar, bytes, cudaMemcpyDeviceToDevice, c.stream));
+        adj_rbgs(c, p_bar, d, iterations, omega, lam);
+        HNS_CUDA(cudaMemcpyAsync(div_bar, d, bytes, cudaMemcpyDeviceToDevice, c.stream));
+        return;
+    }
+    if (use_chip(c, 2 * iterations) && aligned16(p_bar) && chip_fits(c, sizeof(float), true)) {
         launch_chip_transpose(c, c.split_faces(), p_bar, div_bar, iterations, omega);
         return;
     }

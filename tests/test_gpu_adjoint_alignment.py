@@ -1,0 +1,39 @@
+"""The transposed red-black sweeps on arrays that are only 4-byte aligned (views into a program's
+larger buffer), by both launch forms: the values of aligned arrays, to the bit."""
+import pytest
+
+from hnanosolver_b200 import synth
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return torch.device("cuda", 0)
+
+
+@pytest.mark.parametrize("form", ["AUTO", "PER_COLOUR"])
+@pytest.mark.parametrize("shift", [(0, 1), (1, 0), (2, 3)])
+def test_adjoint_rbgs_of_unaligned_arrays(dev, shift, form):
+    from hnanosolver_b200 import lib as hl
+
+    grid = hl.Grid(synth.spheres_topology(64, 3, 6.0, 14.0, seed=9), voxel_size=0.1)
+    grid.set_option(hl.OPT_SPLIT_SOLVE, getattr(hl, "SPLIT_" + form))
+    n = grid.num_voxels
+    gen = torch.Generator(device=dev).manual_seed(5)
+    p_bar, d0 = (torch.randn(n, device=dev, generator=gen) for _ in range(2))
+    got = []
+    for s in ((0, 0), shift):
+        store = [torch.full((n + 8,), 7.0, device=dev) for _ in range(2)]
+        p, d = (x[k:k + n] for x, k in zip(store, s))
+        p.copy_(p_bar), d.copy_(d0)
+        torch.cuda.synchronize()
+        grid.adjoint_rbgs(p, d, 7, 1.4)
+        grid.device_status()
+        assert (store[1][:s[1]] == 7.0).all() and (store[1][s[1] + n:] == 7.0).all()
+        got.append(d.clone())
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
+    grid.close()
