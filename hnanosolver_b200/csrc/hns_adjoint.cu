@@ -681,7 +681,7 @@ void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, fl
         HNS_CUDA(cudaMemcpyAsync(div_bar, d, bytes, cudaMemcpyDeviceToDevice, c.stream));
         return;
     }
-    if (use_chip(c, 2 * iterations) && aligned16(p_bar) && chip_fits(c, sizeof(float), true)) {
+    if (use_chip(c, 2 * iterations) && aligned16(p_bar) && chip_takes(c, ChipUse::kTransposed)) {
         launch_chip_transpose(c, c.split_faces(), p_bar, div_bar, iterations, omega);
         return;
     }

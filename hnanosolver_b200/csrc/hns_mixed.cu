@@ -717,7 +717,8 @@ RefinePlan refine_solve(Context& c, const float* div, double* p, int max_outer, 
         // forecast takes it whatever the option: it most likely returns at once, and one launch
         // then costs a few microseconds where 2 * inner returning half-sweeps cost 2.3 us each.
         // Where the values fit the SMs' shared memory, the solve held there (hns_rbgs_chip.cu).
-        const bool chip = layout == HNS_INNER_SPLIT && use_chip(c, 2 * plan.inner) && chip_fits(c, sizeof(TI));
+        const bool chip = layout == HNS_INNER_SPLIT && use_chip(c, 2 * plan.inner) &&
+                          chip_takes(c, sizeof(TI) == 2 ? ChipUse::kHalf : ChipUse::kPlain);
         const bool persistent = layout == HNS_INNER_SPLIT && (c.split_solve == HNS_SPLIT_PERSISTENT || spare || chip);
         if (chip) {
             if constexpr (sizeof(TI) == 2)

@@ -4,17 +4,17 @@
 //
 // Why. A half-sweep of a grid of a few million voxels is bound by its launch, by L2 latency and by
 // the drain between the colours, not by bytes. The 148 SMs hold 33 MB of shared memory between
-// them, where the values and the right-hand side of a few million voxels fit with a halo.
+// them, where the values and the right-hand side of up to 3.5 million voxels fit with a halo.
 //
-// Measured, us per half-sweep of a box of leaves, one launch per colour -> here:
-//   leaves           59          512         1,493        3,300        5,300        6,594
-//   FP32         3.0 -> 1.1  2.1 -> 1.2   2.3 -> 1.7   2.7 -> 2.8   3.7 -> 3.8      4.3
-//   walls        3.0 -> 1.2  2.1 -> 1.3   2.8 -> 1.9   3.0 -> 3.0   4.2 -> 4.1      4.8
-//   transpose    4.1 -> 1.1  4.5 -> 1.2   6.2 -> 1.8    10 -> 3.0    14 -> 4.0   16 -> 5.0
-//   FP16         1.8 -> 1.1  2.1 -> 1.2   2.3 -> 1.7      2.7          3.0          3.5
-// From 3,300 leaves on the gain is the host's: one launch in place of hundreds. What is left is the
-// shared-memory pipe and instruction issue, and for small grids the exchange's L2 round trip (1.1 us
-// with nothing else to do).
+// Measured, us per half-sweep, one launch per colour -> here; alone / three contexts taking turns on
+// streams of their own (per solve of one of them):
+//   leaves                 59                    592                   1,776                  2,368
+//   FP32       2.1 -> 1.1 / 2.1 -> 0.4  2.0 -> 1.2 / 2.1 -> 0.7  2.1 -> 2.0 / 1.8 -> 1.3  2.7 -> 2.5 / 1.8 -> 1.6
+//   walls      2.1 -> 1.2 / 2.1 -> 0.4  2.1 -> 1.4 / 2.1 -> 0.8  2.3 -> 2.2 / 1.8 -> 1.5  3.0 -> 2.8 / 1.8 -> 1.8
+//   transpose                           4.7 -> 1.3 / 2.9 -> 0.8  7.2 -> 2.1 / 3.8 -> 1.4  8.3 -> 2.7 / 4.5 -> 1.8
+// and the transpose of 4,096 leaves 12.1 -> 3.4 / 7.3 -> 3.3, of 6,512 16.5 -> 4.8 / 11.4 -> 4.8. What is left
+// is the shared-memory pipe and instruction issue, and for small grids the exchange's L2 round trip
+// (1.1 us with nothing else to do).
 //
 // Partition. CTA k owns the P leaves from k P (the caller's leaf order, which is spatially compact
 // for NanoVDB-ordered grids; any order is correct). Leaves are stored colour-split, as in
@@ -53,6 +53,19 @@ constexpr uint32_t kChipMaxPolls = 1u << 20;
 constexpr size_t kChipSmSmem = 233472;   // an SM's shared memory, 228 KB
 constexpr size_t kChipMaxSmem = 232448;  // 227 KB, the most one CTA can have
 constexpr size_t kChipReserve = 1536;    // of each CTA: 1 KB of the system's, its static shared memory
+
+// The largest grids, in leaves per SM, whose solves are held here (chip_takes). A solve holds every SM
+// from its first half-sweep to its last, so beyond some size launches per colour, between which other
+// streams' kernels run, finish more solves. Launches per colour -> here, us, alone / three contexts in turn:
+//   FP32, 100 iterations    2,368 leaves 558 -> 505 / 372 -> 327    2,369 (256 threads) 566 -> 498 / 361 -> 504
+//                           4,096 673 -> 626 / 398 -> 624           6,512 848 -> 896 / 622 -> 895
+//   checked every 10, 100   592 leaves 406 -> 384 / 207 -> 198      750 465 -> 474 / 225 -> 212
+//     (loaded and stored    900 479 -> 506 / 234 -> 241             1,776 551 -> 591 / 292 -> 361
+//     at every check)
+//   FP16, a step of 90      1,184 leaves 504 -> 446 / 375 -> 257    1,776 499 -> 504 / 377 -> 317
+//                           1,777 513 -> 587 / 369 -> 317           2,368 592 -> 630 / 380 -> 392
+// The transpose, whose form launched per colour is far slower, takes every size that fits.
+constexpr int kChipLeavesPerSm = 16, kChipLeavesPerSmChecked = 5, kChipLeavesPerSmHalf = 12;
 
 enum ChipMode { kDirichlet = 0, kWalls = 1, kTranspose = 2 };
 
@@ -421,39 +434,36 @@ size_t chip_smem(int64_t per_cta) {
 }
 
 // How a launch divides the grid: four CTAs an SM, so that one CTA's exchange overlaps the others'
-// updates, where their shared memory fits; else one of 1,024 threads. us per half-sweep (FP32, open
-// walls) with one CTA an SM -> four of 256 threads:
-//   leaves  512: 1.61 -> 1.23   1,493: 2.26 -> 1.71   3,300: 3.46 -> 2.84   5,300: 3.92 -> 3.83
-// Up to four leaves a CTA 128 threads: 256 fill the SM's registers, so that solves of other streams
-// wait. HNS_Advance on 1,493 leaves, us alone / with three contexts taking turns: 788 / 626 with
-// 256 threads, 835 / 513 with 128.
-// FP16 conversions make its update issue-bound: beyond kChipMaxHalfLeaves leaves a CTA full grids
-// launched per colour issue it as fast (2,400 leaves 2.4 us either way, 4,096 2.7 against 2.9 here).
-constexpr int64_t kChipMaxHalfLeaves = 4;
+// updates, of 128 threads up to four leaves a CTA (256 fill the SM's registers, so that other streams
+// wait: HNS_Advance on 1,493 leaves, us alone / three contexts in turn: 788 / 626 with 256 threads, 835 /
+// 513 with 128). The transpose also of 256 beyond, and one CTA of 1,024 threads an SM for the last 5 %
+// of the sizes that fit.
 struct ChipShape {
     int64_t per_cta;  // 0: the grid does not fit
     int threads;
 };
 template <typename T>
-ChipShape chip_shape(const Context& c) {
+ChipShape chip_shape(const Context& c, bool transpose) {
     const int64_t L = c.topo.num_leaves, sms = c.sm_count();
     if (L <= 0) return {0, 0};
     const int64_t quarter = (L + 4 * sms - 1) / (4 * sms), whole = (L + sms - 1) / sms;
-    if (sizeof(T) == 2 && quarter > kChipMaxHalfLeaves) return {0, 0};
-    if (chip_smem<T>(quarter) <= kChipSmSmem / 4 - kChipReserve) return {quarter, quarter <= 4 ? 128 : 256};
-    if (chip_smem<T>(whole) <= kChipMaxSmem - kChipReserve) return {whole, 1024};
+    if (4 * quarter <= kChipLeavesPerSm) return {quarter, 128};
+    if (transpose && chip_smem<T>(quarter) <= kChipSmSmem / 4 - kChipReserve) return {quarter, 256};
+    if (transpose && chip_smem<T>(whole) <= kChipMaxSmem - kChipReserve) return {whole, 1024};
     return {0, 0};
 }
 
 template <typename T, ChipMode kMode>
 void launch_chip(Context& c, ChipArgs<T> A) {
     const int64_t L = c.topo.num_leaves;
-    const ChipShape shape = chip_shape<T>(c);
+    const ChipShape shape = chip_shape<T>(c, kMode == kTranspose);
     A.num_leaves = (int)L;
     A.per_cta = (int)shape.per_cta;
-    auto kern = shape.threads == 1024  ? rbgs_chip_kernel<T, kMode, 1024>
-                : shape.threads == 256 ? rbgs_chip_kernel<T, kMode, 256>
-                                       : rbgs_chip_kernel<T, kMode, 128>;
+    auto kern = rbgs_chip_kernel<T, kMode, 128>;
+    if constexpr (kMode == kTranspose) {
+        if (shape.threads == 256) kern = rbgs_chip_kernel<T, kMode, 256>;
+        if (shape.threads == 1024) kern = rbgs_chip_kernel<T, kMode, 1024>;
+    }
     const unsigned blocks = (unsigned)((L + A.per_cta - 1) / A.per_cta);
     // The same limit for every context of the process, so none lowers another's.
     HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kChipMaxSmem - kChipReserve)));
@@ -493,11 +503,12 @@ void launch_chip(Context& c, ChipArgs<T> A) {
 
 }  // namespace
 
-bool chip_fits(const Context& c, size_t bytes, bool transpose) {
-    const ChipShape s = bytes == 2 ? chip_shape<__half>(c) : chip_shape<float>(c);
-    // One CTA an SM is no faster than full grids launched per colour, but for the transpose, which
-    // has no such form on colour-split leaves.
-    return s.per_cta > 0 && (transpose || s.threads < 1024);
+bool chip_takes(const Context& c, ChipUse use) {
+    if (use == ChipUse::kTransposed) return chip_shape<float>(c, true).per_cta > 0;
+    const int per_sm = use == ChipUse::kChecked ? kChipLeavesPerSmChecked
+                       : use == ChipUse::kHalf  ? kChipLeavesPerSmHalf
+                                                : kChipLeavesPerSm;
+    return c.topo.num_leaves > 0 && c.topo.num_leaves <= (int64_t)per_sm * c.sm_count();
 }
 
 void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,

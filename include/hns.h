@@ -501,11 +501,13 @@ HNS_API hns_status hns_adjoint_advance_mixed(hns_ctx* ctx, const hns_fire_fields
 #define HNS_SPLIT_PERSISTENT 1  /*   one cooperative launch per inner solve, or per run of iterations
                                      between convergence checks, leaf groups ordered by per-group
                                      progress counters instead of launch boundaries. */
-#define HNS_SPLIT_AUTO 2        /*   default: where the grid's values fit the SMs' shared memory (FP32 up
-                                     to about 3.3M voxels; FP16 up to 1.2M), one cooperative launch per
-                                     solve that keeps them there from the first half-sweep to the last,
-                                     else one launch per half-sweep. All three give the same results to
-                                     the bit. */
+#define HNS_SPLIT_AUTO 2        /*   default: on smaller grids (on 148 SMs, FP32 solves of a fixed iteration
+                                     count up to 1.2M voxels, checked ones up to 0.38M, FP16 inner solves
+                                     up to 0.9M; the adjoint's transposed sweeps up to 3.5M) one
+                                     cooperative launch per solve, or per run of iterations between
+                                     checks, that keeps the values in the SMs' shared memory from the
+                                     first half-sweep to the last; else one launch per half-sweep. All
+                                     three give the same results to the bit. */
 #define HNS_OPT_COARSE_SOLVE 5  /* how the FP16 multigrid cycle (HNS_SOLVE_MULTIGRID) solves its coarsest
                                      level, one cell per leaf: */
 #define HNS_COARSE_LAUNCHES 0   /*   two launches per SOR sweep */
