@@ -32,7 +32,8 @@
 // thread that writes a face value of half-sweep h has read, for the same update, the neighbour's
 // value of half-sweep h - 1 across that face, and that value was stored after the neighbour had
 // read the word of half-sweep h - 2. Waits are bounded (kChipMaxPolls polls): one that gives up
-// raises the device error flag and the abort word, and every CTA returns with the solve unfinished.
+// raises the device error flag and the abort word, and every CTA that waits returns, its leaves not
+// stored; one that has no neighbour in another CTA runs to the end and stores its own.
 //
 // The arithmetic of each update is that of the launch-per-colour kernels in the same order, so
 // the values are the same to the bit.
@@ -131,7 +132,8 @@ struct ChipArgs {
     int mid_half;
     double tol2;
     unsigned long long* counters;
-    uint32_t max_polls;  // 0: every wait gives up at once
+    uint32_t max_polls;  // after which a wait gives up
+    bool stall;          // the test hook of the timeout path: no tag is accepted
 };
 
 // Row (a, b) of `leaf`: its values of colour 0 and 1. Slot order holds z = 0 .. 7 in a row; entry j
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
             uint32_t polls = 0;
             for (;;) {
                 get2(src, x, y);
-                if ((uint32_t)(x >> 32) == tag && (uint32_t)(y >> 32) == tag && A.max_polls != 0) break;
+                if (!A.stall && (uint32_t)(x >> 32) == tag && (uint32_t)(y >> 32) == tag) break;
                 if (++polls >= A.max_polls) {
                     atomicExch(A.abort_word, A.tag0);
                     if (A.counters != nullptr) atomicExch(A.counters + 1, 1ull);
@@ -483,8 +485,8 @@ void launch_chip(Context& c, ChipArgs<T> A) {
     }
     A.tag0 = c.chip_tag;
     c.chip_tag += (uint32_t)A.half_sweeps + 1u;
-    const bool stall = c.first_wait_polls >= 0;  // the test hook of the timeout path: no tag is accepted
-    A.max_polls = stall ? 0u : kChipMaxPolls;
+    A.stall = c.first_wait_polls >= 0;
+    A.max_polls = A.stall ? std::min((uint32_t)c.first_wait_polls, kChipMaxPolls) : kChipMaxPolls;
     A.counters = c.counters;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);

@@ -712,7 +712,7 @@ void launch_split_solve(Context& c, const int* nb8, const T* rhs, T* e, int half
     const unsigned blocks = (unsigned)std::min<int64_t>(groups, (int64_t)per_sm * c.sm_count());
     // The test hook: every wait gives up after first_wait_polls polls, its target out of reach.
     const bool stall = c.first_wait_polls >= 0;
-    const uint32_t max_polls = stall ? (uint32_t)c.first_wait_polls : kSolveMaxPolls;
+    const uint32_t max_polls = stall ? std::min((uint32_t)c.first_wait_polls, kSolveMaxPolls) : kSolveMaxPolls;
     const uint32_t unreachable = stall ? (1u << 30) : 0u;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);

@@ -494,13 +494,18 @@ HNS_API hns_status hns_adjoint_advance_mixed(hns_ctx* ctx, const hns_fire_fields
                                     error flag (hns_device_status) and return, leaving p_out
                                     unfinished. The persistent colour-split solves (HNS_SPLIT_PERSISTENT):
                                     every dependency wait behaves as if the neighbour never finished and
-                                    gives up after `value` polls, raising the flag; every CTA then
-                                    returns, leaving the solve unfinished. */
+                                    gives up after `value` polls (at most 2^20), raising the flag; every
+                                    CTA then returns, leaving the solve unfinished. The solves in shared
+                                    memory (HNS_SPLIT_AUTO, the default form, on grids that take it): the
+                                    same; leaves whose CTA has no neighbour in another may have been
+                                    stored. A context with this option set should run only
+                                    the solve under test. */
 #define HNS_OPT_SPLIT_SOLVE 4   /* how the colour-split solves (HNS_RBGS_SPLIT, HNS_INNER_SPLIT) launch: */
 #define HNS_SPLIT_PER_COLOUR 0  /*   one launch per half-sweep (programmatic dependent launches) */
 #define HNS_SPLIT_PERSISTENT 1  /*   one cooperative launch per inner solve, or per run of iterations
                                      between convergence checks, leaf groups ordered by per-group
-                                     progress counters instead of launch boundaries. */
+                                     progress counters instead of launch boundaries. Solves with
+                                     zero-gradient walls have no such form: they launch per half-sweep. */
 #define HNS_SPLIT_AUTO 2        /*   default: on smaller grids (on 148 SMs, FP32 solves of a fixed iteration
                                      count up to 1.2M voxels, checked ones up to 0.38M, FP16 inner solves
                                      up to 0.9M; the adjoint's transposed sweeps up to 3.5M) one
