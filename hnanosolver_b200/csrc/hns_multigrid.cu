@@ -186,8 +186,8 @@ __device__ __forceinline__ LevelCell<LG> level_cell(int64_t q) {
 // Sum of the face neighbours of cell (x, y, z) of `leaf` at level LG present in the domain, and
 // the number missing.
 template <int LG, bool kRead = true>
-__device__ __forceinline__ float level_nsum(const int4* __restrict__ nb8, const float* __restrict__ u, int leaf, int x,
-                                            int y, int z, int num_leaves, int& missing) {
+__device__ __forceinline__ float level_nsum(const int4* __restrict__ nb8, const float* u, int leaf, int x, int y,
+                                            int z, int num_leaves, int& missing) {
     constexpr int s = 1 << LG, m = s - 1;
     const int4 f0 = __ldg(nb8 + 2 * leaf), f1 = __ldg(nb8 + 2 * leaf + 1);
     auto at = [&](int l, int a, int b, int c) -> float {
@@ -207,10 +207,16 @@ __device__ __forceinline__ float level_nsum(const int4* __restrict__ nb8, const 
     return sum;
 }
 
+// The kernels of the FP16 cycle start while the preceding ones still run (programmatic dependent
+// launches) and wait before they read what those write. Such arrays are read by plain loads, through
+// pointers without __restrict__: a non-coherent load (__ldg, or one that the compiler makes of a const
+// __restrict__ pointer) is only allowed on memory that nothing writes while the kernel lives, and may
+// be moved above the wait.
+
 // One colour of SOR at the coarsest level (one cell per leaf): u += omega ((sum - h2 b) / (6 + gamma
 // missing) - u), the colour being the leaf's parity.
 __global__ void __launch_bounds__(kThreads) coarsest_sweep_kernel(TopoView t, const int4* __restrict__ nb8, float* u,
-                                                                  const float* __restrict__ b, int colour, int zero,
+                                                                  const float* b, int colour, int zero,
                                                                   float omega, float h2, float gamma,
                                                                   const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
@@ -234,12 +240,12 @@ __global__ void __launch_bounds__(kThreads) coarsest_sweep_kernel(TopoView t, co
         // u = 0 before this sweep: no neighbour is read.
         float unused = level_nsum<0, false>(nb8, u, (int)q, 0, 0, 0, num_leaves, missing);
         (void)unused;
-        u[q] = omega * (-h2 * __ldg(b + q)) / (6.0f + gamma * (float)missing);
+        u[q] = omega * (-h2 * b[q]) / (6.0f + gamma * (float)missing);
         return;
     }
     const float sum = level_nsum<0>(nb8, u, (int)q, 0, 0, 0, num_leaves, missing);
     const float uq = u[q];
-    u[q] = uq + omega * ((sum - h2 * __ldg(b + q)) / (6.0f + gamma * (float)missing) - uq);
+    u[q] = uq + omega * ((sum - h2 * b[q]) / (6.0f + gamma * (float)missing) - uq);
 }
 
 // All SOR sweeps of the coarsest level (one cell per leaf) in one launch of a thread-block
@@ -322,7 +328,7 @@ __global__ void __launch_bounds__(kCoarseThreads) coarse_table_kernel(TopoView t
 
 __global__ void __launch_bounds__(kCoarseThreads, 1)
     coarsest_cluster_kernel(const uint4* __restrict__ table, const int* __restrict__ counts, float* __restrict__ u_out,
-                            const float* __restrict__ b, int num_leaves, int per_cta, int sweeps, float omega, float h2,
+                            const float* b, int num_leaves, int per_cta, int sweeps, float omega, float h2,
                             const double* __restrict__ check, double tol2) {
     extern __shared__ __align__(16) unsigned char coarse_smem[];
     __shared__ float s_skip;
@@ -343,7 +349,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (rank == 0 && tid == 0 && done(check, tol2)) s_skip = 1.f;
-    for (int i = tid; i < n; i += kCoarseThreads) sb[i] = __ldg(b + lo + i);
+    for (int i = tid; i < n; i += kCoarseThreads) sb[i] = b[lo + i];
     cluster_barrier();
     // Every CTA takes rank 0's decision, so all or none reach the sweeps' barriers; rank 0's
     // memory stays until each has read it.
@@ -416,7 +422,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
 // before the arithmetic: a loop over the four that skips two ran all four for half the lanes each (95.6M
 // voxels 19.5 -> 17.5 us).
 __global__ void __launch_bounds__(kThreads) level1_smooth_rows_kernel(const int4* __restrict__ nb8, float* u,
-                                                                      const float* __restrict__ b, int num_leaves,
+                                                                      const float* b, int num_leaves,
                                                                       int colour, float omega, float h2,
                                                                       float gamma, const double* __restrict__ check,
                                                                       double tol2) {
@@ -430,15 +436,15 @@ __global__ void __launch_bounds__(kThreads) level1_smooth_rows_kernel(const int4
     const int lxp = x < 3 ? leaf : f0.x, lxm = x > 0 ? leaf : f0.y, lyp = y < 3 ? leaf : f0.z, lym = y > 0 ? leaf : f0.w;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto ld4 = [&](int l, int64_t off) { return l < num_leaves ? __ldg(reinterpret_cast<const float4*>(u + off)) : z4; };
+    auto ld4 = [&](int l, int64_t off) { return l < num_leaves ? *reinterpret_cast<const float4*>(u + off) : z4; };
     const int64_t own = row_of(leaf, x, y);
     // The row's cells of the colour are z = p and p + 2: one of them lies at a z end of the leaf.
     const bool p = ((x + y + colour) & 1) != 0;
     const int lz = p ? f1.x : f1.y;
-    const float4 bb = __ldg(reinterpret_cast<const float4*>(b + own)), c = __ldg(reinterpret_cast<const float4*>(u + own));
+    const float4 bb = *reinterpret_cast<const float4*>(b + own), c = *reinterpret_cast<const float4*>(u + own);
     const float4 xp = ld4(lxp, row_of(lxp, (x + 1) & 3, y)), xm = ld4(lxm, row_of(lxm, (x - 1) & 3, y));
     const float4 yp = ld4(lyp, row_of(lyp, x, (y + 1) & 3)), ym = ld4(lym, row_of(lym, x, (y - 1) & 3));
-    const float end = lz < num_leaves ? __ldg(u + row_of(lz, x, y) + (p ? 0 : 3)) : 0.f;
+    const float end = lz < num_leaves ? u[row_of(lz, x, y) + (p ? 0 : 3)] : 0.f;
     const int lateral = (lxp >= num_leaves) + (lxm >= num_leaves) + (lyp >= num_leaves) + (lym >= num_leaves);
     const int ends = lz >= num_leaves;
     auto relax = [&](float vxp, float vxm, float vyp, float vym, float vzp, float vzm, float vb, float vc, int missing) {
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(kThreads) level1_smooth_rows_kernel(const int4
 // colour, (y, z) = (0, p) and (1, 1 - p); 8 loads for the two updates, where a thread per cell of the colour
 // made 16 (95.6M voxels 5.9 -> 4.9 us).
 __global__ void __launch_bounds__(kThreads) level2_smooth_kernel(const int4* __restrict__ nb8, float* u,
-                                                                 const float* __restrict__ b, int num_leaves, int colour,
+                                                                 const float* b, int num_leaves, int colour,
                                                                  float omega, float h2, float gamma,
                                                                  const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
@@ -474,8 +480,8 @@ __global__ void __launch_bounds__(kThreads) level2_smooth_kernel(const int4* __r
     const bool p = ((x + colour) & 1) != 0;
     const int lx = x ? f0.x : f0.y, lza = p ? f1.x : f1.y, lzb = p ? f1.y : f1.x;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    auto quad = [&](const float* q, int l, int cx) { return __ldg(reinterpret_cast<const float4*>(q + ((int64_t)l << 3) + 4 * cx)); };
-    auto cell = [&](int l, int y, int z) { return l < num_leaves ? __ldg(u + ((int64_t)l << 3) + 4 * x + 2 * y + z) : 0.f; };
+    auto quad = [&](const float* q, int l, int cx) { return *reinterpret_cast<const float4*>(q + ((int64_t)l << 3) + 4 * cx); };
+    auto cell = [&](int l, int y, int z) { return l < num_leaves ? u[((int64_t)l << 3) + 4 * x + 2 * y + z] : 0.f; };
     // A quad's cells: .x (0, 0), .y (0, 1), .z (1, 0), .w (1, 1).
     const float4 c = quad(u, leaf, x), in = quad(u, leaf, x ^ 1), bb = quad(b, leaf, x);
     const float4 out = lx < num_leaves ? quad(u, lx, x ^ 1) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -504,8 +510,8 @@ __global__ void __launch_bounds__(kThreads) level2_smooth_kernel(const int4* __r
 // bc (level LG - 1) = the mean of the residuals b - (sum - (6 + gamma missing) u) / h2 of each
 // coarse cell's 8 children at level LG.
 template <int LG>
-__global__ void __launch_bounds__(kThreads) mgl_restrict_kernel(const int4* __restrict__ nb8, const float* __restrict__ u,
-                                                                const float* __restrict__ b, float* __restrict__ bc,
+__global__ void __launch_bounds__(kThreads) mgl_restrict_kernel(const int4* __restrict__ nb8, const float* u,
+                                                                const float* b, float* bc,
                                                                 int num_leaves, float inv_h2, float gamma,
                                                                 const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
@@ -521,7 +527,7 @@ __global__ void __launch_bounds__(kThreads) mgl_restrict_kernel(const int4* __re
         const int64_t f = ((int64_t)cc.leaf << (3 * LG)) + (((x << LG) + y) << LG) + z;
         int missing;
         const float ns = level_nsum<LG>(nb8, u, cc.leaf, x, y, z, num_leaves, missing);
-        sum += __ldg(b + f) - (ns - (6.0f + gamma * (float)missing) * u[f]) * inv_h2;
+        sum += b[f] - (ns - (6.0f + gamma * (float)missing) * u[f]) * inv_h2;
     }
     bc[q] = 0.125f * sum;
 }
@@ -531,9 +537,8 @@ __global__ void __launch_bounds__(kThreads) mgl_restrict_kernel(const int4* __re
 // order of mgl_restrict_kernel, each one's neighbours in the sweeps' order. The first
 // red sweep of level 2 from u = 0 is made in passing. 95.6M voxels: 34 -> 19 us.
 __global__ void __launch_bounds__(kThreads, 3) restrict_level1_kernel(const int4* __restrict__ nb8,
-                                                                      const float* __restrict__ u,
-                                                                      const float* __restrict__ b, float* __restrict__ b2,
-                                                                      float* __restrict__ u2, int num_leaves, float inv_h2,
+                                                                      const float* u, const float* b, float* b2, float* u2,
+                                                                      int num_leaves, float inv_h2,
                                                                       float gamma, float omega2, float h22, float gamma2,
                                                                       const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
@@ -547,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 3) restrict_level1_kernel(const int4
     const bool mzp = f1.x >= num_leaves, mzm = f1.y >= num_leaves;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     auto ld4 = [&](const float* p, int l, int x, int y) {
-        return __ldg(reinterpret_cast<const float4*>(p + ((int64_t)l << 6) + (((x & 3) << 2) + (y & 3)) * 4));
+        return *reinterpret_cast<const float4*>(p + ((int64_t)l << 6) + (((x & 3) << 2) + (y & 3)) * 4);
     };
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     const int x0 = 2 * X, y0 = 2 * Y;
@@ -560,8 +565,8 @@ __global__ void __launch_bounds__(kThreads, 3) restrict_level1_kernel(const int4
             c[i][j] = ld4(u, leaf, x0 + i, y0 + j);
             r[i][j] = ld4(b, leaf, x0 + i, y0 + j);
             const int row = ((x0 + i) * 4 + y0 + j) * 4;
-            zlo[i][j] = mzm ? 0.f : __ldg(u + ((int64_t)f1.y << 6) + row + 3);
-            zhi[i][j] = mzp ? 0.f : __ldg(u + ((int64_t)f1.x << 6) + row);
+            zlo[i][j] = mzm ? 0.f : u[((int64_t)f1.y << 6) + row + 3];
+            zhi[i][j] = mzp ? 0.f : u[((int64_t)f1.x << 6) + row];
         }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {  // k: the coordinate along the side
@@ -607,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 3) restrict_level1_kernel(const int4
 // LC + 1 takes the trilinear interpolation between cell centres: along each axis 3/4 of the
 // parent and 1/4 of the parent's neighbour on the child's side.
 template <int LC>
-__device__ __forceinline__ void gather27(const TopoView& t, const float* __restrict__ uc, int leaf, int X, int Y, int Z,
+__device__ __forceinline__ void gather27(const TopoView& t, const float* uc, int leaf, int X, int Y, int Z,
                                          float v[27]) {
     constexpr int sc = 1 << LC;
 #pragma unroll
@@ -618,7 +623,7 @@ __device__ __forceinline__ void gather27(const TopoView& t, const float* __restr
         int l = leaf;
         if (ox | oy | oz) l = __ldg(t.nbr27 + (int64_t)leaf * 27 + (ox + 1) * 9 + (oy + 1) * 3 + (oz + 1));
         cx -= ox * sc, cy -= oy * sc, cz -= oz * sc;
-        v[k] = l < 0 ? 0.f : __ldg(uc + ((int64_t)l << (3 * LC)) + (((cx << LC) + cy) << LC) + cz);
+        v[k] = l < 0 ? 0.f : uc[((int64_t)l << (3 * LC)) + (((cx << LC) + cy) << LC) + cz];
     }
 }
 
@@ -750,7 +755,7 @@ __global__ void __launch_bounds__(kThreads, 3) mg16_restrict_kernel(const int4* 
 // it (4 contiguous floats each, and one value past each end), interpolated along z once for the
 // rows that share them. A thread per fine row loaded 4 columns and 12 table entries for 8 voxels and
 // was bound by issue: 95.6M voxels 102 -> 51 us, 23.1M voxels 37 -> 20 us.
-__global__ void __launch_bounds__(kThreads, 3) mg16_prolong_kernel(TopoView t, const float* __restrict__ u1, __half* e,
+__global__ void __launch_bounds__(kThreads, 3) mg16_prolong_kernel(TopoView t, const float* u1, __half* e,
                                                                    const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -784,9 +789,9 @@ __global__ void __launch_bounds__(kThreads, 3) mg16_prolong_kernel(TopoView t, c
             }
             const int off = (((cx & 3) << 2) + (cy & 3)) << 2;
             const float4 m = l < 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
-                                   : __ldg(reinterpret_cast<const float4*>(u1 + ((int64_t)l << 6) + off));
-            const float lo = lm < 0 ? 0.f : __ldg(u1 + ((int64_t)lm << 6) + off + 3);
-            const float hi = lp < 0 ? 0.f : __ldg(u1 + ((int64_t)lp << 6) + off);
+                                   : *reinterpret_cast<const float4*>(u1 + ((int64_t)l << 6) + off);
+            const float lo = lm < 0 ? 0.f : u1[((int64_t)lm << 6) + off + 3];
+            const float hi = lp < 0 ? 0.f : u1[((int64_t)lp << 6) + off];
             const float col[6] = {lo, m.x, m.y, m.z, m.w, hi};
 #pragma unroll
             for (int Z = 0; Z < 4; ++Z) {
@@ -820,9 +825,8 @@ __global__ void __launch_bounds__(kThreads, 3) mg16_prolong_kernel(TopoView t, c
 
 // u (level LG) += the correction uc (level LG - 1), one thread per coarse cell.
 template <int LG>
-__global__ void __launch_bounds__(kThreads) mgl_prolong_kernel(TopoView t, const float* __restrict__ uc,
-                                                               float* __restrict__ u, const double* __restrict__ check,
-                                                               double tol2) {
+__global__ void __launch_bounds__(kThreads) mgl_prolong_kernel(TopoView t, const float* uc, float* u,
+                                                               const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -843,9 +847,8 @@ __global__ void __launch_bounds__(kThreads) mgl_prolong_kernel(TopoView t, const
 // are the 2 x 2 rows of level 1 above them, read and written as 16 bytes each; the 3 x 3 level-2
 // columns around it are read once (8 bytes and one value past each end). The sums are interp8's, in
 // its order. 95.6M voxels: 28 -> 14 us.
-__global__ void __launch_bounds__(kThreads, 3) prolong_level2_kernel(TopoView t, const float* __restrict__ uc,
-                                                                     float* __restrict__ u, const double* __restrict__ check,
-                                                                     double tol2) {
+__global__ void __launch_bounds__(kThreads, 3) prolong_level2_kernel(TopoView t, const float* uc, float* u,
+                                                                     const double* __restrict__ check, double tol2) {
     if (done(check, tol2)) return;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (tid >= (t.num_leaves << 2)) return;
@@ -881,10 +884,10 @@ __global__ void __launch_bounds__(kThreads, 3) prolong_level2_kernel(TopoView t,
             const int off = ((cx << 1) + cy) << 1;
             const int(&q)[3] = l[a == 2][c == 2];
             const float2 m = q[1] < 0 ? make_float2(0.f, 0.f)
-                                      : __ldg(reinterpret_cast<const float2*>(uc + ((int64_t)q[1] << 3) + off));
-            v[a][c][0] = q[0] < 0 ? 0.f : __ldg(uc + ((int64_t)q[0] << 3) + off + 1);
+                                      : *reinterpret_cast<const float2*>(uc + ((int64_t)q[1] << 3) + off);
+            v[a][c][0] = q[0] < 0 ? 0.f : uc[((int64_t)q[0] << 3) + off + 1];
             v[a][c][1] = m.x, v[a][c][2] = m.y;
-            v[a][c][3] = q[2] < 0 ? 0.f : __ldg(uc + ((int64_t)q[2] << 3) + off);
+            v[a][c][3] = q[2] < 0 ? 0.f : uc[((int64_t)q[2] << 3) + off];
         }
     // The neighbour on child i's side lies across the leaf's side where i == X, else within.
 #pragma unroll

@@ -61,9 +61,10 @@ constexpr int64_t kTwoLeafLimit = 6000;
 constexpr int kNbXp = 22, kNbXm = 4, kNbYp = 16, kNbYm = 10, kNbZp = 14, kNbZm = 12;
 
 __device__ __forceinline__ uint2 ld8(const __half* p) { return __ldg(reinterpret_cast<const uint2*>(p)); }
-// Loads that other threads of this launch may write: the colour being updated is only read by
-// the thread that writes it, so plain (non-.nc) loads of it are enough; the other colour is
-// read-only during the launch.
+// Loads of e. Plain ones, of both colours: a half-sweep starts while the preceding one, which writes the
+// other colour, still runs (programmatic dependent launch), and a non-coherent load (__ldg) is only
+// allowed on memory that nothing writes while the kernel lives; the compiler may move it above
+// griddepcontrol.wait. They cost the same.
 __device__ __forceinline__ uint2 ld8_rw(const __half* p) { return *reinterpret_cast<const uint2*>(p); }
 
 __device__ __forceinline__ uint32_t half_at(uint2 v, int j) {
@@ -111,10 +112,7 @@ __device__ __forceinline__ uint2 relax_row(uint2 XP, uint2 XM, uint2 YP, uint2 Y
 //
 // kZero: e = 0 before this (red) half-sweep, the first of a solve: every neighbour and old
 // value is 0, nothing of e is read, and the row's black entries are written as 0.
-// kShared: other CTAs of the same launch write e (the persistent solve): every load of e takes
-// the coherent path; otherwise the colour not being updated is read-only during the launch and
-// goes through the read-only cache. kPdl: wait for the preceding launch (griddepcontrol.wait)
-// before the first load of e.
+// kPdl: wait for the preceding launch (griddepcontrol.wait) before the first load of e.
 //
 // Warp w of a leaf takes the 32 rows of parity w of a + b, lane l the row at R = 32 w + l
 // (a = l / 4, b = 2 (l % 4) + ((a + w) & 1)), so the z parity of the colour is uniform in a warp
@@ -125,14 +123,13 @@ __device__ __forceinline__ uint2 relax_row(uint2 XP, uint2 XM, uint2 YP, uint2 Y
 // zero leaf. Offsets are 32-bit element counts (fewer than 2^22 leaves).
 constexpr int kLeavesPerGroup = kLeavesPerBlock * kLeavesPerThread;
 
-template <bool kZero, bool kShared, bool kPdl, int kLeaves, typename Mid>
+template <bool kZero, bool kPdl, int kLeaves, typename Mid>
 __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const __half* __restrict__ rhs, __half* e,
                                             int num_leaves, int g, int colour, float omega, Mid&& mid) {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;
     const int a = lane >> 2, b = 2 * (lane & 3) + ((a + w) & 1);
     const int p = (w + colour) & 1;  // z parity of this colour in the warp's rows
     const uint32_t rowc = ((uint32_t)colour << 8) | (uint32_t)(4 * (32 * w + lane));  // own entries within a leaf
-    auto lde = [](const __half* q) { return kShared ? ld8_rw(q) : ld8(q); };
     const int leaf0 = g * (kLeavesPerBlock * kLeaves) + (int)(threadIdx.x >> 6);
     uint32_t own[kLeaves];
     bool live[kLeaves];
@@ -177,17 +174,17 @@ __device__ __forceinline__ void relax_group(const int* __restrict__ nb8, const _
 #pragma unroll
         for (int k = 0; k < kLeaves; ++k) {
             C[k] = ld8_rw(e + own[k]);
-            K[k] = lde(e + (own[k] ^ 256u));
+            K[k] = ld8_rw(e + (own[k] ^ 256u));
         }
 #pragma unroll
         for (int k = 0; k < kLeaves; ++k) {
             const uint32_t lf = own[k] >> 9;
-            XP[k] = lde(e + row(a == 7 ? nx[k] : lf, (a + 1) & 7, b));
-            XM[k] = lde(e + row(a == 0 ? nx[k] : lf, (a - 1) & 7, b));
-            YP[k] = lde(e + row(b == 7 ? ny[k] : lf, a, (b + 1) & 7));
-            YM[k] = lde(e + row(b == 0 ? ny[k] : lf, a, (b - 1) & 7));
+            XP[k] = ld8_rw(e + row(a == 7 ? nx[k] : lf, (a + 1) & 7, b));
+            XM[k] = ld8_rw(e + row(a == 0 ? nx[k] : lf, (a - 1) & 7, b));
+            YP[k] = ld8_rw(e + row(b == 7 ? ny[k] : lf, a, (b + 1) & 7));
+            YM[k] = ld8_rw(e + row(b == 0 ? ny[k] : lf, a, (b - 1) & 7));
             const __half* zq = e + ((nz[k] << 9) | ((own[k] ^ 256u) & 511u)) + 3u * (uint32_t)(p ^ 1);
-            ZC[k] = kShared ? (uint32_t)*reinterpret_cast<const unsigned short*>(zq) : (uint32_t)__half_as_ushort(__ldg(zq));
+            ZC[k] = (uint32_t)*reinterpret_cast<const unsigned short*>(zq);
         }
         mid();  // every load of the pass is in flight
 #pragma unroll
@@ -218,7 +215,7 @@ __global__ void __launch_bounds__(kThreads, kLeaves == 4 ? kHalfCtasPerSm : kHal
     constexpr int kPerGroup = kLeavesPerBlock * kLeaves;
     const int groups = (num_leaves + kPerGroup - 1) / kPerGroup;
     for (int g = blockIdx.x; g < groups; g += gridDim.x)
-        relax_group<kZero, false, true, kLeaves>(nb8, rhs, e, num_leaves, g, colour, omega, [] {});
+        relax_group<kZero, true, kLeaves>(nb8, rhs, e, num_leaves, g, colour, omega, [] {});
 }
 
 // ---- FP32 ---------------------------------------------------------------------------------
@@ -269,14 +266,13 @@ __device__ __forceinline__ float4 relax_row_f32(float4 XP, float4 XM, float4 YP,
 // scales the right-hand side.
 constexpr int kF32LeavesPerGroup = kF32LeavesPerBlock * kF32LeavesPerThread;
 
-template <bool kZero, bool kShared, bool kPdl, bool kWalls, typename Mid>
+template <bool kZero, bool kPdl, bool kWalls, typename Mid>
 __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, const float* __restrict__ rhs, float* e,
                                                 int num_leaves, int g, int colour, float omega, float dx2, Mid&& mid) {
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 1;
     const int a = lane >> 2, b = 2 * (lane & 3) + ((a + w) & 1);
     const int p = (w + colour) & 1;
     const uint32_t rowc = ((uint32_t)colour << 8) | (uint32_t)(4 * (32 * w + lane));
-    auto lde = [](const float* q) { return kShared ? ldf4_rw(q) : ldf4(q); };
     const int leaf0 = g * kF32LeavesPerGroup + (int)(threadIdx.x >> 6);
     uint32_t own[kF32LeavesPerThread];
     bool live[kF32LeavesPerThread];
@@ -330,17 +326,17 @@ __device__ __forceinline__ void relax_group_f32(const int* __restrict__ nb8, con
 #pragma unroll
         for (int k = 0; k < kF32LeavesPerThread; ++k) {
             C[k] = ldf4_rw(e + own[k]);
-            K[k] = lde(e + (own[k] ^ 256u));
+            K[k] = ldf4_rw(e + (own[k] ^ 256u));
         }
 #pragma unroll
         for (int k = 0; k < kF32LeavesPerThread; ++k) {
             const uint32_t lf = own[k] >> 9;
-            XP[k] = lde(e + row(a == 7 ? nx[k] : lf, (a + 1) & 7, b));
-            XM[k] = lde(e + row(a == 0 ? nx[k] : lf, (a - 1) & 7, b));
-            YP[k] = lde(e + row(b == 7 ? ny[k] : lf, a, (b + 1) & 7));
-            YM[k] = lde(e + row(b == 0 ? ny[k] : lf, a, (b - 1) & 7));
+            XP[k] = ldf4_rw(e + row(a == 7 ? nx[k] : lf, (a + 1) & 7, b));
+            XM[k] = ldf4_rw(e + row(a == 0 ? nx[k] : lf, (a - 1) & 7, b));
+            YP[k] = ldf4_rw(e + row(b == 7 ? ny[k] : lf, a, (b + 1) & 7));
+            YM[k] = ldf4_rw(e + row(b == 0 ? ny[k] : lf, a, (b - 1) & 7));
             const float* zq = e + ((nz[k] << 9) | ((own[k] ^ 256u) & 511u)) + 3u * (uint32_t)(p ^ 1);
-            ZC[k] = kShared ? *zq : __ldg(zq);
+            ZC[k] = *zq;
         }
         mid();  // every load of the pass is in flight
 #pragma unroll
@@ -368,7 +364,7 @@ __global__ void __launch_bounds__(kF32Threads, kF32ShortGridCtasPerSm)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int groups = (num_leaves + kF32LeavesPerGroup - 1) / kF32LeavesPerGroup;
     for (int g = blockIdx.x; g < groups; g += gridDim.x)
-        relax_group_f32<kZero, false, true, kWalls>(nb8, rhs, e, num_leaves, g, colour, omega, dx2, [] {});
+        relax_group_f32<kZero, true, kWalls>(nb8, rhs, e, num_leaves, g, colour, omega, dx2, [] {});
 }
 
 // ---- The persistent solve -------------------------------------------------------------------
@@ -486,14 +482,14 @@ __global__ void __launch_bounds__(kThreads, kShortGridCtasPerSm) rbgs_split_solv
         };
         if constexpr (kHalf) {
             if (kZeroFirst && h == 0)
-                relax_group<true, true, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, 0, omega, mid);
+                relax_group<true, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, 0, omega, mid);
             else
-                relax_group<false, true, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, h & 1, omega, mid);
+                relax_group<false, false, kLeavesPerThread>(nb8, rhs, e, num_leaves, g, h & 1, omega, mid);
         } else {
             if (kZeroFirst && h == 0)
-                relax_group_f32<true, true, false, false>(nb8, rhs, e, num_leaves, g, 0, omega, dx2, mid);
+                relax_group_f32<true, false, false>(nb8, rhs, e, num_leaves, g, 0, omega, dx2, mid);
             else
-                relax_group_f32<false, true, false, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, dx2, mid);
+                relax_group_f32<false, false, false>(nb8, rhs, e, num_leaves, g, h & 1, omega, dx2, mid);
         }
         ph = h, pg = g;
         h = nh, g = ng, x = nx, ok = nok;
