@@ -210,6 +210,9 @@ struct Context {
     int spare_graph_ok = -1;
     void release_spare_graphs();
     SpareGraph* find_graph(const std::vector<uintptr_t>& key);
+    // The latest factors of checked FP32 solves that no loop graph was made for (hns_step.cu).
+    std::vector<float> loop_omegas;
+    static constexpr size_t kMaxLoopOmegas = 16;
     // Whether the context's stream is being captured into a graph (work enqueued now runs only
     // when the graph does: a table built under capture is not marked built).
     bool stream_capturing() const;

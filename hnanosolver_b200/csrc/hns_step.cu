@@ -34,34 +34,48 @@ namespace {
 
 __device__ __forceinline__ bool passed(const double* c, double tol2) { return c[0] <= tol2 * c[1]; }
 
-// The loop over a solve's checks (run_check_loop): `acc` takes the residual of the check being
-// evaluated, *next its number. enter: after check 0; step: after the iterations of one check.
-__global__ void loop_enter_kernel(cudaGraphConditionalHandle h, const double* __restrict__ slots, double* acc, int* next,
-                                  int nchecks, double tol2) {
-    acc[0] = acc[1] = 0.0;
-    *next = 1;
-    cudaGraphSetConditional(h, nchecks > 1 && !passed(slots, tol2) ? 1u : 0u);
+// The loop over a solve's checks (run_check_loop): the residual of the check being evaluated, its
+// number, and the solve's tolerance and checks, which the graph reads here.
+struct CheckLoop {
+    double acc[2];
+    double tol2;
+    int next, nchecks;
+};
+__global__ void loop_set_kernel(CheckLoop* s, int nchecks, double tol2) { *s = CheckLoop{{0.0, 0.0}, tol2, 1, nchecks}; }
+// enter: after check 0; step: after the iterations of one check.
+__global__ void loop_enter_kernel(cudaGraphConditionalHandle h, const double* __restrict__ slots, const CheckLoop* s) {
+    cudaGraphSetConditional(h, s->nchecks > 1 && !passed(slots, s->tol2) ? 1u : 0u);
 }
-__global__ void loop_step_kernel(cudaGraphConditionalHandle h, double* slots, double* acc, int* next, int nchecks,
-                                 double tol2) {
-    const int c = *next;
-    slots[2 * c] = acc[0], slots[2 * c + 1] = acc[1];
-    const bool done = passed(acc, tol2);
-    acc[0] = acc[1] = 0.0;
-    *next = c + 1;
-    cudaGraphSetConditional(h, !done && c + 1 < nchecks ? 1u : 0u);
+__global__ void loop_step_kernel(cudaGraphConditionalHandle h, double* slots, CheckLoop* s) {
+    const int c = s->next;
+    slots[2 * c] = s->acc[0], slots[2 * c + 1] = s->acc[1];
+    const bool done = passed(s->acc, s->tol2);
+    s->acc[0] = s->acc[1] = 0.0;
+    s->next = c + 1;
+    cudaGraphSetConditional(h, !done && c + 1 < s->nchecks ? 1u : 0u);
 }
 
-// Runs `body` (the iterations between two checks and the residual's evaluation into acc, as
+// Runs `body` (the iterations between two checks and the residual's evaluation into state->acc, as
 // launches that test no check) once per check from check 1 on, until one passes: a graph whose
 // conditional node repeats on the device, in place of launches for every check up to the cap that
-// return at once after convergence (11 us each on 45,198 leaves). The graph is made on the first
-// call with this key. Returns false, with nothing enqueued, where a graph cannot be made.
-bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots, double* acc, int* next, int nchecks,
-                    double tol2, const std::function<void()>& body) {
+// return at once after convergence (11 us each on 45,198 leaves). Returns false, with nothing enqueued,
+// where there is no graph.
+// The key holds what the launches bake in. A graph is made for the first factor omega of a context and
+// for one that comes again: a program that solves with another one each time would make, and throw
+// away, a graph per solve. (The half-sweeps do not read omega from memory: 32.4 -> 33.3 us each on
+// 45,198 leaves.)
+bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots, CheckLoop* state, int nchecks, double tol2,
+                    float omega, const std::function<void()>& body) {
     if (c.spare_graph_ok == 0) return false;
     Context::SpareGraph* found = c.find_graph(key);
     if (found == nullptr) {
+        auto& seen = c.loop_omegas;
+        if (!seen.empty() && std::find(seen.begin(), seen.end(), omega) == seen.end()) {
+            if (seen.size() >= Context::kMaxLoopOmegas) seen.erase(seen.begin());
+            seen.push_back(omega);
+            return false;
+        }
+        if (seen.empty()) seen.push_back(omega);
         if (c.spare_graphs.size() >= Context::kMaxSpareGraphs) c.release_spare_graphs();
         Context::SpareGraph sg;
         sg.key = key;
@@ -72,7 +86,7 @@ bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots
         if (ok) ok = cudaGraphConditionalHandleCreate(&h, sg.graph, 0, 0) == cudaSuccess;
         if (ok) {
             cudaKernelNodeParams kp = {};
-            void* args[] = {&h, &slots, &acc, &next, &nchecks, &tol2};
+            void* args[] = {&h, &slots, &state};
             kp.func = reinterpret_cast<void*>(loop_enter_kernel);
             kp.gridDim = dim3(1);
             kp.blockDim = dim3(1);
@@ -96,7 +110,7 @@ bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots
             if (ok) {
                 try {
                     body();
-                    loop_step_kernel<<<1, 1, 0, c.stream>>>(h, slots, acc, next, nchecks, tol2);
+                    loop_step_kernel<<<1, 1, 0, c.stream>>>(h, slots, state);
                     HNS_LAUNCHED();
                 } catch (const Error&) {
                     ok = false;
@@ -118,16 +132,11 @@ bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots
         c.spare_graphs.push_back(sg);
         found = &c.spare_graphs.back();
     }
+    loop_set_kernel<<<1, 1, 0, c.stream>>>(state, nchecks, tol2);
+    HNS_LAUNCHED();
     HNS_CUDA(cudaGraphLaunch(found->exec, c.stream));
     HNS_LAUNCHED();  // the kernel before the loop
     return true;
-}
-
-template <typename T>
-uintptr_t bits_of(T v) {
-    uint64_t b = 0;
-    std::memcpy(&b, &v, sizeof v);
-    return (uintptr_t)b;
 }
 
 }  // namespace
@@ -198,6 +207,7 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
         // Check 0's iterations as launches, the later checks' as the device-side loop; the rest, past
         // the last check, below.
         const int E = plan->check_every;
+        auto* state = reinterpret_cast<CheckLoop*>(c.scratch_f32("check_loop", sizeof(CheckLoop) / sizeof(float)));
         auto iterations = [&](int n, bool from_zero) {
             for (int q = 0; q < n; ++q) {
                 launch_rbgs_split_half_f32(c, w.nb8, w.rhs, w.e, 0, from_zero && q == 0, omega, dx2, nullptr, tol2, false,
@@ -211,12 +221,13 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
             iterations(1, false);
         };
         one_check(plan->slots, zero);
-        double* acc = reinterpret_cast<double*>(c.scratch_f32("check_loop", 8));
-        int* next = reinterpret_cast<int*>(acc + 2);
-        const std::vector<uintptr_t> key = {
-            (uintptr_t)0x6c6f6f70, (uintptr_t)w.rhs, (uintptr_t)w.e, (uintptr_t)w.nb8, (uintptr_t)plan->slots, (uintptr_t)acc,
-            (uintptr_t)E, (uintptr_t)plan->num_checks, bits_of(omega), bits_of(tol2), (uintptr_t)walls};
-        if (run_check_loop(c, key, plan->slots, acc, next, plan->num_checks, tol2, [&] { one_check(acc, false); }))
+        uint32_t omega_bits = 0;
+        std::memcpy(&omega_bits, &omega, sizeof omega_bits);
+        const std::vector<uintptr_t> key = {(uintptr_t)0x6c6f6f70, (uintptr_t)w.rhs, (uintptr_t)w.e,
+                                            (uintptr_t)w.nb8, (uintptr_t)plan->slots, (uintptr_t)state,
+                                            (uintptr_t)E, (uintptr_t)walls, (uintptr_t)omega_bits};
+        if (run_check_loop(c, key, plan->slots, state, plan->num_checks, tol2, omega,
+                           [&] { one_check(state->acc, false); }))
             it = plan->num_checks * E;
         else
             it = E;
