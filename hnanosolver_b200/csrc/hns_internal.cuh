@@ -340,9 +340,10 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
 // must have been written by kernels that finished before that one started.
 void launch_split_face_table(const Context& c, int* nb8);
 // short_grid: one wave of CTAs looping over the leaves, for a launch expected to find the
-// refinement converged and return at once.
+// refinement converged and return at once. in_cycle: one of a multigrid cycle's.
 void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, void* e, int colour, bool e_zero,
-                            float omega, const double* check, double tol2, bool short_grid = false);
+                            float omega, const double* check, double tol2, bool short_grid = false,
+                            bool in_cycle = false);
 // A whole FP16 inner solve on colour-split leaves in one cooperative launch: half_sweeps
 // half-sweeps (red first), the values of as many launch_rbgs_split_half calls to the bit. e_zero:
 // e = 0 before it. Follows any kernel (no programmatic dependency).

@@ -1135,8 +1135,8 @@ void mg16_vcycle(Context& c, const int* nb8, const void* rhat, void* e, bool e_z
     }
     auto fine = [&](bool zero_first) {
         for (int it = 0; it < kMgNu; ++it) {
-            launch_rbgs_split_half(c, nb8, rhat, e, 0, zero_first && it == 0, 1.0f, check, tol2, false);
-            launch_rbgs_split_half(c, nb8, rhat, e, 1, false, 1.0f, check, tol2, false);
+            launch_rbgs_split_half(c, nb8, rhat, e, 0, zero_first && it == 0, 1.0f, check, tol2, false, true);
+            launch_rbgs_split_half(c, nb8, rhat, e, 1, false, 1.0f, check, tol2, false, true);
         }
     };
     fine(e_zero);

@@ -51,11 +51,17 @@ constexpr int kLeavesPerThread = 4;  // leaves a thread relaxes its row in
 constexpr int kThreads = 64 * kLeavesPerBlock;
 constexpr int kShortGridCtasPerSm = 6;  // the register limit at 80 registers and 128 threads
 constexpr int kHalfCtasPerSm = 6;       // the half-sweep kernel's launch bound
-// Grids of up to kTwoLeafLimit leaves take two leaves per thread at eight CTAs per SM: with four, less
-// than a wave of CTAs is spread unevenly over the SMs. us per half-sweep, four -> two: 1,493 leaves
-// 3.4 -> 2.3, 3,300 2.8 -> 2.7, 4,096 3.5 -> 2.7, 5,300 3.5 -> 3.0, 6,594 3.5 -> 3.8, 10,000 4.75 -> 4.8.
+// Smaller grids take two leaves per thread at eight CTAs per SM: with four, less than a wave of CTAs is
+// spread unevenly over the SMs. Where the launches of several streams fill the SMs between them, four
+// leaves in flight per thread win from about 4,000 leaves on in the red-black solves, hundreds of these
+// launches in a row; the multigrid cycle's few sit between other kernels. Step of three outer iterations,
+// us, four -> two, alone / three contexts taking turns:
+//   leaves                      1,500                   3,700                   4,500                   5,900
+//   red-black  863 -> 725 / 481 -> 469  1037 -> 859 / 504 -> 505  1081 -> 922 / 569 -> 585  1128 -> 1110 / 698 -> 742
+//   multigrid  587 -> 573 / 377 -> 374   801 -> 777 / 446 -> 439   878 -> 845 / 503 -> 496    934 ->  934 / 573 -> 571
+// 6,594 leaves, us per half-sweep: 3.5 -> 3.8.
 constexpr int kHalfCtasPerSm2 = 8;
-constexpr int64_t kTwoLeafLimit = 6000;
+constexpr int64_t kTwoLeafLimit = 4000, kTwoLeafLimitCycle = 6000;
 
 // nbr27 indices of the six face neighbours: (dx+1)*9 + (dy+1)*3 + (dz+1).
 constexpr int kNbXp = 22, kNbXm = 4, kNbYp = 16, kNbYm = 10, kNbZp = 14, kNbZm = 12;
@@ -643,11 +649,11 @@ void launch_split_face_table(const Context& c, int* nb8) {
 }
 
 void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, void* e, int colour, bool e_zero,
-                            float omega, const double* check, double tol2, bool short_grid) {
+                            float omega, const double* check, double tol2, bool short_grid, bool in_cycle) {
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     if (L >= (int64_t(1) << 22)) fail(HNS_ERR_INVALID_ARG, "too many leaves for the colour-split inner solve");
-    const bool two = L <= kTwoLeafLimit;
+    const bool two = L <= (in_cycle ? kTwoLeafLimitCycle : kTwoLeafLimit);
     const int per_block = kLeavesPerBlock * (two ? 2 : kLeavesPerThread);
     unsigned blocks = (unsigned)((L + per_block - 1) / per_block);
     // A launch that will most likely return at once (the refinement expected to have converged)
