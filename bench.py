@@ -707,7 +707,7 @@ def ours(args, wl):
             "clocks": clk,
             "adjoint": adjoint,
         }
-        print(json.dumps(line), flush=True)
+        print_line(line, args)
     g.close()
     replicas.finish(R)
 
@@ -1118,7 +1118,7 @@ def ours_fire(args, wl):
             "clocks": clk,
             "adjoint": adjoint,
         }
-        print(json.dumps(line), flush=True)
+        print_line(line, args)
     g.close()
     replicas.finish(R)
 
@@ -1255,9 +1255,31 @@ def box64_ours(args):
                         "d2h_bytes_per_step": 16 * n, "steps": e2e_steps,
                         "path": "hns_step_plain_host (C ABI, pinned FP32 host buffers), zero-gradient walls"},
                 "gpu_launches": z["kernel_launches"], "clocks": z["clocks"]}
-        print(json.dumps(line), flush=True)
+        print_line(line, args)
     g.close()
     replicas.finish(R)
+
+
+def reference_unavailable():
+    """Why the reference's library (oracle/_ref) cannot be used here, None where it can. It is built
+    first where the reference's sources are and the library is not."""
+    from oracle import binding
+
+    if not os.path.exists(binding.REF_SO):
+        try:
+            binding.build()
+        except (OSError, subprocess.CalledProcessError) as e:
+            return f"oracle/_ref/libhns_ref.so is not built and could not be: {e}"
+        if not os.path.exists(binding.REF_SO):
+            return "oracle/_ref/libhns_ref.so is not built: no reference sources (HNS_REFERENCE or the recipe's default checkout)"
+    return None
+
+
+def print_line(line, args):
+    """Prints one result line; a CPU baseline that could not run is named in its details."""
+    if args.cpu_unavailable:
+        line["details"]["cpu_baseline"] = "unavailable: " + args.cpu_unavailable
+    print(json.dumps(line), flush=True)
 
 
 def main():
@@ -1294,14 +1316,14 @@ def main():
     args = ap.parse_args()
     if args.warmup < 3:
         ap.error("--warmup must be at least 3")
-    from oracle import binding
-
-    if not os.path.exists(binding.REF_SO):  # built from the reference's sources (oracle/Makefile)
-        if args.impl == "reference":
-            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libhns_ref.so is not built: no reference sources"}),
-                  flush=True)
+    args.cpu_unavailable = None
+    if dist_info()[0] == 0 and (args.impl == "reference" or not args.no_cpu_baseline):
+        args.cpu_unavailable = reference_unavailable()
+        if args.cpu_unavailable and args.impl == "reference":
+            print(json.dumps({"impl": "reference", "unavailable": args.cpu_unavailable}), flush=True)
             return
-        args.no_cpu_baseline = True
+        if args.cpu_unavailable:  # the line says so under details
+            args.no_cpu_baseline = True
     if args.workload == "box64":
         (box64_reference if args.impl == "reference" else box64_ours)(args)
         return
