@@ -257,6 +257,19 @@ struct Context {
     double* reduce_slots(int count);
 };
 
+// The stream that the context's own graphs are captured on: the context's non-blocking one, whatever
+// stream the caller gave it (nothing is enqueued there). A caller's stream may be blocking, and while
+// such a stream captures, any other thread's work on the legacy default stream fails and ends the capture; or
+// it may be the default stream, which cannot capture.
+struct CaptureStream {
+    Context& c;
+    cudaStream_t saved;
+    explicit CaptureStream(Context& ctx) : c(ctx), saved(ctx.stream) { c.stream = c.own_stream; }
+    ~CaptureStream() { c.stream = saved; }
+    CaptureStream(const CaptureStream&) = delete;
+    CaptureStream& operator=(const CaptureStream&) = delete;
+};
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev);

@@ -446,6 +446,7 @@ bool run_spare_graph(Context& c, const std::vector<uintptr_t>& key, const double
         }
         if (ok) {
             // The body's launches are captured, not run; no phase events inside the graph.
+            const CaptureStream on(c);
             const bool prof = c.profiling;
             c.profiling = false;
             ok = cudaStreamBeginCaptureToGraph(c.stream, body_graph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) ==

@@ -103,6 +103,7 @@ bool run_check_loop(Context& c, const std::vector<uintptr_t>& key, double* slots
             if (ok) body_graph = cp.conditional.phGraph_out[0];
         }
         if (ok) {
+            const CaptureStream on(c);
             const bool prof = c.profiling;
             c.profiling = false;
             ok = cudaStreamBeginCaptureToGraph(c.stream, body_graph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) ==
