@@ -12,7 +12,8 @@ LIB = os.path.join(PKG, "libhns.so")
 
 # -fmad=false: no implicit multiply-add contraction, so that the FP32 kernels round exactly
 # as the reference's operations are written (explicit fmaf only where the reference calls
-# __fmaf_rn). The kernels are memory-bound; the extra FP instructions cost nothing measurable.
+# __fmaf_rn). The issue-bound kernels (the advections, the confinement) pay for the separate
+# multiplications and additions; the rounding of the reference's results asks for them.
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17", "-fmad=false",

@@ -1,13 +1,12 @@
-// Vorticity confinement (vorticityConfinement, src/Cuda/Kernel.cu:682-727, with the curl of
-// computeVorticityMag, src/Cuda/Utils.cuh:226-243) on a leaf tile in shared memory.
+// The curl of a leaf and of a one-voxel ring around it (computeVorticityMag, src/Cuda/Utils.cuh:226-243) on a
+// tile in shared memory: the first pass of the confinement's adjoint (hns_adjoint.cu). The forward
+// steps take half rows instead (hns_confine_rows.cuh).
 //
-// A voxel's force needs the curl at the voxel and |curl| at the voxels fs away along each axis
-// (fs = int(factorScale)); each curl reads the six face neighbours. For |fs| <= 1 every value a
-// leaf needs lies in the box of local coordinates [-2, 9]^3 around it: the tile stages that box's
-// velocity once (0 outside the domain), computes the curl and its magnitude once for each cell of
-// [-1, 8]^3, and each voxel then reads its curl and the six magnitudes from shared memory. The
-// gather form recomputes the 7 curls of every voxel from 42 global vec3 reads; the values and the
-// order of every operation are the same, so are the results.
+// A voxel's force (vorticityConfinement, src/Cuda/Kernel.cu:682-727) needs the curl at the voxel and |curl|
+// at the voxels fs away along each axis (fs = int(factorScale)); each curl reads the six face neighbours.
+// For |fs| <= 1 every value a leaf needs lies in the box of local coordinates [-2, 9]^3 around it: the
+// tile stages that box's velocity once (0 outside the domain) and computes the curl and its magnitude
+// once for each cell of [-1, 8]^3.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -57,25 +56,6 @@ __device__ __forceinline__ void confine_tile(const LeafNbhd& L, const V* __restr
         T.m[c] = __fsqrt_rn(ox * ox + oy * oy + oz * oz);
     }
     __syncthreads();
-}
-
-// The confinement force's velocity at local voxel (a, b, d) of the tile: u + scale (N x omega) dt.
-__device__ __forceinline__ float3 confine_at(const ConfineTile& T, int a, int b, int d, int fs, float inv_dx, float dt,
-                                             float scale) {
-    const int c = conf_wi(a, b, d);
-    const float ox = T.w[0][c], oy = T.w[1][c], oz = T.w[2][c];
-    const float mpx = T.m[conf_wi(a + fs, b, d)], mmx = T.m[conf_wi(a - fs, b, d)];
-    const float mpy = T.m[conf_wi(a, b + fs, d)], mmy = T.m[conf_wi(a, b - fs, d)];
-    const float mpz = T.m[conf_wi(a, b, d + fs)], mmz = T.m[conf_wi(a, b, d - fs)];
-    const float gx = (mpx - mmx) * 0.5f * inv_dx;
-    const float gy = (mpy - mmy) * 0.5f * inv_dx;
-    const float gz = (mpz - mmz) * 0.5f * inv_dx;
-    const float glen = sqrtf(gx * gx + gy * gy + gz * gz) + 1e-5f;
-    const float nx = gx / glen, ny = gy / glen, nz = gz / glen;
-    const int q = conf_vi(a, b, d);
-    const float3 u = make_float3(T.v[0][q], T.v[1][q], T.v[2][q]);
-    const float fx = scale * (ny * oz - nz * oy), fy = scale * (nz * ox - nx * oz), fz = scale * (nx * oy - ny * ox);
-    return make_float3(u.x + fx * dt, u.y + fy * dt, u.z + fz * dt);
 }
 
 }  // namespace dev

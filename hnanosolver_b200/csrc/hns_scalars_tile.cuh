@@ -23,7 +23,7 @@ struct ScalarPass {
     float* out[kScalarsPerPass];
 };
 
-// kCount fields; kFifth: the fifth rides with the velocity.
+// kCount fields, the fifth beside the velocity.
 template <int kCount>
 struct ScalarCell {
     float4 v, f;

@@ -18,8 +18,9 @@
 // Bound by the two reads of the voxel list and by the call's allocations and three host waits: the
 // band of a 512^3 shell (12M voxels, padding 2, 46,000 leaves), context made and destroyed, took
 // 8.7 ms with a radix sort of one key per voxel (1.4 ms of kernels, 300 MB of temporary arrays), 2.1 ms
-// with the tables in three allocations, and takes 1.7 ms with them in two (0.23 ms of kernels; an
-// allocation and its release cost the host 0.6 ms).
+// with the tables in three allocations, and takes 1.7 ms with them in two, in a process that does
+// nothing else (0.23 ms of kernels; an allocation and its release cost the host 0.6 ms, and more beside
+// other contexts: 2.3 to 3.4 ms with three taking turns).
 #include <cuda_runtime.h>
 
 #include <algorithm>
