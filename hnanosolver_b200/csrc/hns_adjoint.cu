@@ -686,7 +686,7 @@ void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, fl
         return;
     }
     const size_t n = (size_t)c.num_voxels();
-    if (lam == nullptr) lam = adj_scratch(c);
+    if (lam == nullptr) lam = c.scratch_f32("adjoint_lam", n);
     HNS_CUDA(cudaMemcpyAsync(lam, p_bar, n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
     const float a = omega * dev::kInv6;
     const float dx2 = c.dx * c.dx;
@@ -706,12 +706,13 @@ namespace {
 // projection: vel_bar - D^T M^T G^T vel_bar, accumulated in place.
 void adj_project(Context& c, float* vel_bar, int iterations, float omega) {
     const size_t n = (size_t)c.num_voxels();
-    float* p_bar = adj_scratch(c) + n;
-    float* div_bar = adj_scratch(c) + 2 * n;
+    float* lam = adj_scratch(c);
+    float* p_bar = lam + n;
+    float* div_bar = lam + 2 * n;
     HNS_CUDA(cudaMemsetAsync(p_bar, 0, n * sizeof(float), c.stream));
     HNS_CUDA(cudaMemsetAsync(div_bar, 0, n * sizeof(float), c.stream));
     launch_adj_gradient(c, vel_bar, p_bar);
-    adj_rbgs(c, p_bar, div_bar, iterations, omega);
+    adj_rbgs(c, p_bar, div_bar, iterations, omega, lam);
     launch_adj_divergence(c, div_bar, vel_bar);
 }
 

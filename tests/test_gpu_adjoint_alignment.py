@@ -37,3 +37,23 @@ def test_adjoint_rbgs_of_unaligned_arrays(dev, shift, form):
         got.append(d.clone())
     assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
     grid.close()
+
+
+def test_adjoint_rbgs_takes_one_array_of_scratch(dev):
+    """hns_adjoint_rbgs alone, launched per colour, allocates a copy of p_bar and no block for the other
+    adjoints (two of 2 MiB granules and the tables besides)."""
+    from hnanosolver_b200 import lib as hl
+
+    used = []
+    for edge in (16, 200):  # the small grid loads the kernels
+        grid = hl.Grid(synth.sort_leaves_nanovdb(synth._box_leaves(edge)), voxel_size=0.1)
+        grid.set_option(hl.OPT_SPLIT_SOLVE, hl.SPLIT_PER_COLOUR)
+        p_bar, d = torch.randn(grid.num_voxels, device=dev), torch.zeros(grid.num_voxels, device=dev)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info(dev)[0]
+        grid.adjoint_rbgs(p_bar, d, 4, 1.4)
+        grid.device_status()
+        used.append(before - torch.cuda.mem_get_info(dev)[0])
+        n = grid.num_voxels
+        grid.close()
+    assert used[1] <= 4 * n + (8 << 20)
