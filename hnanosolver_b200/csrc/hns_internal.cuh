@@ -374,7 +374,7 @@ void launch_rbgs_split_half_f32(const Context& c, const int* nb8, const float* r
                                 bool pdl = true, bool walls = false);
 // The solve held in the SMs' shared memory (hns_rbgs_chip.cu): `half_sweeps` half-sweeps (red
 // first) in one cooperative launch, the values of the launch-per-colour kernels to the bit.
-// chip_takes: whether the grid fits and its solve is faster there. The slots flags: the array is in slot order, else colour-split. walls:
+// chip_takes: whether the grid fits, all CTAs at once, and its solve is faster there. The slots flags: the array is in slot order, else colour-split. walls:
 // zero-gradient walls. The launch does nothing when `check` has passed, and ends before half-sweep
 // mid_half when check_mid has.
 enum class ChipUse {
@@ -383,7 +383,7 @@ enum class ChipUse {
     kHalf,       // an FP16 inner solve
     kTransposed  // launch_chip_transpose
 };
-bool chip_takes(const Context& c, ChipUse use);
+bool chip_takes(const Context& c, ChipUse use, bool walls = false);
 void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,
                            int half_sweeps, bool e_zero, float omega, float dx2, bool walls, const double* check,
                            const double* check_mid, int mid_half, double tol2);

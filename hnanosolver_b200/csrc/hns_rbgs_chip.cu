@@ -456,19 +456,40 @@ ChipShape chip_shape(const Context& c, bool transpose) {
 }
 
 template <typename T, ChipMode kMode>
+auto chip_kernel(int threads) {
+    auto kern = rbgs_chip_kernel<T, kMode, 128>;
+    if constexpr (kMode == kTranspose) {
+        if (threads == 256) kern = rbgs_chip_kernel<T, kMode, 256>;
+        if (threads == 1024) kern = rbgs_chip_kernel<T, kMode, 1024>;
+    }
+    // The same limit for every context of the process, so none lowers another's.
+    HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kChipMaxSmem - kChipReserve)));
+    return kern;
+}
+
+// Whether every CTA of a launch is resident at once, as a cooperative launch must be. Asked before each
+// solve: a program may prefer L1 over shared memory (cudaDeviceSetCacheConfig), which leaves room for
+// one CTA an SM. (A carveout preference of the kernel's own would overrule that, but was slower where
+// several contexts solve: with 40 % of shared memory no two grids share the SMs, HNS_Advance on 1,493
+// leaves 454 -> 670 us, and with all of it the adjoint step of a 128^3 box 703 -> 744.)
+template <typename T, ChipMode kMode>
+bool chip_resident(const Context& c) {
+    const ChipShape shape = chip_shape<T>(c, kMode == kTranspose);
+    if (shape.per_cta <= 0) return false;
+    int per_sm = 0;
+    HNS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chip_kernel<T, kMode>(shape.threads), shape.threads,
+                                                           chip_smem<T>(shape.per_cta)));
+    return (int64_t)per_sm * c.sm_count() >= (c.topo.num_leaves + shape.per_cta - 1) / shape.per_cta;
+}
+
+template <typename T, ChipMode kMode>
 void launch_chip(Context& c, ChipArgs<T> A) {
     const int64_t L = c.topo.num_leaves;
     const ChipShape shape = chip_shape<T>(c, kMode == kTranspose);
     A.num_leaves = (int)L;
     A.per_cta = (int)shape.per_cta;
-    auto kern = rbgs_chip_kernel<T, kMode, 128>;
-    if constexpr (kMode == kTranspose) {
-        if (shape.threads == 256) kern = rbgs_chip_kernel<T, kMode, 256>;
-        if (shape.threads == 1024) kern = rbgs_chip_kernel<T, kMode, 1024>;
-    }
+    auto kern = chip_kernel<T, kMode>(shape.threads);
     const unsigned blocks = (unsigned)((L + A.per_cta - 1) / A.per_cta);
-    // The same limit for every context of the process, so none lowers another's.
-    HNS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kChipMaxSmem - kChipReserve)));
     // Face words and the abort word, cleared once. Each launch takes tags that no earlier launch of
     // the context has used, so nothing is cleared between launches; a captured launch runs with the
     // same tags at every replay, so the words are cleared before it.
@@ -505,12 +526,15 @@ void launch_chip(Context& c, ChipArgs<T> A) {
 
 }  // namespace
 
-bool chip_takes(const Context& c, ChipUse use) {
-    if (use == ChipUse::kTransposed) return chip_shape<float>(c, true).per_cta > 0;
+bool chip_takes(const Context& c, ChipUse use, bool walls) {
+    if (use == ChipUse::kTransposed) return chip_resident<float, kTranspose>(c);
     const int per_sm = use == ChipUse::kChecked ? kChipLeavesPerSmChecked
                        : use == ChipUse::kHalf  ? kChipLeavesPerSmHalf
                                                 : kChipLeavesPerSm;
-    return c.topo.num_leaves > 0 && c.topo.num_leaves <= (int64_t)per_sm * c.sm_count();
+    if (c.topo.num_leaves > (int64_t)per_sm * c.sm_count()) return false;
+    return use == ChipUse::kHalf ? chip_resident<__half, kDirichlet>(c)
+           : walls               ? chip_resident<float, kWalls>(c)
+                                 : chip_resident<float, kDirichlet>(c);
 }
 
 void launch_chip_solve_f32(Context& c, const int* nb8, const float* rhs, bool rhs_slots, float* e, bool e_slots,

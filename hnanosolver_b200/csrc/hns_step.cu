@@ -151,7 +151,7 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
     const float dx2 = c.dx * c.dx;
     const bool zero = (flags & HNS_SOLVE_ZERO_INIT) != 0;
     const bool walls = (flags & HNS_SOLVE_NEUMANN) != 0;
-    if (plan == nullptr && use_chip(c, 2 * K) && chip_takes(c, ChipUse::kPlain)) {
+    if (plan == nullptr && use_chip(c, 2 * K) && chip_takes(c, ChipUse::kPlain, walls)) {
         // The whole solve in one launch, from and to the caller's slot order.
         launch_chip_solve_f32(c, c.split_faces(), div, true, p, true, 2 * K, zero, omega, dx2, walls, nullptr, nullptr, 0, 0.0);
         return;
@@ -184,7 +184,7 @@ void split32_solve(Context& c, const float* div, float* p, int K, float omega, u
         convert_split_f32(c, w.e, p, false);
         return;
     }
-    if (plan != nullptr && use_chip(c, 2 * plan->check_every) && chip_takes(c, ChipUse::kChecked)) {
+    if (plan != nullptr && use_chip(c, 2 * plan->check_every) && chip_takes(c, ChipUse::kChecked, walls)) {
         // One launch from each residual evaluation to the next: iteration (c + 1) E - 1, which tests
         // the check before it, and from the second iteration on the check just evaluated.
         const int E = plan->check_every;
