@@ -27,6 +27,7 @@ void fail(hns_status s, const std::string& msg) { throw Error(s, msg); }
 
 void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
     if (e == cudaSuccess) return;
+    (void)cudaGetLastError();  // or the next call's launch check would read it
     const hns_status s = (e == cudaErrorMemoryAllocation) ? HNS_ERR_OUT_OF_MEMORY : HNS_ERR_CUDA;
     throw Error(s, std::string(cudaGetErrorString(e)) + " in " + what + " (" + file + ":" + std::to_string(line) + ")");
 }
