@@ -133,6 +133,38 @@ __device__ __forceinline__ void vel_row(const V* __restrict__ v, int64_t s, floa
         for (int z = 0; z < 4; ++z) u[z] = vload(v, s + z);
     }
 }
+// The same of an array that the kernel writes (in place, the thread's own voxels): plain loads.
+template <bool kVec>
+__device__ __forceinline__ void vel_row_rw(const float* v, int64_t s, float3 u[4]) {
+    if constexpr (kVec) {
+        const float4* q = reinterpret_cast<const float4*>(v + 3 * s);
+        const float4 a = q[0], b = q[1], c = q[2];
+        u[0] = make_float3(a.x, a.y, a.z), u[1] = make_float3(a.w, b.x, b.y);
+        u[2] = make_float3(b.z, b.w, c.x), u[3] = make_float3(c.y, c.z, c.w);
+    } else {
+#pragma unroll
+        for (int z = 0; z < 4; ++z) u[z] = make_float3(v[3 * (s + z)], v[3 * (s + z) + 1], v[3 * (s + z) + 2]);
+    }
+}
+template <bool kVec>
+__device__ __forceinline__ void vel_row_rw(const __nv_bfloat16* v, int64_t s, float3 u[4]) {
+    uint32_t w[6];
+    if constexpr (kVec) {
+        const uint2* q = reinterpret_cast<const uint2*>(v + 3 * s);
+        const uint2 a = q[0], b = q[1], c = q[2];
+        w[0] = a.x, w[1] = a.y, w[2] = b.x, w[3] = b.y, w[4] = c.x, w[5] = c.y;
+    } else {
+        const unsigned short* q = reinterpret_cast<const unsigned short*>(v) + 3 * s;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) w[i] = (uint32_t)q[2 * i] | ((uint32_t)q[2 * i + 1] << 16);
+    }
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+        const int e = 3 * z;
+        u[z] = make_float3(bf16_bits(w[e >> 1], e & 1), bf16_bits(w[(e + 1) >> 1], (e + 1) & 1),
+                           bf16_bits(w[(e + 2) >> 1], (e + 2) & 1));
+    }
+}
 template <bool kVec, typename V>
 __device__ __forceinline__ void store_vel_row(V* v, int64_t s, const float3 u[4]) {
     if constexpr (kVec) {
@@ -257,16 +289,7 @@ __global__ void __launch_bounds__(kRowThreads) gradient_rows_kernel(TopoView t, 
     const float zin = __ldg(p + zin_s), zface = zface_s >= 0 ? __ldg(p + zface_s) : kWalls ? c[r.h ? 3 : 0] : 0.f;
     const float zlo = r.h ? zin : zface, zhi = r.h ? zface : zin;
     float3 u[4];
-    // Read through the ordinary path: in place, the thread's own voxels.
-    if constexpr (kVec) {
-        const float4* v = reinterpret_cast<const float4*>(vel + 3 * r.own);
-        const float4 a = v[0], b = v[1], e = v[2];
-        u[0] = make_float3(a.x, a.y, a.z), u[1] = make_float3(a.w, b.x, b.y);
-        u[2] = make_float3(b.z, b.w, e.x), u[3] = make_float3(e.y, e.z, e.w);
-    } else {
-#pragma unroll
-        for (int z = 0; z < 4; ++z) u[z] = make_float3(vel[3 * (r.own + z)], vel[3 * (r.own + z) + 1], vel[3 * (r.own + z) + 2]);
-    }
+    vel_row_rw<kVec>(vel, r.own, u);
     const float h = 0.5f * inv_dx;
 #pragma unroll
     for (int z = 0; z < 4; ++z) {
@@ -299,7 +322,7 @@ __global__ void __launch_bounds__(kRowThreads) gradient_mixed_kernel(TopoView t,
     const double zin = __ldg(p + zin_s), zface = zface_s < 0 ? 0.0 : __ldg(p + zface_s);
     const double zlo = r.h ? zin : zface, zhi = r.h ? zface : zin;
     float3 u[4];
-    vel_row<kVec>(vel, r.own, u);
+    vel_row_rw<kVec>(vel, r.own, u);
     const double hh = 0.5 * (double)inv_dx;
 #pragma unroll
     for (int z = 0; z < 4; ++z) {

@@ -36,3 +36,18 @@ def test_arrays_of_the_solve_are_read_by_plain_loads(name):
         restricted = re.findall(r"\bconst\s+\w+\s*\*\s*__restrict__\s+(\w+)", params)
         assert set(read) | set(restricted) <= FIXED, (fn, read, restricted)
     assert found >= 2
+
+
+@pytest.mark.parametrize("name", ["hns_rows.cuh", "hns_advance.cu", "hns_fire.cu", "hns_mixed.cu", "hns_adjoint.cu"])
+def test_arrays_that_a_kernel_writes_are_read_by_plain_loads(name):
+    """In-place kernels: a pointer that is not const is not given to a load that is __ldg inside."""
+    loads = r"(?<!\w)(?:__ldg|vload|sload|ld3|ld_half4|vel_z|(?:vel|scalar)_row<\w+>|vel_half_row)\((?:reinterpret_cast<[^>]*>\()?\s*(\w+)"
+    found = 0
+    for fn, params, body in _functions(name):
+        if "__global__" not in params and "kernel" not in fn + params:
+            continue
+        found += 1
+        pointers = re.findall(r"(const\s+)?[\w:]+\s*\*\s*(?:__restrict__\s+)?(\w+)", params)
+        written = {p for const, p in pointers if not const}
+        assert not written & set(re.findall(loads, body)), (fn, params[:120])
+    assert found
