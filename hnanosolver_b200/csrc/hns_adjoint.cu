@@ -193,16 +193,16 @@ __global__ void __launch_bounds__(kThreads) adj_advect_step_kernel(TopoView t, c
             r.x += d * w.x, r.y += d * w.y, r.z += d * w.z;
         }
     };
-    // The scalar shares the velocity's records but not its adjoint: where it has none, a trace of a
-    // velocity that is not finite (weights NaN) adds nothing to it.
-    auto scalar_part = [](float g, float w) { return g != 0.f ? g * w : 0.f; };
+    // The scalar shares the velocity's records but not its adjoint: where one of them has none, a trace of
+    // a velocity that is not finite (weights NaN) adds nothing to it.
+    auto part = [](float g, float w) { return g != 0.f ? g * w : 0.f; };
     auto nonzero = [](const float g[4]) { return g[0] != 0.f || g[1] != 0.f || g[2] != 0.f || g[3] != 0.f; };
     if (nonzero(gpb)) {
         position(tf, gpb, fb);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float w = weight(tf, q);
-            if (tf.s[q] >= 0) dev::red4(rec4 + tf.s[q], gpb[0] * w, gpb[1] * w, gpb[2] * w, scalar_part(gpb[3], w));
+            if (tf.s[q] >= 0) dev::red4(rec4 + tf.s[q], part(gpb[0], w), part(gpb[1], w), part(gpb[2], w), part(gpb[3], w));
         }
     }
     for (int c = 1; c < F.count; ++c) {
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kThreads) adj_advect_step_kernel(TopoView t, c
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float w = weight(tb, q);
-            if (tb.s[q] >= 0) dev::red4(rec4 + tb.s[q], gpf[0] * w, gpf[1] * w, gpf[2] * w, scalar_part(gpf[3], w));
+            if (tb.s[q] >= 0) dev::red4(rec4 + tb.s[q], part(gpf[0], w), part(gpf[1], w), part(gpf[2], w), part(gpf[3], w));
         }
     }
     // back = x - vo sdt.

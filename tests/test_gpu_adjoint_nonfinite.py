@@ -84,3 +84,26 @@ def test_scalar_beside_a_velocity_with_adjoints(dev, bad):
     assert torch.isfinite(got[0]).all()
     assert (got[0] - got[1]).abs().max() <= 0.012
     grid.close()
+
+
+@pytest.mark.parametrize("bad", BAD[:1])
+def test_velocity_beside_a_scalar_with_adjoints(dev, bad):
+    """A scalar's adjoint next to a bad velocity: its forward trace ends at NaN, in the cell at the origin,
+    where the velocity's own adjoint is 0 and stays so (bit for bit: nothing else reaches that corner)."""
+    from hnanosolver_b200 import lib as hl
+
+    o = synth.sort_leaves_nanovdb(synth._box_leaves(32))
+    grid = hl.Grid(o, voxel_size=0.1)
+    ijk = torch.from_numpy(synth.leaf_dense_coords(o)).to(dev)
+    at = (ijk == torch.tensor([21, 13, 18], device=dev, dtype=ijk.dtype)).all(dim=1)
+    vel = torch.full((grid.num_voxels, 3), 0.3, device=dev)
+    vel[at] = bad
+    dens = torch.rand(grid.num_voxels, device=dev, generator=torch.Generator(device=dev).manual_seed(4))
+    out_bar = (((ijk - ijk[at]).abs().amax(dim=1) <= 2) & ~at).float()
+    dens_bar, vel_bar = torch.zeros_like(dens), torch.zeros_like(vel)
+    torch.cuda.synchronize()
+    grid.adjoint_advect_scalar(vel, dens, out_bar, dens_bar, vel_bar, 0.1)
+    grid.synchronize()
+    corner = (ijk <= 8).all(dim=1)
+    assert (vel_bar[corner] == 0.0).all()
+    grid.close()
