@@ -162,6 +162,9 @@ __global__ void __launch_bounds__(kThreads, 2) adj_advect_scalars_kernel(TopoVie
         const float wx = (q & 1) ? tx : 1.0f - tx, wy = (q & 2) ? ty : 1.0f - ty, wz = (q & 4) ? tz : 1.0f - tz;
         return make_float3(((q & 1) ? wy : -wy) * wz, ((q & 2) ? wx : -wx) * wz, ((q & 4) ? wx : -wx) * wy);
     };
+    // The fields share records but not adjoints: one without an adjoint takes nothing, also where the trace
+    // of a velocity that is not finite makes the weights NaN.
+    auto part = [](float g, float w) { return g != 0.f ? g * w : 0.f; };
     const bool fwd = gpb[0] != 0.f || gpb[1] != 0.f || gpb[2] != 0.f || gpb[3] != 0.f || gpb[4] != 0.f;
     const bool back = gpf[0] != 0.f || gpf[1] != 0.f || gpf[2] != 0.f || gpf[3] != 0.f || gpf[4] != 0.f;
     float3 fb = make_float3(0.f, 0.f, 0.f), bb = make_float3(0.f, 0.f, 0.f);
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 2) adj_advect_scalars_kernel(TopoVie
             const float3 w = grad(fx, fy, fz, q);
             fb.x += a * w.x, fb.y += a * w.y, fb.z += a * w.z;
             const float m = fw[q];
-            dev::red4(rec4 + fs[q], gpb[0] * m, gpb[1] * m, gpb[2] * m, gpb[3] * m);
+            dev::red4(rec4 + fs[q], part(gpb[0], m), part(gpb[1], m), part(gpb[2], m), part(gpb[3], m));
             if (gpb[4] != 0.f) atomicAdd(&vel4[fs[q]].w, gpb[4] * m);
         }
     }
@@ -192,8 +195,9 @@ __global__ void __launch_bounds__(kThreads, 2) adj_advect_scalars_kernel(TopoVie
             const float3 w = grad(bx, by, bz, q);
             bb.x += a * w.x, bb.y += a * w.y, bb.z += a * w.z;
             const float m = bw[q];
-            if (back) dev::red4(rec4 + bs[q], gpf[0] * m, gpf[1] * m, gpf[2] * m, gpf[3] * m);
-            if (trace || gpf[4] != 0.f) dev::red4(vel4 + bs[q], vfb.x * m, vfb.y * m, vfb.z * m, gpf[4] * m);
+            if (back) dev::red4(rec4 + bs[q], part(gpf[0], m), part(gpf[1], m), part(gpf[2], m), part(gpf[3], m));
+            if (trace || gpf[4] != 0.f)
+                dev::red4(vel4 + bs[q], part(vfb.x, m), part(vfb.y, m), part(vfb.z, m), part(gpf[4], m));
         }
     }
     bb.x += fb.x, bb.y += fb.y, bb.z += fb.z;

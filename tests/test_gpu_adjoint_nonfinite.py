@@ -107,3 +107,35 @@ def test_velocity_beside_a_scalar_with_adjoints(dev, bad):
     corner = (ijk <= 8).all(dim=1)
     assert (vel_bar[corner] == 0.0).all()
     grid.close()
+
+
+def test_fire_fields_after_a_bad_velocity_source(dev):
+    """The fire step's scalars are advected back together. A velocity source with a NaN in it makes the
+    projected velocity NaN around it, which spoils the gradients of the fields that have adjoints, not those
+    of fields whose adjoints are 0, one in each place of the records."""
+    from hnanosolver_b200 import lib as hl
+
+    o = synth.sort_leaves_nanovdb(synth._box_leaves(32))
+    grid = hl.Grid(o, voxel_size=0.1)
+    n = grid.num_voxels
+    gen = torch.Generator(device=dev).manual_seed(4)
+    names = ("density", "temperature", "fuel", "waste", "flame")
+    fields = {k: torch.rand(n, device=dev, generator=gen) for k in names}
+    fields["velocity"] = torch.rand((n, 3), device=dev, generator=gen)
+    source = torch.zeros((n, 3), device=dev)
+    source[n // 2] = float("nan")
+    p = hl.CombustionParams()
+    p.vorticityScale, p.factorScale, p.substeps = 0.3, 1.0, 1
+    model = hl.ForceModel(combustion=2, burn_rate=0.0, heat_release=0.0, ignition_temp=0.0, density_buoyancy=0.0)
+    for live in ("density", "flame"):
+        out_bar = {k: torch.zeros(n, device=dev) for k in names}
+        out_bar["velocity"] = torch.zeros((n, 3), device=dev)
+        out_bar[live] = torch.randn(n, device=dev, generator=gen)
+        in_bar = {k: torch.zeros_like(v) for k, v in fields.items()}
+        torch.cuda.synchronize()
+        grid.adjoint_advance(fields, {"velocity": source}, out_bar, in_bar, 0.1, 4, p, model)
+        grid.synchronize()
+        assert not torch.isfinite(in_bar[live]).all()
+        for k in ("fuel", "waste", "flame"):  # the buoyancy gives the others the velocity's adjoint
+            assert k == live or (in_bar[k] == 0.0).all(), (live, k)
+    grid.close()
