@@ -248,6 +248,13 @@ __device__ __forceinline__ int64_t inner_slot(int64_t q) {
     else return q;
 }
 
+// The scale of one outer iteration, rms(r); at least FLT_MIN, below which 1 / s overflows (a residual of
+// that size, of velocities about 1e-33 and less, would become NaN).
+__device__ __forceinline__ float residual_scale(const double* check, int64_t n) {
+    const double rms = sqrt(check[0] / (double)n);
+    return rms > 0.0 ? fmaxf((float)rms, 1.17549435e-38f) : 1.0f;
+}
+
 // r^ = r / s with s = rms(r) from the latest check (stored into *scale); FP16 or FP32;
 // r^ in the inner solve's layout kLayout.
 template <typename TI, int kLayout>
@@ -255,8 +262,7 @@ __global__ void __launch_bounds__(kThreads) refine_scale_kernel(const float* __r
                                                                  int64_t n, const double* __restrict__ check,
                                                                  double tol2, float* __restrict__ scale) {
     if (converged(check, tol2)) return;
-    const double rms = sqrt(check[0] / (double)n);
-    const float sc = rms > 0.0 ? (float)rms : 1.0f;
+    const float sc = residual_scale(check, n);
     const float inv = 1.0f / sc;
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale = sc;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
@@ -272,8 +278,7 @@ __global__ void __launch_bounds__(kThreads) refine_scale_split_kernel(const floa
                                                                        const double* __restrict__ check, double tol2,
                                                                        float* __restrict__ scale) {
     if (converged(check, tol2)) return;
-    const double rms = sqrt(check[0] / (double)n);
-    const float sc = rms > 0.0 ? (float)rms : 1.0f;
+    const float sc = residual_scale(check, n);
     const float inv = 1.0f / sc;
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale = sc;
     auto h16 = [](float v) { return (uint32_t)__half_as_ushort(__float2half_rn(v)); };
