@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "hns.h"
+#include "hns_chip_tags.hpp"
 
 namespace hns {
 
@@ -180,8 +181,7 @@ struct Context {
     int inner_layout = HNS_INNER_SPLIT;  // hns_set_option(HNS_OPT_INNER_LAYOUT)
     int first_wait_polls = -1;           // hns_set_option(HNS_OPT_WAIT_POLLS); -1: the kernel's default
     int split_solve = HNS_SPLIT_AUTO;    // hns_set_option(HNS_OPT_SPLIT_SOLVE)
-    uint32_t chip_tag = 1;       // the next launch's first tag (hns_rbgs_chip.cu)
-    bool chip_words_clear = false;  // its face words have been cleared
+    ChipTags chip_tags;          // of the solves held in shared memory (hns_rbgs_chip.cu)
     int coarse_solve = HNS_COARSE_CLUSTER;   // hns_set_option(HNS_OPT_COARSE_SOLVE)
     int l2_persist = 1;                      // hns_set_option(HNS_OPT_L2_PERSIST)
     // The access-policy window of the inner solve's launches while a refined solve runs

@@ -25,7 +25,7 @@
 // brings all such faces into shared memory together, so that their latency is paid once.
 //
 // Order. Every value in `faces` is stored together with a tag, as one 8-byte word: the number of
-// the half-sweep that made it, counted on from launch to launch. A reader polls the words
+// the half-sweep that made it, counted on from launch to launch (ChipTags). A reader polls the words
 // themselves until they carry the tag it waits for, so a half-sweep costs one store and one load
 // through L2 between CTAs, with no fence, flag or grid barrier (with flags behind a fence a
 // half-sweep of a 64^3 box took 3.9 us). A word is safe to overwrite: the
@@ -490,22 +490,18 @@ void launch_chip(Context& c, ChipArgs<T> A) {
     A.per_cta = (int)shape.per_cta;
     auto kern = chip_kernel<T, kMode>(shape.threads);
     const unsigned blocks = (unsigned)((L + A.per_cta - 1) / A.per_cta);
-    // Face words and the abort word, cleared once. Each launch takes tags that no earlier launch of
-    // the context has used, so nothing is cleared between launches; a captured launch runs with the
-    // same tags at every replay, so the words are cleared before it.
+    // Face words and the abort word, cleared where the tags need it (ChipTags).
     const size_t words = (size_t)L * 2 * 6 * kFaceWords;
     auto* w = reinterpret_cast<uint64_t*>(c.scratch_f32("chip_faces", 2 * words + 2));
-    const bool captured = c.stream_capturing();
-    if (!c.chip_words_clear || captured) HNS_CUDA(cudaMemsetAsync(w, 0, words * 8 + 8, c.stream));
-    if (!captured) c.chip_words_clear = true;
+    const ChipTags::Launch tags = c.chip_tags.take((uint32_t)A.half_sweeps, c.stream_capturing());
+    if (tags.clear) {
+        const cudaError_t cleared = cudaMemsetAsync(w, 0, words * 8 + 8, c.stream);
+        if (cleared != cudaSuccess) c.chip_tags = ChipTags();
+        HNS_CUDA(cleared);
+    }
     A.faces = w;
     A.abort_word = reinterpret_cast<unsigned*>(w + words);
-    if (c.chip_tag > 0xF0000000u) {
-        c.chip_tag = 1u;
-        HNS_CUDA(cudaMemsetAsync(w, 0, words * 8 + 8, c.stream));
-    }
-    A.tag0 = c.chip_tag;
-    c.chip_tag += (uint32_t)A.half_sweeps + 1u;
+    A.tag0 = tags.first;
     A.stall = c.first_wait_polls >= 0;
     A.max_polls = A.stall ? std::min((uint32_t)c.first_wait_polls, kChipMaxPolls) : kChipMaxPolls;
     A.counters = c.counters;
