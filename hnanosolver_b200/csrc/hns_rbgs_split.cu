@@ -53,15 +53,16 @@ constexpr int kShortGridCtasPerSm = 6;  // the register limit at 80 registers an
 constexpr int kHalfCtasPerSm = 6;       // the half-sweep kernel's launch bound
 // Smaller grids take two leaves per thread at eight CTAs per SM: with four, less than a wave of CTAs is
 // spread unevenly over the SMs. Where the launches of several streams fill the SMs between them, four
-// leaves in flight per thread win from about 4,000 leaves on in the red-black solves, hundreds of these
+// leaves in flight per thread win from about 4,500 leaves on in the red-black solves, hundreds of these
 // launches in a row; the multigrid cycle's few sit between other kernels. Step of three outer iterations,
 // us, four -> two, alone / three contexts taking turns:
 //   leaves                      1,500                   3,700                   4,500                   5,900
 //   red-black  863 -> 725 / 481 -> 469  1037 -> 859 / 504 -> 505  1081 -> 922 / 569 -> 585  1128 -> 1110 / 698 -> 742
 //   multigrid  587 -> 573 / 377 -> 374   801 -> 777 / 446 -> 439   878 -> 845 / 503 -> 496    934 ->  934 / 573 -> 571
-// 6,594 leaves, us per half-sweep: 3.5 -> 3.8.
+// Five outer iterations, red-black: 4,100 leaves 1301 -> 1072 / 677 -> 672, 4,300 1315 -> 1115 / 672 -> 671, 4,500
+// 1326 -> 1139 / 672 -> 682, 4,700 1331 -> 1163 / 673 -> 707. 6,594 leaves, us per half-sweep: 3.5 -> 3.8.
 constexpr int kHalfCtasPerSm2 = 8;
-constexpr int64_t kTwoLeafLimit = 4000, kTwoLeafLimitCycle = 6000;
+constexpr int64_t kTwoLeafLimit = 4400, kTwoLeafLimitCycle = 6000;
 
 // nbr27 indices of the six face neighbours: (dx+1)*9 + (dy+1)*3 + (dz+1).
 constexpr int kNbXp = 22, kNbXm = 4, kNbYp = 16, kNbYm = 10, kNbZp = 14, kNbZm = 12;
