@@ -474,6 +474,7 @@ HNS_API hns_status hns_advance_mixed_host(hns_ctx* ctx, const hns_fire_f32* fiel
         Context* c = check_ctx(ctx);
         if (!fields || !fields->velocity) fail(HNS_ERR_INVALID_ARG, "null host fields");
         DeviceGuard dg(c->device);
+        const HostCall waits(*c);
         const size_t n = (size_t)c->num_voxels();
         float* host[6] = {fields->velocity, fields->density, fields->temperature, fields->fuel, fields->waste, fields->flame};
         static const char* names[6] = {"velocity", "density", "temperature", "fuel", "waste", "flame"};

@@ -182,6 +182,7 @@ struct Context {
     int first_wait_polls = -1;           // hns_set_option(HNS_OPT_WAIT_POLLS); -1: the kernel's default
     int split_solve = HNS_SPLIT_AUTO;    // hns_set_option(HNS_OPT_SPLIT_SOLVE)
     ChipTags chip_tags;          // of the solves held in shared memory (hns_rbgs_chip.cu)
+    bool host_call = false;      // in a call on host arrays, which waits for its work (HostCall)
     int coarse_solve = HNS_COARSE_CLUSTER;   // hns_set_option(HNS_OPT_COARSE_SOLVE)
     int l2_persist = 1;                      // hns_set_option(HNS_OPT_L2_PERSIST)
     // The access-policy window of the inner solve's launches while a refined solve runs
@@ -268,6 +269,16 @@ struct CaptureStream {
     ~CaptureStream() { c.stream = saved; }
     CaptureStream(const CaptureStream&) = delete;
     CaptureStream& operator=(const CaptureStream&) = delete;
+};
+
+// Marks the running call as one on host arrays: it waits for its work, so a program that makes its calls
+// from one thread has no other context's work beside it.
+struct HostCall {
+    Context& c;
+    explicit HostCall(Context& ctx) : c(ctx) { c.host_call = true; }
+    ~HostCall() { c.host_call = false; }
+    HostCall(const HostCall&) = delete;
+    HostCall& operator=(const HostCall&) = delete;
 };
 
 struct DeviceGuard {

@@ -1095,6 +1095,7 @@ HNS_API hns_status hns_step_mixed_host(hns_ctx* ctx, float* vel, float* const* s
         if (!vel) fail(HNS_ERR_INVALID_ARG, "null velocity");
         if (nscalars < 0 || (nscalars > 0 && !scalars)) fail(HNS_ERR_INVALID_ARG, "bad scalar arrays");
         DeviceGuard dg(c->device);
+        const HostCall waits(*c);
         const size_t n = (size_t)c->num_voxels();
         // Host data is FP32 (the reference's GridIndexedData); it is staged in FP32, converted
         // to BF16/FP16 on the device, stepped, and converted back. The host link is the bound:

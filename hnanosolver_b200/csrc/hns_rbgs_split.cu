@@ -62,6 +62,8 @@ constexpr int kHalfCtasPerSm = 6;       // the half-sweep kernel's launch bound
 // Five outer iterations, red-black: 4,100 leaves 1301 -> 1072 / 677 -> 672, 4,300 1315 -> 1115 / 672 -> 671, 4,500
 // 1326 -> 1139 / 672 -> 682, 4,700 1331 -> 1163 / 673 -> 707. 6,594 leaves, us per half-sweep: 3.5 -> 3.8.
 constexpr int kHalfCtasPerSm2 = 8;
+// A call on host arrays waits for its work, so it goes by the times alone, with the cycle's limit: step of 16 outer
+// iterations, four -> two: 4,913 leaves 5260 -> 4810, 5,832 leaves 5578 -> 5550.
 constexpr int64_t kTwoLeafLimit = 4400, kTwoLeafLimitCycle = 6000;
 
 // nbr27 indices of the six face neighbours: (dx+1)*9 + (dy+1)*3 + (dz+1).
@@ -654,7 +656,7 @@ void launch_rbgs_split_half(const Context& c, const int* nb8, const void* rhs, v
     const int64_t L = c.topo.num_leaves;
     if (L == 0) return;
     if (L >= (int64_t(1) << 22)) fail(HNS_ERR_INVALID_ARG, "too many leaves for the colour-split inner solve");
-    const bool two = L <= (in_cycle ? kTwoLeafLimitCycle : kTwoLeafLimit);
+    const bool two = L <= (in_cycle || c.host_call ? kTwoLeafLimitCycle : kTwoLeafLimit);
     const int per_block = kLeavesPerBlock * (two ? 2 : kLeavesPerThread);
     unsigned blocks = (unsigned)((L + per_block - 1) / per_block);
     // A launch that will most likely return at once (the refinement expected to have converged)
