@@ -133,7 +133,7 @@ struct ChipArgs {
     double tol2;
     unsigned long long* counters;
     uint32_t max_polls;  // after which a wait gives up
-    bool stall;          // the test hook of the timeout path: no tag is accepted
+    uint32_t refuse;     // the test hook of the timeout path: ~0, with which no tag is accepted; else 0
 };
 
 // Row (a, b) of `leaf`: its values of colour 0 and 1. Slot order holds z = 0 .. 7 in a row; entry j
@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
     // Brings the other CTAs' faces of colour k, tagged `tag`, into the halo; true if a wait gave up.
     auto get_faces = [&](int k, uint32_t tag) {
         const uint64_t* faces = A.faces + k * colour_stride;
+        const uint32_t want = tag | A.refuse;
         bool failed = false;
         for (int q = tid; q < nf * kPieces; q += kChipThreads) {
             const int i = q & (kPieces - 1), lf = foreign[q / kPieces], l = lf >> 3, f = lf & 7;
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kChipThreads, 1024 / kChipThreads) rbgs_chip_k
             uint32_t polls = 0;
             for (;;) {
                 get2(src, x, y);
-                if (!A.stall && (uint32_t)(x >> 32) == tag && (uint32_t)(y >> 32) == tag) break;
+                if ((uint32_t)(x >> 32) == want && (uint32_t)(y >> 32) == want) break;
                 if (++polls >= A.max_polls) {
                     atomicExch(A.abort_word, A.tag0);
                     if (A.counters != nullptr) atomicExch(A.counters + 1, 1ull);
@@ -502,8 +503,9 @@ void launch_chip(Context& c, ChipArgs<T> A) {
     A.faces = w;
     A.abort_word = reinterpret_cast<unsigned*>(w + words);
     A.tag0 = tags.first;
-    A.stall = c.first_wait_polls >= 0;
-    A.max_polls = A.stall ? std::min((uint32_t)c.first_wait_polls, kChipMaxPolls) : kChipMaxPolls;
+    const bool stall = c.first_wait_polls >= 0;
+    A.refuse = stall ? ~0u : 0u;
+    A.max_polls = stall ? std::min((uint32_t)c.first_wait_polls, kChipMaxPolls) : kChipMaxPolls;
     A.counters = c.counters;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
