@@ -573,6 +573,19 @@ __global__ void __launch_bounds__(kThreads) accumulate_kernel(const float* __res
 
 }  // namespace
 
+// The adjoints' scratch block of 8 n floats: lam, p_bar and div_bar of the projection, then the
+// records of the advection that follows it.
+float* adj_scratch(Context& c) { return c.scratch_f32("adjoint_work", 8 * (size_t)c.num_voxels()); }
+
+// That block where the context has it, else `floats` n of scratch: a projection or a confinement that is
+// differentiated alone needs no records. (The block is not made from the smaller one by growing it, which
+// would free what a captured call uses.)
+float* adj_scratch(Context& c, const char* own, size_t floats) {
+    const auto block = c.scratch.find("adjoint_work");
+    return block != c.scratch.end() && block->second.ptr ? adj_scratch(c)
+                                                         : c.scratch_f32(own, floats * (size_t)c.num_voxels());
+}
+
 void launch_adj_accumulate(const Context& c, const float* src, float* dst, int64_t n) {
     if (n <= 0) return;
     accumulate_kernel<<<blocks_for(n), kThreads, 0, c.stream>>>(src, dst, n);
@@ -584,7 +597,7 @@ void launch_adj_advect(Context& c, const float* vel, const float* vel_out_bar, c
                        float* work) {
     const int64_t n = c.num_voxels();
     if (n == 0) return;
-    if (work == nullptr) work = c.scratch_f32("adjoint_work", 8 * (size_t)n);
+    if (work == nullptr) work = adj_scratch(c);
     auto* rec4 = reinterpret_cast<float4*>(work);
     auto* in4 = rec4 + n;
     int base = 0;
@@ -639,7 +652,7 @@ void launch_adj_confinement(Context& c, const float* vel, const float* out_bar, 
     if (n == 0) return;
     const int fs = (int)factor_scale;
     if (fs == 1 || fs == -1) {
-        if (work == nullptr) work = c.scratch_f32("adjoint_work", 8 * (size_t)n);
+        if (work == nullptr) work = adj_scratch(c, "adjoint_confinement_work", 6);
         float *wb = work, *gb = work + 3 * n;
         const float f = 0.5f * (1.0f / c.dx);
         adj_confine_force_kernel<<<(unsigned)c.topo.num_leaves, kThreads, 0, c.stream>>>(c.topo.view, vel, out_bar, wb, gb, dt,
@@ -662,10 +675,6 @@ void launch_adj_confinement(Context& c, const float* vel, const float* out_bar, 
 // ---- C ABI -----------------------------------------------------------------------------------
 
 namespace hns {
-
-// The adjoints' scratch block of 8 n floats: lam, p_bar and div_bar of the projection, then the
-// records of the advection that follows it.
-float* adj_scratch(Context& c) { return c.scratch_f32("adjoint_work", 8 * (size_t)c.num_voxels()); }
 
 // The adjoint of `iterations` red-black iterations from p = 0 (the forward's
 // HNS_SOLVE_ZERO_INIT): the half-sweeps' transposes in reverse order, black first, in place on
@@ -703,10 +712,9 @@ void adj_rbgs(Context& c, const float* p_bar, float* div_bar, int iterations, fl
 namespace {
 
 // vel_bar (the adjoint of the projected velocity) -> the adjoint of the velocity before the
-// projection: vel_bar - D^T M^T G^T vel_bar, accumulated in place.
-void adj_project(Context& c, float* vel_bar, int iterations, float omega) {
+// projection: vel_bar - D^T M^T G^T vel_bar, accumulated in place. lam: 3 n floats of scratch.
+void adj_project(Context& c, float* vel_bar, int iterations, float omega, float* lam) {
     const size_t n = (size_t)c.num_voxels();
-    float* lam = adj_scratch(c);
     float* p_bar = lam + n;
     float* div_bar = lam + 2 * n;
     HNS_CUDA(cudaMemsetAsync(p_bar, 0, n * sizeof(float), c.stream));
@@ -786,7 +794,7 @@ HNS_API hns_status hns_adjoint_project(hns_ctx* ctx, float* vel_bar, int iterati
         need(vel_bar, "velocity adjoint");
         if (iterations < 0) fail(HNS_ERR_INVALID_ARG, "negative iteration count");
         DeviceGuard g(c->device);
-        adj_project(*c, vel_bar, iterations, default_omega(*c, omega));
+        adj_project(*c, vel_bar, iterations, default_omega(*c, omega), adj_scratch(*c, "adjoint_project_work", 3));
     });
 }
 
@@ -817,7 +825,7 @@ HNS_API hns_status hns_adjoint_step_plain(hns_ctx* ctx, const float* vel_in, con
         // Adjoint of the advected velocity: the output adjoint through the projection.
         float* adv_bar = c->scratch_f32("adjoint_adv_bar", (size_t)n3);
         HNS_CUDA(cudaMemcpyAsync(adv_bar, vel_out_bar, (size_t)n3 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
-        adj_project(*c, adv_bar, iterations, default_omega(*c, omega));
+        adj_project(*c, adv_bar, iterations, default_omega(*c, omega), adj_scratch(*c));
         // Velocity self-advection and the scalars' advection along the same velocity.
         launch_adj_advect(*c, vel_in, adv_bar, scalars_in, scalars_out_bar, scalars_in_bar, nscalars, vel_in_bar, dt);
     });

@@ -57,3 +57,26 @@ def test_adjoint_rbgs_takes_one_array_of_scratch(dev):
         n = grid.num_voxels
         grid.close()
     assert used[1] <= 4 * n + (8 << 20)
+
+
+@pytest.mark.parametrize("name,floats", [("project", 3), ("confinement", 6)])
+def test_adjoints_alone_take_their_own_scratch(dev, name, floats):
+    """The adjoint of a projection or of the confinement alone allocates its arrays, not the block of eight
+    floats a voxel that the advections' records need (8 MiB of granules and tables besides)."""
+    from hnanosolver_b200 import lib as hl
+
+    used = []
+    for edge in (16, 200):  # the small grid loads the kernels
+        grid = hl.Grid(synth.sort_leaves_nanovdb(synth._box_leaves(edge)), voxel_size=0.1)
+        n = grid.num_voxels
+        vel, bar, out = (torch.randn((n, 3), device=dev) for _ in range(3))
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info(dev)[0]
+        if name == "project":
+            grid.adjoint_project(bar, 4, 1.4)
+        else:
+            grid.adjoint_vorticity_confinement(vel, bar, out, 0.1, 0.4, 1.0)
+        grid.device_status()
+        used.append(before - torch.cuda.mem_get_info(dev)[0])
+        grid.close()
+    assert used[1] <= 4 * floats * n + (8 << 20)
